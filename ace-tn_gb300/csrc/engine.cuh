@@ -35,12 +35,20 @@ void to_f64(Ctx& c, const float* x, double* y, int64_t n);
 // ~u cond^2 after the shifted stage, i.e. about 1e-3 in FP32, for bases that
 // are only multiplied again in lower precision).
 void orthonormalize(Ctx& c, double* Y, int64_t n, int64_t q, double* R, int stages = 3);
+// Shifted Cholesky-QR3 of Y without the Householder fallback: bit 1 of
+// *failed (device, cleared first) is set when the result is not orthonormal
+// to working precision, and Y and R then mean nothing.
+void orthonormalize_try(Ctx& c, double* Y, int64_t n, int64_t q, double* R, int* failed);
 // The same in FP32 arithmetic (mixed path).
 void orthonormalize(Ctx& c, float* Y, int64_t n, int64_t q, float* R, int stages = 3);
 // Thin SVD of X (m x n, row-major, m >= n is not required):
 // X = U diag(S) V^T, U (m x r), S (r) descending, V (n x r), r = min(m, n).
 void svd_thin(Ctx& c, const double* X, int64_t m, int64_t n, double* U, double* S,
               double* V);
+// FP32 one-sided Jacobi on the rows of Mc (q x q): Jc (q x q) the accumulated
+// rotations (orthogonal to FP32 accuracy), norms the final row norms; *flags
+// gets bit 2 when the sweep limit is reached.
+void jacobi_rotations(Ctx& c, const float* Mc, int64_t q, float* Jc, float* norms, int* flags);
 // Thin SVD of B (q x n, q <= min(n, 1024)) for the mixed path, from
 // Bt = B^T (n x q, FP32): R of a shifted Cholesky-QR3 of Bt (B = R^T Qb^T),
 // FP32 one-sided Jacobi on the columns of R with accumulated rotations

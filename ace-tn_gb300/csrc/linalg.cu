@@ -4,9 +4,6 @@
 //    42 (2020) A477) built on the GETT engine, with an orthogonality check
 //    and a one-CTA Householder QR that runs instead when the check fails
 //    (numerically rank-deficient input) or the problem is small.
-//  * svd_thin(): one-sided (Hestenes) Jacobi SVD with the round-robin pair
-//    ordering, run as a cooperative multi-CTA kernel with a bounded grid
-//    barrier (Demmel & Veselic, SIAM J. Matrix Anal. Appl. 13 (1992) 1204).
 //  * truncation of the singular spectrum and column scaling of the
 //    projectors (acetn/renormalization/projectors.py:163-167).
 #include "engine.cuh"
@@ -880,158 +877,6 @@ __global__ void __launch_bounds__(1024) orthogonality_check_kernel(const T* G, i
   if (threadIdx.x == 0 && bad) atomicOr(flags, 1);
 }
 
-// ------------------------------------------------------------- Jacobi SVD
-struct JacobiArgs {
-  double* W;      // p x L, row j = column j being orthogonalised
-  double* J;      // p x p, row j = column j of the accumulated rotation
-  int64_t p, L;
-  int64_t pp;     // p rounded up to even
-  double tol;
-  int max_sweeps;
-  unsigned* bar;  // [0] arrival count, [1] generation, [2] abort, [3..4] sweep flags
-  int* flags;
-  int64_t spin_limit;
-};
-
-// Bounded grid barrier.  Returns false when this CTA gave up waiting (the
-// abort word is then set and the status flag records the timeout).
-__device__ bool grid_sync(const JacobiArgs& a) {
-  __syncthreads();
-  __shared__ int ok;
-  if (threadIdx.x == 0) {
-    volatile unsigned* gen = a.bar + 1;
-    volatile unsigned* abort_w = a.bar + 2;
-    ok = 1;
-    const unsigned g = *gen;
-    __threadfence();
-    const unsigned arrived = atomicAdd(a.bar, 1u);
-    if (arrived == gridDim.x - 1) {
-      atomicExch(a.bar, 0u);
-      __threadfence();
-      atomicAdd(const_cast<unsigned*>(gen), 1u);
-    } else {
-      int64_t it = 0;
-      while (*gen == g) {
-        if (*abort_w != 0u || ++it > a.spin_limit) {
-          atomicExch(const_cast<unsigned*>(abort_w), 1u);
-          atomicOr(a.flags, 2);
-          ok = 0;
-          break;
-        }
-        __nanosleep(64);
-      }
-    }
-    __threadfence();
-  }
-  __syncthreads();
-  return ok != 0;
-}
-
-__device__ __forceinline__ int64_t rr_pos(int64_t i, int64_t r, int64_t pp) {
-  return i == 0 ? 0 : ((i - 1 + r) % (pp - 1)) + 1;
-}
-
-__global__ void __launch_bounds__(64) jacobi_sweeps_kernel(const JacobiArgs a) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warps_per_cta = blockDim.x >> 5;
-  const int64_t gw = blockIdx.x * warps_per_cta + (threadIdx.x >> 5);
-  const int64_t total_w = gridDim.x * warps_per_cta;
-  const int64_t npairs = a.pp / 2;
-  for (int sweep = 0; sweep < a.max_sweeps; ++sweep) {
-    unsigned* rotated = a.bar + 3 + (sweep & 1);
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicExch(a.bar + 3 + ((sweep + 1) & 1), 0u);
-    for (int64_t r = 0; r < a.pp - 1; ++r) {
-      for (int64_t k = gw; k < npairs; k += total_w) {
-        int64_t i = rr_pos(k, r, a.pp), j = rr_pos(a.pp - 1 - k, r, a.pp);
-        if (i > j) { const int64_t t = i; i = j; j = t; }
-        if (j >= a.p) continue;  // dummy partner
-        double* wi = a.W + i * a.L;
-        double* wj = a.W + j * a.L;
-        double al = 0.0, be = 0.0, ga = 0.0;
-        for (int64_t t = lane; t < a.L; t += 32) {
-          const double x = wi[t], y = wj[t];
-          al = fma(x, x, al);
-          be = fma(y, y, be);
-          ga = fma(x, y, ga);
-        }
-        al = warp_sum(al);
-        be = warp_sum(be);
-        ga = warp_sum(ga);
-        if (al == 0.0 || be == 0.0 || !(fabs(ga) > a.tol * sqrt(al) * sqrt(be))) continue;
-        const double zeta = (be - al) / (2.0 * ga);
-        const double t = copysign(1.0, zeta) / (fabs(zeta) + sqrt(fma(zeta, zeta, 1.0)));
-        const double cs = 1.0 / sqrt(fma(t, t, 1.0));
-        const double sn = cs * t;
-        for (int64_t u = lane; u < a.L; u += 32) {
-          const double x = wi[u], y = wj[u];
-          wi[u] = cs * x - sn * y;
-          wj[u] = sn * x + cs * y;
-        }
-        double* ji = a.J + i * a.p;
-        double* jj = a.J + j * a.p;
-        for (int64_t u = lane; u < a.p; u += 32) {
-          const double x = ji[u], y = jj[u];
-          ji[u] = cs * x - sn * y;
-          jj[u] = sn * x + cs * y;
-        }
-        if (lane == 0) atomicExch(rotated, 1u);
-      }
-      if (!grid_sync(a)) return;
-    }
-    const unsigned any = *(volatile unsigned*)rotated;
-    if (!grid_sync(a)) return;
-    if (any == 0u) return;
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(a.flags, 2);
-}
-
-// Sorts the Jacobi result by descending column norm and writes U, S, V.
-// trans == 0: W rows are columns of X (m >= n): U = W_j / s_j, V = J.
-// trans == 1: W rows are rows of X (m < n):  U = J, V = W_j / s_j.
-__global__ void jacobi_finish_kernel(const double* W, const double* J, int64_t p, int64_t L,
-                                     int trans, double* U, double* S, double* V) {
-  const int64_t j = blockIdx.x;
-  if (j >= p) return;
-  __shared__ double sh[LT / 32];
-  __shared__ double s_norm;
-  __shared__ int64_t s_rank;
-  double part = 0.0;
-  for (int64_t t = threadIdx.x; t < L; t += blockDim.x) part = fma(W[j * L + t], W[j * L + t], part);
-  const double nj2 = block_sum(part, sh);
-  // rank: strictly larger norms (ties broken by index); norms recomputed per
-  // column so every block sees identical values
-  int64_t cnt = 0;
-  for (int64_t i = threadIdx.x; i < p; i += blockDim.x) {
-    if (i == j) continue;
-    double ni2 = 0.0;
-    for (int64_t t = 0; t < L; ++t) ni2 = fma(W[i * L + t], W[i * L + t], ni2);
-    if (ni2 > nj2 || (ni2 == nj2 && i < j)) ++cnt;
-  }
-  const double c = block_sum(double(cnt), sh);
-  if (threadIdx.x == 0) {
-    s_norm = sqrt(nj2);
-    s_rank = static_cast<int64_t>(c + 0.5);
-  }
-  __syncthreads();
-  const double sj = s_norm;
-  const int64_t rk = s_rank;
-  const double inv = sj > 0.0 ? 1.0 / sj : 0.0;
-  if (threadIdx.x == 0) S[rk] = sj;
-  if (trans == 0) {
-    for (int64_t t = threadIdx.x; t < L; t += blockDim.x) U[t * p + rk] = W[j * L + t] * inv;
-    for (int64_t t = threadIdx.x; t < p; t += blockDim.x) V[t * p + rk] = J[j * p + t];
-  } else {
-    for (int64_t t = threadIdx.x; t < p; t += blockDim.x) U[t * p + rk] = J[j * p + t];
-    for (int64_t t = threadIdx.x; t < L; t += blockDim.x) V[t * p + rk] = W[j * L + t] * inv;
-  }
-}
-
-__global__ void identity_kernel(double* X, int64_t p) {
-  for (int64_t idx = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; idx < p * p;
-       idx += int64_t(gridDim.x) * blockDim.x)
-    X[idx] = (idx / p == idx % p) ? 1.0 : 0.0;
-}
-
 // ------------------------------------------------------------- truncation
 __global__ void truncation_kernel(const double* s, int64_t r, int64_t chi, double cutoff,
                                   double* f, int64_t cap, int64_t* chi_new) {
@@ -1419,7 +1264,8 @@ void slab_gram(Ctx& c, const float* Y, int64_t n, int64_t q, const float* Lt, fl
 }
 
 template <class T>
-void orthonormalize_impl(Ctx& c, T* Y, int64_t n, int64_t q, T* R, int stages) {
+void orthonormalize_impl(Ctx& c, T* Y, int64_t n, int64_t q, T* R, int stages,
+                         int* failed = nullptr) {
   CTM_REQUIRE(n >= q && q >= 1, CTM_ERR_INVALID, "orthonormalize: needs n >= q >= 1");
   CTM_REQUIRE(stages == 2 || stages == 3, CTM_ERR_INVALID, "orthonormalize: 2 or 3 stages");
   Scope scope(c);
@@ -1427,7 +1273,9 @@ void orthonormalize_impl(Ctx& c, T* Y, int64_t n, int64_t q, T* R, int stages) {
   T* beta = c.alloc<T>(q);
   // the one-CTA Householder QR for small problems (its cost grows as q^2
   // barriers); the FP32 slab kernels beat it from q = 32 on
-  const bool small = (sizeof(T) == 4 && q >= 32) ? false : double(n) * q * q <= 4.0e6;
+  const bool small = (failed != nullptr || (sizeof(T) == 4 && q >= 32))
+                         ? false
+                         : double(n) * q * q <= 4.0e6;
   if (small) {
     if (c.sizing()) return;
     KernelTimer kt(c.stream, "householder_qr_kernel", kUnitFlop, 4.0 * double(n) * q * q);
@@ -1444,10 +1292,10 @@ void orthonormalize_impl(Ctx& c, T* Y, int64_t n, int64_t q, T* R, int stages) {
   T* Lt = c.alloc<T>(size_t(q) * q);
   T* Rt = c.alloc<T>(size_t(q) * q);
   T* Rt2 = c.alloc<T>(size_t(q) * q);
-  int* flags = c.alloc<int>(1);
+  int* flags = failed != nullptr ? failed : c.alloc<int>(1);
   // keep the input for the fallback in V
   if (!c.sizing()) {
-    CTM_CUDA(cudaMemcpyAsync(V, Y, sizeof(T) * n * q, cudaMemcpyDeviceToDevice, c.stream));
+    if (failed == nullptr) CTM_CUDA(cudaMemcpyAsync(V, Y, sizeof(T) * n * q, cudaMemcpyDeviceToDevice, c.stream));
     CTM_CUDA(cudaMemsetAsync(flags, 0, sizeof(int), c.stream));
   }
   T* cur = Y;
@@ -1516,6 +1364,7 @@ void orthonormalize_impl(Ctx& c, T* Y, int64_t n, int64_t q, T* R, int stages) {
     CTM_CUDA(cudaMemcpyAsync(Y, cur, sizeof(T) * n * q, cudaMemcpyDeviceToDevice, c.stream));
   if (R != nullptr)
     CTM_CUDA(cudaMemcpyAsync(R, Rt, sizeof(T) * q * q, cudaMemcpyDeviceToDevice, c.stream));
+  if (failed != nullptr) return;  // the caller looks at the flag
   // when flagged: Y = the saved input, then its Householder QR
   householder_qr_kernel<T><<<1, LT, 0, c.stream>>>(Y, n, q, R, hv, beta, flags, 1, V);
   CTM_LAUNCH_CHECK();
@@ -1525,60 +1374,12 @@ void orthonormalize(Ctx& c, double* Y, int64_t n, int64_t q, double* R, int stag
   orthonormalize_impl<double>(c, Y, n, q, R, stages);
 }
 
-void orthonormalize(Ctx& c, float* Y, int64_t n, int64_t q, float* R, int stages) {
-  orthonormalize_impl<float>(c, Y, n, q, R, stages);
+void orthonormalize_try(Ctx& c, double* Y, int64_t n, int64_t q, double* R, int* failed) {
+  orthonormalize_impl<double>(c, Y, n, q, R, 3, failed);
 }
 
-void svd_thin(Ctx& c, const double* X, int64_t m, int64_t n, double* U, double* S, double* V) {
-  CTM_REQUIRE(m >= 1 && n >= 1, CTM_ERR_INVALID, "svd_thin: empty matrix");
-  const int trans = m >= n ? 0 : 1;
-  const int64_t p = std::min(m, n), L = std::max(m, n);
-  Scope scope(c);
-  double* W = c.alloc<double>(size_t(p) * L);
-  double* J = c.alloc<double>(size_t(p) * p);
-  unsigned* bar = c.alloc<unsigned>(8);
-  if (c.sizing()) return;
-  // W rows = columns of X (trans 0) or rows of X (trans 1)
-  if (trans == 0)
-    copy2d(c, View(X, {m, n}).permute({1, 0}), W, L);
-  else
-    CTM_CUDA(cudaMemcpyAsync(W, X, sizeof(double) * m * n, cudaMemcpyDeviceToDevice, c.stream));
-  identity_kernel<<<grid_for(p * p, 256), 256, 0, c.stream>>>(J, p);
-  CTM_LAUNCH_CHECK();
-  CTM_CUDA(cudaMemsetAsync(bar, 0, 8 * sizeof(unsigned), c.stream));
-  JacobiArgs a{};
-  a.W = W;
-  a.J = J;
-  a.p = p;
-  a.L = L;
-  a.pp = p + (p & 1);
-  a.tol = 2.220446049250313e-16 * std::sqrt(double(L));
-  a.max_sweeps = 60;
-  a.bar = bar;
-  a.flags = status_flags(c);
-  a.spin_limit = int64_t(20) * 1000 * 1000;  // ~1-2 s of 64 ns sleeps
-  if (p > 1) {
-    int dev = 0, sms = 0, per_sm = 0;
-    CTM_CUDA(cudaGetDevice(&dev));
-    CTM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const int threads = 64;
-    CTM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, jacobi_sweeps_kernel, threads, 0));
-    const int64_t npairs = a.pp / 2;
-    int64_t blocks = (npairs + 1) / 2;
-    blocks = std::min<int64_t>(blocks, int64_t(sms) * std::max(per_sm, 1));
-    blocks = std::min<int64_t>(blocks, sms);
-    blocks = std::max<int64_t>(blocks, 1);
-    void* args[] = {&a};
-    KernelTimer kt(c.stream, "jacobi_sweeps_kernel", kUnitFlop, 0.0);
-    CTM_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(jacobi_sweeps_kernel),
-                                         dim3(unsigned(blocks)), dim3(threads), args, 0, c.stream));
-    CTM_LAUNCH_CHECK();
-  }
-  {
-    KernelTimer kt(c.stream, "jacobi_finish_kernel", kUnitFlop, 2.0 * double(p) * p * L);
-    jacobi_finish_kernel<<<unsigned(p), LT, 0, c.stream>>>(W, J, p, L, trans, U, S, V);
-    CTM_LAUNCH_CHECK();
-  }
+void orthonormalize(Ctx& c, float* Y, int64_t n, int64_t q, float* R, int stages) {
+  orthonormalize_impl<float>(c, Y, n, q, R, stages);
 }
 
 void truncation_factors(Ctx& c, const double* s, int64_t r, int64_t chi, double cutoff, double* f,
@@ -1650,14 +1451,12 @@ __global__ void scale_columns_f32_kernel(float* x, int64_t rows, int cols, const
     x[idx] = float(double(x[idx]) * f[idx % cols]);
 }
 
-// Singular values and left singular vectors of L (q x q) given as the rows
-// of Mc (FP32): one-sided Jacobi on the columns of L^T with the rotations
-// accumulated, then sorted.  Ub (q x q FP64), S, inv_s (q).
-void jacobi_left_singular(Ctx& c, const float* Mc, int64_t q, double* Ub, double* S,
-                          double* inv_s) {
+// FP32 one-sided Jacobi on the rows of Mc (q x q): Jc (q x q) = the accumulated
+// rotations (row j: those of row j), norms = the final row norms.  *flags gets
+// bit 2 when the sweep limit is reached.
+void jacobi_rotations_impl(Ctx& c, const float* Mc, int64_t q, float* Jc, float* norms,
+                           int* flags) {
   Scope scope(c);
-  float* Jc = c.alloc<float>(size_t(q) * q);
-  float* norms = c.alloc<float>(q);
   // the Jacobi matrices stay in shared memory up to q = 160, in global
   // memory (L2) beyond
   const size_t wjac = size_t(2) * q * jacobi_ld(int(q)) * sizeof(float);
@@ -1696,7 +1495,7 @@ void jacobi_left_singular(Ctx& c, const float* Mc, int64_t q, double* Ub, double
       cfg.attrs = attr;
       cfg.numAttrs = 1;
       CTM_CUDA(cudaLaunchKernelEx(&cfg, kern, static_cast<const float*>(Mc), int(q), b, Jc, norms,
-                                  40, 4e-6f, status_flags(c)));
+                                  40, 4e-6f, flags));
     };
     switch (ldj / (4 * kPairThreads)) {
       case 3: launch(jacobi_cluster_f32_kernel<3, kPairThreads>); break;
@@ -1707,7 +1506,6 @@ void jacobi_left_singular(Ctx& c, const float* Mc, int64_t q, double* Ub, double
       default: launch(jacobi_cluster_f32_kernel<8, kPairThreads>); break;
     }
     CTM_LAUNCH_CHECK();
-    sort_singular(c.stream, Jc, norms, q, Ub, S, inv_s);
     return;
   }
   // FP32 dot products of length q carry ~sqrt(q) u relative error: 4e-6
@@ -1719,7 +1517,7 @@ void jacobi_left_singular(Ctx& c, const float* Mc, int64_t q, double* Ub, double
       CTM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(wjac)));
       KernelTimer kt(c.stream, "jacobi_onesided_f32_kernel", kUnitFlop, 0.0);
       kern<<<1, jthreads, wjac, c.stream>>>(Mc, int(q), int(pp), Jc, norms, 40, 4e-6f,
-                                           status_flags(c), nullptr);
+                                           flags, nullptr);
     };
     switch (jacobi_ld(int(q)) / 32) {
       case 1: launch(jacobi_onesided_f32_kernel<true, 1>); break;
@@ -1732,13 +1530,28 @@ void jacobi_left_singular(Ctx& c, const float* Mc, int64_t q, double* Ub, double
   } else {
     KernelTimer kt(c.stream, "jacobi_onesided_f32_kernel", kUnitFlop, 0.0);
     jacobi_onesided_f32_kernel<false, 0><<<1, jthreads, 0, c.stream>>>(
-        Mc, int(q), int(pp), Jc, norms, 40, 4e-6f, status_flags(c), Wg);
+        Mc, int(q), int(pp), Jc, norms, 40, 4e-6f, flags, Wg);
   }
   CTM_LAUNCH_CHECK();
-  sort_singular(c.stream, Jc, norms, q, Ub, S, inv_s);
+}
+
+// Singular values and left singular vectors of L (q x q) given as the rows
+// of Mc (FP32): one-sided Jacobi on the columns of L^T with the rotations
+// accumulated, then sorted.  Ub (q x q FP64), S, inv_s (q).
+void jacobi_left_singular(Ctx& c, const float* Mc, int64_t q, double* Ub, double* S,
+                          double* inv_s) {
+  Scope scope(c);
+  float* Jc = c.alloc<float>(size_t(q) * q);
+  float* norms = c.alloc<float>(q);
+  jacobi_rotations_impl(c, Mc, q, Jc, norms, c.sizing() ? nullptr : status_flags(c));
+  if (!c.sizing()) sort_singular(c.stream, Jc, norms, q, Ub, S, inv_s);
 }
 
 }  // namespace
+
+void jacobi_rotations(Ctx& c, const float* Mc, int64_t q, float* Jc, float* norms, int* flags) {
+  jacobi_rotations_impl(c, Mc, q, Jc, norms, flags);
+}
 
 void svd_via_qr(Ctx& c, const float* Bt, int64_t q, int64_t n, double* Ub, double* S, float* V) {
   CTM_REQUIRE(q >= 1 && q <= 1024 && q <= n, CTM_ERR_UNSUPPORTED,
