@@ -1,0 +1,748 @@
+// FP64 contractions as exact digit products on the tensor cores.
+//
+// GB300's FP64 units deliver 1.1 TFLOP/s and its BF16 tensor cores 1945, so an
+// FP64 product is formed from BF16 products that carry no rounding error
+// (error-free splitting after Ozaki, Ogita, Oishi and Rump, Numer. Algorithms
+// 59 (2012) 95):
+//
+//  * every row of an operand (its entries over the contracted index) is scaled
+//    by a power of two to |x| < 1, rounded to 62 fractional bits and written in
+//    eight balanced base-256 digits, each in [-128, 127] (the top one in
+//    [-64, 64]) and so exact in BF16;
+//  * the 36 products of digit i of A with digit j of B, i + j <= 7, accumulate
+//    in eight FP32 accumulators by s = i + j.  A digit product is an integer of
+//    at most 2^14 (2^13 with a top digit, 2^12 with two), so the partial sums
+//    of the groups s <= 5 over up to 192 contracted indices are integers below
+//    2^24: exact in FP32, in any order.  (Groups 6 and 7 reach 2^24.2 and
+//    2^24.4 when all digits are extreme; an error of one there is 2^-60 of the
+//    scales.)
+//  * after every 192 indices the accumulators go from tensor memory into a
+//    96-bit integer per output, and the last step rounds that integer to FP64
+//    once.
+//
+// What is dropped is the digit products with i + j >= 8, at most 7 K 2^14 /
+// 2^76 of the product of the two rows' scales and about sqrt(K) 2^-60 of it on
+// data without sign structure, against K 2^-53 (sqrt(K) 2^-54) of the entries'
+// products for a chain of FMAs: on random operands the result is 10 to 100
+// times closer to the exact one than the FMA chain's.
+//
+// A row or column with an infinity or a NaN has no digits; outputs on it are
+// formed by the FMA chain in the epilogue.
+#include <cuda_bf16.h>
+
+#include <algorithm>
+
+#include "gett.cuh"
+#include "tcgen05.cuh"
+
+namespace ctm {
+
+namespace {
+
+using bf16 = __nv_bfloat16;
+
+constexpr int kDigits = 8;
+constexpr int kBadRow = 0x40000000;  // exponent of a row with a non-finite entry
+
+// ------------------------------------------------------------- splitting
+struct SplitSide {
+  const double* x;
+  Group R;         // rows: R.m[].s0 is this operand's stride
+  Group K;
+  int k_is_s1;     // the contracted group's stride of this operand is s1 (second operand)
+  int64_t rows;
+  int kfast;       // the contracted index has unit stride (else rows are read fastest)
+  int* exps;       // rows: exponent E with |x| < 2^(E - 1023), or kBadRow
+  bf16* dig;       // [digit][row][Kp]
+};
+
+struct SplitArgs {
+  SplitSide s[2];
+  int64_t K, Kp;
+  int rb, kc;            // rows and contracted indices per CTA
+  int64_t blocks0;       // CTAs of side 0
+  int64_t kblocks;       // K blocks (1: exponents are found here)
+};
+
+__device__ __forceinline__ int exponent_field(double x) {
+  return int((unsigned long long)__double_as_longlong(x) >> 52) & 0x7ff;
+}
+
+// Loads the CTA's rows x indices block into shared memory (row stride kc + 1);
+// walks whichever index has unit stride across the lanes.
+__device__ void load_block(const SplitSide& s, const SplitArgs& a, int64_t r0, int64_t k0,
+                           double* sx, int64_t* s_ro, int64_t* s_ko) {
+  const int tid = threadIdx.x, nth = blockDim.x, lane = tid & 31, warp = tid >> 5;
+  const int nwarps = nth >> 5;
+  const int nr = int(min(int64_t(a.rb), s.rows - r0)), nk = int(min(int64_t(a.kc), a.K - k0));
+  for (int i = tid; i < nr + nk; i += nth) {
+    int64_t o0, o1;
+    if (i < nr) {
+      decode(s.R, r0 + i, o0, o1);
+      s_ro[i] = o0;
+    } else {
+      decode(s.K, k0 + i - nr, o0, o1);
+      s_ko[i - nr] = s.k_is_s1 ? o1 : o0;
+    }
+  }
+  __syncthreads();
+  const int ld = a.kc + 1;
+  if (s.kfast) {
+    for (int r = warp; r < nr; r += nwarps) {
+      const double* xr = s.x + s_ro[r];
+#pragma unroll 4
+      for (int k = lane; k < nk; k += 32) sx[r * ld + k] = xr[s_ko[k]];
+    }
+  } else {
+    const int rblocks = (nr + 31) / 32;
+#pragma unroll 4
+    for (int q = warp; q < nk * rblocks; q += nwarps) {
+      const int k = q / rblocks, r = (q - k * rblocks) * 32 + lane;
+      if (r < nr) sx[r * ld + k] = s.x[s_ro[r] + s_ko[k]];
+    }
+  }
+  __syncthreads();
+}
+
+// Largest exponent field of each row of the block, 1 at least; 2047 when an
+// entry is not finite.  Four lanes per row.
+__device__ void row_exponents(const SplitArgs& a, int nr, int nk, const double* sx, int* s_e) {
+  const int ld = a.kc + 1;
+  for (int q = threadIdx.x; q < a.rb * 4; q += blockDim.x) {
+    const int r = q >> 2;
+    int e = 1;
+    if (r < nr)
+      for (int k = q & 3; k < nk; k += 4) e = max(e, exponent_field(sx[r * ld + k]));
+    e = max(e, __shfl_xor_sync(0xffffffffu, e, 1));
+    e = max(e, __shfl_xor_sync(0xffffffffu, e, 2));
+    if ((q & 3) == 0) s_e[r] = e;
+  }
+  __syncthreads();
+}
+
+__global__ void __launch_bounds__(256) row_exponent_kernel(const SplitArgs a) {
+  extern __shared__ __align__(16) double sx[];
+  __shared__ int64_t s_ro[128], s_ko[256];
+  __shared__ int s_e[128];
+  const bool second = int64_t(blockIdx.x) >= a.blocks0;
+  const SplitSide& s = a.s[second ? 1 : 0];
+  const int64_t b = second ? int64_t(blockIdx.x) - a.blocks0 : int64_t(blockIdx.x);
+  const int64_t r0 = b / a.kblocks * a.rb, k0 = b % a.kblocks * a.kc;
+  load_block(s, a, r0, k0, sx, s_ro, s_ko);
+  const int nr = int(min(int64_t(a.rb), s.rows - r0)), nk = int(min(int64_t(a.kc), a.K - k0));
+  row_exponents(a, nr, nk, sx, s_e);
+  for (int r = threadIdx.x; r < nr; r += blockDim.x) atomicMax(s.exps + r0 + r, s_e[r]);
+}
+
+// Digit b (0..7, 0 the least significant) of the biased word w as BF16 bits in
+// the upper half: the byte minus 128, exact.
+__device__ __forceinline__ uint32_t digit_f32(uint32_t w, int byte) {
+  const uint32_t u = __byte_perm(w, 0x4B000000u, 0x7650u | uint32_t(byte));
+  return __float_as_uint(__uint_as_float(u) - 8388736.f);  // 2^23 + 128
+}
+
+__global__ void __launch_bounds__(256) split_digits_kernel(const SplitArgs a) {
+  extern __shared__ __align__(16) double sx[];
+  __shared__ int64_t s_ro[128], s_ko[256];
+  __shared__ int s_e[128];
+  const bool second = int64_t(blockIdx.x) >= a.blocks0;
+  const SplitSide& s = a.s[second ? 1 : 0];
+  const int64_t b = second ? int64_t(blockIdx.x) - a.blocks0 : int64_t(blockIdx.x);
+  const int64_t r0 = b / a.kblocks * a.rb, k0 = b % a.kblocks * a.kc;
+  load_block(s, a, r0, k0, sx, s_ro, s_ko);
+  const int nr = int(min(int64_t(a.rb), s.rows - r0)), nk = int(min(int64_t(a.kc), a.K - k0));
+  if (a.kblocks == 1) {
+    row_exponents(a, nr, nk, sx, s_e);
+    for (int r = threadIdx.x; r < nr; r += blockDim.x)
+      s.exps[r0 + r] = s_e[r] == 2047 ? kBadRow : s_e[r] + 1;
+  } else {  // row_exponent_kernel has left the largest field
+    for (int r = threadIdx.x; r < nr; r += blockDim.x) s_e[r] = max(1, s.exps[r0 + r]);
+    __syncthreads();
+  }
+  const int ld = a.kc + 1;
+  // 16-byte groups of 8 digits; two lanes cover 32 contiguous bytes of a row
+  const int ng = int((min(a.Kp - k0, int64_t(a.kc)) + 7) / 8), ng2 = (ng + 1) / 2;
+  const int64_t plane = s.rows * a.Kp;
+  for (int q = threadIdx.x; q < ng2 * a.rb * 2; q += blockDim.x) {
+    const int pair = q / (a.rb * 2), rest = q - pair * (a.rb * 2);
+    const int r = rest >> 1, g = pair * 2 + (rest & 1);
+    if (r >= nr || g >= ng) continue;
+    const int E = s_e[r] + 1;
+    uint32_t lo[8], hi[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int k = g * 8 + i;
+      const double x = k < nk ? sx[r * ld + k] : 0.0;
+      const long long bits = __double_as_longlong(x);
+      const int ex = int((unsigned long long)bits >> 52) & 0x7ff;
+      long long mant = (bits & 0xfffffffffffffll) | (ex != 0 ? 0x10000000000000ll : 0ll);
+      const int sh = max(ex, 1) - E + 10;  // x 2^62 / 2^(E - 1023) = mant 2^sh, sh <= 9
+      long long t;
+      if (sh >= 0) t = mant << sh;
+      else if (sh >= -54) t = (mant + (1ll << (-sh - 1))) >> -sh;
+      else t = 0;
+      if (bits < 0) t = -t;
+      const unsigned long long u =
+          ((unsigned long long)t + 0x0080808080808080ull) ^ 0x8000000000000000ull;
+      lo[i] = uint32_t(u);
+      hi[i] = uint32_t(u >> 32);
+    }
+    bf16* dst = s.dig + (r0 + r) * a.Kp + k0 + g * 8;
+#pragma unroll
+    for (int d = 0; d < kDigits; ++d) {  // digit 0 is the top byte
+      uint32_t w[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint32_t f0 = digit_f32(d < 4 ? hi[2 * i] : lo[2 * i], 3 - (d & 3));
+        const uint32_t f1 = digit_f32(d < 4 ? hi[2 * i + 1] : lo[2 * i + 1], 3 - (d & 3));
+        w[i] = __byte_perm(f0, f1, 0x7632);
+      }
+      *reinterpret_cast<uint4*>(dst + int64_t(d) * plane) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+  }
+}
+
+// The exponents that row_exponent_kernel leaves (largest field, 2047 for
+// non-finite) in the form the products read.
+__global__ void finish_exponents_kernel(int* exps, int64_t n) {
+  const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  if (i < n) {
+    const int e = max(1, exps[i]);
+    exps[i] = e == 2047 ? kBadRow : e + 1;
+  }
+}
+
+// ------------------------------------------------------------- products
+constexpr int kM = 128;             // rows per tile (tensor-memory lanes)
+constexpr int kStageK = 32;         // contracted indices per stage (64-byte rows)
+constexpr int kStages = 2;
+constexpr int kChunkStages = 6;     // stages between two reads of the accumulators
+constexpr int kDThreads = 384;      // producer, MMA issuer, two idle warps, eight epilogue warps
+constexpr uint32_t kABytes = kDigits * kM * kStageK * 2;
+
+struct DigitArgs {
+  int64_t M, N, K;      // rows, columns, contracted
+  Group GM, GN;         // output strides of rows and columns (m[].s1)
+  const int* ea;
+  const int* eb;
+  double* C;            // C, or the split-K partials
+  int64_t ldm, ldn;     // partial sums: strides of rows and columns (split > 1)
+  int64_t part_stride;
+  double alpha, beta;
+  int ntile, m_tiles, n_tiles, tiles, n_fast;
+  int split;            // K ranges
+  int stages_per_split; // multiple of kChunkStages
+  int stages_total;
+  int* status;
+  // operands, for rows and columns without digits
+  const double* a;
+  const double* b;
+  Group FM, FN, FK;     // FM.m[].s0, FN.m[].s0, FK: (row operand, column operand) strides
+  int swapped;          // the row operand is the contraction's second one
+};
+
+// (hi 2^32 + lo) 2^e rounded to nearest even.
+__device__ __forceinline__ double round_96(long long hi, uint32_t lo, int e) {
+  const bool neg = hi < 0;
+  if (neg) {
+    lo = 0u - lo;
+    hi = ~hi + (lo == 0u ? 1 : 0);
+  }
+  if (hi == 0 && lo == 0u) return 0.0;
+  const int lz = hi != 0 ? __clzll(hi) : 64 + __clz(int(lo));
+  unsigned long long m;
+  uint32_t rest = 0u;
+  if (lz >= 64) {
+    m = (unsigned long long)lo << (lz - 32);
+  } else if (lz >= 32) {
+    m = ((unsigned long long)hi << lz) | ((unsigned long long)lo << (lz - 32));
+  } else {
+    m = ((unsigned long long)hi << lz) | (((unsigned long long)lo << lz) >> 32);
+    rest = lo << lz;
+  }
+  unsigned long long r = m >> 11;  // 53 bits
+  const uint32_t low = uint32_t(m) & 0x7ffu;
+  if (low > 0x400u || (low == 0x400u && (rest != 0u || (r & 1ull) != 0ull))) ++r;
+  const int ef = 95 - lz + e + 1023;  // exponent field of the leading bit
+  double v;
+  if (ef >= 1 && ef < 2046)
+    v = __longlong_as_double((long long)(((unsigned long long)(ef - 1) << 52) + r));
+  else  // overflow and gradual underflow
+    v = scalbn(double((long long)r), ef - 1023 - 52);
+  return neg ? -v : v;
+}
+
+// One output by the FMA chain, for rows and columns with non-finite entries.
+__device__ __noinline__ double chain_dot(const DigitArgs& p, int64_t m, int64_t n, int64_t k0,
+                                         int64_t k1) {
+  int64_t mo, no, t0, t1;
+  decode(p.FM, m, mo, t0);
+  decode(p.FN, n, no, t0);
+  double v = 0.0;
+  for (int64_t k = k0; k < k1; ++k) {
+    decode(p.FK, k, t0, t1);
+    v = fma(p.a[mo + (p.swapped ? t1 : t0)], p.b[no + (p.swapped ? t0 : t1)], v);
+  }
+  return v;
+}
+
+__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z,
+                                            uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(smem_u32(dst)),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
+      : "memory");
+}
+
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, float (&v)[4]) {
+  uint32_t r[4];
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(taddr));
+#pragma unroll
+  for (int i = 0; i < 4; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// Integer value of f, |f| < 2^22 (an FP32 addition; the conversion unit does
+// 16 values per cycle and SM, these adders 128).
+__device__ __forceinline__ int int_small(float f) {
+  return __float_as_int(f + 12582912.f) - 0x4B400000;
+}
+// The same for |f| < 2^25: multiples of 8 and the rest.
+__device__ __forceinline__ int int_wide(float f) {
+  const float t = f + 100663296.f;  // 1.5 2^26: unit 8
+  const float r = f - (t - 100663296.f);
+  return 8 * (__float_as_int(t) - 0x4CC00000) + int_small(r);
+}
+
+// Tiles of 128 rows x ntile columns, persistent over blockIdx.x.  The eight
+// accumulators of a tile fill tensor memory (8 x 64 columns).  One stage holds
+// 32 contracted indices of all eight digits of both operands (64 + 32 KB, two
+// stages), loaded by two TMA copies; for digit i of A the digits j = 0..7-i of
+// B are adjacent rows of one operand whose products fall into adjacent
+// accumulators, so 12 MMAs of up to 256 columns do the 36 products of 16
+// indices.  Warp 0 lane 0 loads, warp 1 lane 0 issues, warps 4-11 read tensor
+// memory (warp w: lanes 32 (w % 4).., half (w - 4) / 4 of the columns).
+template <int kHalf>
+__global__ void __launch_bounds__(kDThreads, 1)
+    digit_gemm_kernel(const __grid_constant__ CUtensorMap tA,
+                      const __grid_constant__ CUtensorMap tB, const DigitArgs p) {
+  extern __shared__ uint8_t dyn_smem[];
+  uint8_t* base = reinterpret_cast<uint8_t*>(
+      (reinterpret_cast<uintptr_t>(dyn_smem) + 1023) & ~uintptr_t(1023));
+  constexpr int NT = 2 * kHalf;
+  constexpr uint32_t b_bytes = uint32_t(kDigits) * NT * kStageK * 2;
+  constexpr uint32_t stage_bytes = kABytes + b_bytes;
+  uint64_t* full = reinterpret_cast<uint64_t*>(base + size_t(kStages) * stage_bytes);
+  uint64_t* empty = full + kStages;
+  uint64_t* tfull = empty + kStages;
+  uint64_t* tempty = tfull + 1;
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(tempty + 1);
+  __shared__ int s_fail, s_epi_fail[2];
+  __shared__ int64_t s_cn[2][NT];
+  __shared__ int s_eb[2][NT];
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    s_fail = 0;
+    s_epi_fail[0] = s_epi_fail[1] = 0;
+    for (int s = 0; s < kStages; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    mbar_init(tfull, 1);
+    mbar_init(tempty, 8);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_u32(tmem_holder)),
+                 "r"(512u)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_holder;
+  const int work = p.tiles * p.split;
+  // item -> tile origin and stage range
+  auto item = [&](int it, int& m0, int& n0, int& s0, int& s1, int& sp) {
+    sp = it / p.tiles;
+    const int t = it - sp * p.tiles;
+    int mt, nt;
+    if (p.n_fast) {
+      mt = t / p.n_tiles;
+      nt = t - mt * p.n_tiles;
+    } else {
+      nt = t / p.m_tiles;
+      mt = t - nt * p.m_tiles;
+    }
+    m0 = mt * kM;
+    n0 = nt * NT;
+    s0 = sp * p.stages_per_split;
+    s1 = min(p.stages_total, s0 + p.stages_per_split);
+  };
+  int issued = 0;
+  if (threadIdx.x == 0) {
+    // ---------------- TMA producer
+    int g = 0;
+    bool fail = false;
+    for (int it = blockIdx.x; it < work && !fail; it += gridDim.x) {
+      int m0, n0, s0, s1, sp;
+      item(it, m0, n0, s0, s1, sp);
+      for (int s = s0; s < s1; ++s, ++g) {
+        const int st = g % kStages;
+        if (!mbar_wait_spin(&empty[st], ((g / kStages) & 1) ^ 1)) {
+          atomicOr(&s_fail, 1);
+          fail = true;
+          break;
+        }
+        uint8_t* sm = base + size_t(st) * stage_bytes;
+        mbar_expect_tx(&full[st], stage_bytes);
+        tma_load_3d(sm, &tA, s * kStageK, m0, 0, &full[st]);
+        tma_load_3d(sm + kABytes, &tB, s * kStageK, n0, 0, &full[st]);
+        issued = g + 1;
+      }
+    }
+  } else if (threadIdx.x == 32) {
+    // ---------------- MMA issuer
+    int g = 0, chunk = 0;
+    bool fail = false;
+    for (int it = blockIdx.x; it < work && !fail; it += gridDim.x) {
+      int m0, n0, s0, s1, sp;
+      item(it, m0, n0, s0, s1, sp);
+      for (int s = s0; s < s1; ++s, ++g) {
+        const bool first = (s - s0) % kChunkStages == 0;
+        if (first && !mbar_wait_spin(tempty, (chunk & 1) ^ 1)) {
+          atomicOr(&s_fail, 1);
+          fail = true;
+          break;
+        }
+        const int st = g % kStages;
+        if (!mbar_wait_spin(&full[st], (g / kStages) & 1)) {
+          atomicOr(&s_fail, 1);
+          fail = true;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint64_t da = smem_desc(base + size_t(st) * stage_bytes, kStageK);
+        const uint64_t db = smem_desc(base + size_t(st) * stage_bytes + kABytes, kStageK);
+        const int steps = p.K - int64_t(s) * kStageK > 16 ? 2 : 1;
+        for (int kk = 0; kk < steps; ++kk) {
+#pragma unroll
+          for (int i = 0; i < kDigits; ++i) {
+            constexpr int kGroup = 256 / NT;  // digits of B per MMA
+#pragma unroll
+            for (int j = 0; j < kDigits - i; j += kGroup) {
+              const int cnt = min(kGroup, kDigits - i - j);
+              mma_bf16(tmem + uint32_t((i + j) * NT),
+                       da + uint64_t((i * kM * kStageK * 2 + kk * 32) >> 4),
+                       db + uint64_t((j * NT * kStageK * 2 + kk * 32) >> 4),
+                       idesc_bf16(kM, cnt * NT), (first && kk == 0 && i == 0) ? 0u : 1u);
+            }
+          }
+        }
+        mma_commit(&empty[st]);
+        if ((s - s0) % kChunkStages == kChunkStages - 1 || s == s1 - 1) {
+          mma_commit(tfull);
+          ++chunk;
+        }
+      }
+    }
+  } else if (warp >= 4) {
+    // ---------------- epilogue
+    const int etid = threadIdx.x - 128;
+    const int lane_base = (warp & 3) * 32, half = (warp - 4) >> 2;
+    const uint32_t trow = tmem + (uint32_t(lane_base) << 16) + uint32_t(half * kHalf);
+    int chunk = 0, par = 0;
+    for (int it = blockIdx.x; it < work; it += gridDim.x, par ^= 1) {
+      int m0, n0, s0, s1, sp;
+      item(it, m0, n0, s0, s1, sp);
+      for (int c = etid; c < NT; c += 256) {
+        const int64_t n = int64_t(n0) + c;
+        int64_t off = -1, t;
+        int e = 0;
+        if (n < p.N) {
+          if (p.split > 1) off = n * p.ldn;
+          else decode(p.GN, n, t, off);
+          e = p.eb[n];
+        }
+        s_cn[par][c] = off;
+        s_eb[par][c] = e;
+      }
+      const int64_t row = int64_t(m0) + lane_base + lane;
+      int64_t ro = 0, t0;
+      int er = 0;
+      if (row < p.M) {
+        if (p.split > 1) ro = row * p.ldm + sp * p.part_stride;
+        else decode(p.GM, row, t0, ro);
+        er = p.ea[row];
+      }
+      long long hi[kHalf];
+      uint32_t lo[kHalf];
+#pragma unroll
+      for (int j = 0; j < kHalf; ++j) {
+        hi[j] = 0;
+        lo[j] = 0u;
+      }
+      const int chunks = (s1 - s0 + kChunkStages - 1) / kChunkStages;
+      bool lost = false;
+      for (int ch = 0; ch < chunks; ++ch, ++chunk) {
+        bool ok = mbar_wait(tfull, chunk & 1);
+        __syncwarp();
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) {
+          lost = true;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+        for (int c = 0; c < kHalf; c += 4) {
+          float f[kDigits][4];
+#pragma unroll
+          for (int s = 0; s < kDigits; ++s) tmem_ld4(trow + uint32_t(s * NT + c), f[s]);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          // the loaded registers are valid only after the wait
+#pragma unroll
+          for (int s = 0; s < kDigits; ++s)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) asm volatile("" : "+f"(f[s][j]));
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int g01 = int_small(f[0][j]) * 256 + int_small(f[1][j]);
+            const int g23 = int_wide(f[2][j]) * 256 + int_wide(f[3][j]);
+            const long long h = (long long)g01 * 65536 + g23;
+            long long l = (long long)int_wide(f[4][j]) * 16777216 + lo[c + j];
+            l += (long long)__float2int_rn(f[5][j]) * 65536;
+            l += (long long)__float2int_rn(f[6][j]) * 256;
+            l += __float2int_rn(f[7][j]);
+            lo[c + j] = uint32_t(l);
+            hi[c + j] += h + (l >> 32);
+          }
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        if (lane == 0) mbar_arrive(tempty);
+      }
+      // all eight warps arrive and decide together (a flag per parity: a warp
+      // already at the next item cannot change this one's)
+      if (lost && lane == 0) s_epi_fail[par] = 1;
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      if (s_epi_fail[par]) {
+        if (etid == 0) atomicOr(&s_fail, 1);
+        break;
+      }
+      if (row < p.M) {
+        double* out = p.C + ro;
+        const int64_t k0 = int64_t(s0) * kStageK, k1 = min(p.K, int64_t(s1) * kStageK);
+#pragma unroll
+        for (int c = 0; c < kHalf; ++c) {
+          const int64_t off = s_cn[par][half * kHalf + c];
+          const int e = s_eb[par][half * kHalf + c];
+          if (off < 0) continue;
+          // units of 2^-68 of the scales (digit s of the product: 2^(-12 - 8 s))
+          double v;
+          if (((er | e) & kBadRow) != 0) v = chain_dot(p, row, int64_t(n0) + half * kHalf + c, k0, k1);
+          else v = round_96(hi[c], lo[c], er + e - 2 * 1023 - 68);
+          if (p.split == 1 && !(p.alpha == 1.0 && p.beta == 0.0)) {
+            v *= p.alpha;
+            if (p.beta != 0.0) v = fma(p.beta, out[off], v);
+          }
+          out[off] = v;
+        }
+      }
+    }
+  }
+  __syncwarp();
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  // on failure: let in-flight copies land before the CTA's memory goes away
+  if (threadIdx.x == 0 && s_fail) {
+    for (int i = max(0, issued - kStages); i < issued; ++i)
+      (void)mbar_wait(&full[i % kStages], (i / kStages) & 1);
+    atomicOr(p.status, 2);
+  }
+  __syncthreads();
+  if (warp == 0) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u)
+                 : "memory");
+  }
+}
+
+void digit_map(CUtensorMap* map, const bf16* dig, int64_t rows, int64_t Kp, uint32_t box_rows) {
+  const cuuint64_t dims[3] = {cuuint64_t(Kp), cuuint64_t(rows), cuuint64_t(kDigits)};
+  const cuuint64_t strides[2] = {cuuint64_t(Kp) * 2, cuuint64_t(rows) * cuuint64_t(Kp) * 2};
+  const cuuint32_t box[3] = {uint32_t(kStageK), box_rows, uint32_t(kDigits)};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  const CUresult res = encode_tiled()(
+      map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<bf16*>(dig), dims, strides, box, estr,
+      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
+      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  CTM_REQUIRE(res == CUDA_SUCCESS, CTM_ERR_CUDA,
+              "cuTensorMapEncodeTiled failed with code " + std::to_string(int(res)));
+}
+
+// Cycles of one stage of a tile of ntile columns: 36 products of 32 indices
+// at 4096 multiply-adds per cycle, or its bytes at about 45 per cycle and SM.
+double stage_cycles(int ntile) {
+  return std::max(36.0 * ntile, (65536.0 + 512.0 * ntile) / 45.0);
+}
+
+int best_ntile(int64_t n) {
+  int best = 64;
+  double least = 1e300;
+  for (int t : {64, 48, 32, 16}) {
+    const double cost = double((n + t - 1) / t) * stage_cycles(t);
+    if (cost < least) {
+      least = cost;
+      best = t;
+    }
+  }
+  return best;
+}
+
+bool unit_stride(const Group& g, bool second) {
+  return g.n > 0 && (second ? g.m[g.n - 1].s1 : g.m[g.n - 1].s0) == 1;
+}
+
+}  // namespace
+
+// From about 2e7 multiply-adds on the digit form is the faster one: 256^3 takes
+// 40 us in the FP64 GETT, 400^3 (6.4e7) 70 us in digits and about 150 in the
+// GETT; 5184 x 5184 x 144 takes 0.33 ms against 11 ms.
+bool digits_pay(const GettArgs<double>& p) {
+  if (p.bext != 1 || p.Kt < 1) return false;
+  const double mnk = double(p.Mt) * double(p.Nt) * double(p.Kt);
+  return mnk >= 2.0e7 && p.Kt >= 16 && std::min(p.Mt, p.Nt) >= 16;
+}
+
+void digit_contract(Ctx& c, const GettArgs<double>& p) {
+  const int64_t K = p.Kt, Kp = (K + 7) / 8 * 8;
+  const int sms = sm_count_linalg();
+  // which operand's rows lie on the tensor-memory lanes: fewer waves of tiles,
+  // and when equal the one whose rows are contiguous in C (a warp stores one
+  // column of 32 rows)
+  auto waves = [&](int64_t m, int64_t n) {
+    const int nt = best_ntile(n);
+    const int64_t tiles = (m + kM - 1) / kM * ((n + nt - 1) / nt);
+    return double((tiles + sms - 1) / sms) * stage_cycles(nt);
+  };
+  const double w0 = waves(p.Mt, p.Nt), w1 = waves(p.Nt, p.Mt);
+  const bool swap = w1 < 0.98 * w0 || (w1 <= 1.02 * w0 && unit_stride(p.M, true) < unit_stride(p.N, true));
+  const int64_t M = swap ? p.Nt : p.Mt, N = swap ? p.Mt : p.Nt;
+  const int nt = best_ntile(N);
+  Scope scope(c);
+  bf16* da = c.alloc<bf16>(size_t(kDigits) * M * Kp);
+  bf16* db = c.alloc<bf16>(size_t(kDigits) * N * Kp);
+  int* ex = c.alloc<int>(size_t(M + N));
+  const int64_t m_tiles = (M + kM - 1) / kM, n_tiles = (N + nt - 1) / nt;
+  const int64_t tiles = m_tiles * n_tiles;
+  const int64_t stages = (K + kStageK - 1) / kStageK;
+  // K ranges when the tiles leave most SMs idle; at least two reads of the
+  // accumulators' worth of stages each
+  int64_t split = 1;
+  if (tiles * 2 <= sms) split = std::min<int64_t>(sms / tiles, stages / (2 * kChunkStages));
+  split = std::max<int64_t>(split, 1);
+  int64_t per = (stages + split - 1) / split;
+  per = (per + kChunkStages - 1) / kChunkStages * kChunkStages;
+  split = (stages + per - 1) / per;
+  double* part = split > 1 ? c.alloc<double>(size_t(split) * p.Mt * p.Nt) : nullptr;
+  if (c.sizing()) return;
+  CTM_REQUIRE(tiles * split < (int64_t(1) << 31), CTM_ERR_UNSUPPORTED, "einsum: grid too large");
+
+  SplitArgs sa{};
+  auto side = [&](SplitSide& s, bool first, int64_t rows, int* exps, bf16* dig) {
+    s.x = first ? p.A : p.B;
+    s.R = first ? p.M : p.N;
+    s.K = p.K;
+    s.k_is_s1 = first ? 0 : 1;
+    s.rows = rows;
+    s.kfast = unit_stride(p.K, !first) && !unit_stride(s.R, false) ? 1 : 0;
+    s.exps = exps;
+    s.dig = dig;
+  };
+  side(sa.s[0], !swap, M, ex, da);
+  side(sa.s[1], swap, N, ex + M, db);
+  sa.K = K;
+  sa.Kp = Kp;
+  sa.kblocks = (K + 255) / 256;
+  sa.kc = int(sa.kblocks == 1 ? Kp : 256);
+  sa.rb = sa.kc <= 64 ? 128 : sa.kc <= 128 ? 64 : 32;
+  sa.blocks0 = (M + sa.rb - 1) / sa.rb * sa.kblocks;
+  const int64_t blocks = sa.blocks0 + (N + sa.rb - 1) / sa.rb * sa.kblocks;
+  const size_t ssm = size_t(sa.rb) * (sa.kc + 1) * sizeof(double);
+  if (sa.kblocks > 1) {
+    CTM_CUDA(cudaMemsetAsync(ex, 0, sizeof(int) * size_t(M + N), c.stream));
+    CTM_CUDA(cudaFuncSetAttribute(row_exponent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ssm)));
+    KernelTimer kt(c.stream, "row_exponent_kernel", kUnitByte, 8.0 * double(M + N) * K);
+    row_exponent_kernel<<<unsigned(blocks), 256, ssm, c.stream>>>(sa);
+    CTM_LAUNCH_CHECK();
+  }
+  {
+    CTM_CUDA(cudaFuncSetAttribute(split_digits_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ssm)));
+    KernelTimer kt(c.stream, "split_digits_kernel", kUnitByte, 24.0 * double(M + N) * K);
+    split_digits_kernel<<<unsigned(blocks), 256, ssm, c.stream>>>(sa);
+    CTM_LAUNCH_CHECK();
+  }
+  if (sa.kblocks > 1) {
+    finish_exponents_kernel<<<unsigned((M + N + 255) / 256), 256, 0, c.stream>>>(ex, M + N);
+    CTM_LAUNCH_CHECK();
+  }
+
+  DigitArgs d{};
+  d.M = M;
+  d.N = N;
+  d.K = K;
+  d.GM = swap ? p.N : p.M;
+  d.GN = swap ? p.M : p.N;
+  d.ea = ex;
+  d.eb = ex + M;
+  d.C = split > 1 ? part : p.C;
+  d.ldm = swap ? 1 : p.Nt;
+  d.ldn = swap ? p.Nt : 1;
+  d.part_stride = p.Mt * p.Nt;
+  d.alpha = p.alpha;
+  d.beta = p.beta;
+  d.ntile = nt;
+  d.m_tiles = int(m_tiles);
+  d.n_tiles = int(n_tiles);
+  d.tiles = int(tiles);
+  d.n_fast = N <= M ? 1 : 0;
+  d.split = int(split);
+  d.stages_per_split = int(per);
+  d.stages_total = int(stages);
+  d.status = status_flags(c);
+  d.a = swap ? p.B : p.A;
+  d.b = swap ? p.A : p.B;
+  d.FM = d.GM;
+  d.FN = d.GN;
+  d.FK = p.K;
+  d.swapped = swap ? 1 : 0;
+  CUtensorMap tA, tB;
+  digit_map(&tA, da, M, Kp, kM);
+  digit_map(&tB, db, N, Kp, uint32_t(nt));
+  const size_t smem = 1024 + size_t(kStages) * (kABytes + size_t(kDigits) * nt * kStageK * 2) + 128;
+  const unsigned grid = unsigned(std::min<int64_t>(tiles * split, sms));
+  auto launch = [&](auto kern) {
+    CTM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    const double flops = 2.0 * double(M) * N * K;
+    KernelTimer timer(c.stream, kTagGettF64, flops);
+    KernelTimer kt(c.stream, "digit_gemm_kernel", kUnitFlop, flops);
+    kern<<<grid, kDThreads, smem, c.stream>>>(tA, tB, d);
+  };
+  if (nt == 64) launch(digit_gemm_kernel<32>);
+  else if (nt == 48) launch(digit_gemm_kernel<24>);
+  else if (nt == 32) launch(digit_gemm_kernel<16>);
+  else launch(digit_gemm_kernel<8>);
+  CTM_LAUNCH_CHECK();
+  if (split > 1) {
+    GettArgs<double> r = p;
+    r.splitk = int(split);
+    r.part = part;
+    splitk_reduce(c, r);
+  }
+}
+
+}  // namespace ctm

@@ -8,63 +8,15 @@
 // merges modes that are adjacent in every operand, and launches one kernel
 // whose tile loaders decode multi-mode indices into strided addresses.
 #include "engine.cuh"
+#include "gett.cuh"
 
 #include <algorithm>
 #include <map>
+#include <type_traits>
 
 namespace ctm {
 
 namespace {
-
-constexpr int kMaxModes = 4;
-
-struct Mode {
-  int64_t ext;
-  int64_t s0;  // stride in the first operand of the pair
-  int64_t s1;  // stride in the second operand of the pair
-};
-
-struct Group {
-  int n;
-  Mode m[kMaxModes];
-};
-
-template <class T>
-struct GettArgs {
-  const T* A;
-  const T* B;
-  T* C;
-  Group M, N, K;  // M: (A, C) strides, N: (B, C), K: (A, B)
-  int64_t Mt, Nt, Kt;
-  int64_t bext, bsa, bsb, bsc;
-  T alpha, beta;
-  int splitk;
-  int64_t kchunk;
-  T* part;
-  int kfa, kfb;  // tile loaders walk K fastest (K is the unit-stride mode of A / B)
-  int swap_xy;   // grid x runs over column tiles (more than 65535 of them)
-};
-
-// Group index -> the two operands' offsets.  Decoded in 32-bit arithmetic
-// (every group's extent is below 2^31, checked on the host): a 64-bit
-// division by a run-time divisor is a long software sequence, and the tile
-// loaders decode 16 K indices per step.
-__device__ __forceinline__ void decode(const Group& g, int64_t idx, int64_t& o0, int64_t& o1) {
-  o0 = 0;
-  o1 = 0;
-  uint32_t rem = uint32_t(idx);
-#pragma unroll
-  for (int j = kMaxModes - 1; j >= 0; --j) {
-    if (j < g.n) {
-      const uint32_t e = uint32_t(g.m[j].ext);
-      const uint32_t q = rem / e;
-      const int64_t r = int64_t(rem - q * e);
-      rem = q;
-      o0 += r * g.m[j].s0;
-      o1 += r * g.m[j].s1;
-    }
-  }
-}
 
 constexpr int BM = 64, BN = 64, BK = 16, NT = 256;
 
@@ -354,6 +306,16 @@ int64_t group_size(const Group& g) {
 }  // namespace
 
 template <class T>
+void splitk_reduce_impl(Ctx& c, const GettArgs<T>& p) {
+  KernelTimer kt(c.stream, "gett_splitk_reduce", kUnitByte,
+                 double(sizeof(T)) * (p.splitk + 1.0) * p.bext * p.Mt * p.Nt);
+  gett_splitk_reduce<T><<<grid_for(p.bext * p.Mt * p.Nt, 256), 256, 0, c.stream>>>(p);
+  CTM_LAUNCH_CHECK();
+}
+
+void splitk_reduce(Ctx& c, const GettArgs<double>& p) { splitk_reduce_impl<double>(c, p); }
+
+template <class T>
 void einsum_impl(Ctx& c, const char* spec, const ViewT<T>& A, const ViewT<T>& B, const ViewT<T>& C,
                  double alpha, double beta) {
   std::string s(spec);
@@ -472,6 +434,12 @@ void einsum_impl(Ctx& c, const char* spec, const ViewT<T>& A, const ViewT<T>& B,
     CTM_LAUNCH_CHECK();
     return;
   }
+  if constexpr (std::is_same<T, double>::value) {
+    if (digits_pay(p)) {
+      digit_contract(c, p);
+      return;
+    }
+  }
   const int64_t tiles = ((p.Mt + BM - 1) / BM) * ((p.Nt + BN - 1) / BN) * bext;
   int splitk = 1;
   // split K until the grid holds about one CTA per SM: two per SM measured
@@ -503,12 +471,7 @@ void einsum_impl(Ctx& c, const char* spec, const ViewT<T>& A, const ViewT<T>& B,
     gett_kernel<T><<<grid, NT, 0, c.stream>>>(p);
     CTM_LAUNCH_CHECK();
   }
-  if (splitk > 1) {
-    KernelTimer kt(c.stream, "gett_splitk_reduce", kUnitByte,
-                   double(sizeof(T)) * (splitk + 1.0) * bext * p.Mt * p.Nt);
-    gett_splitk_reduce<T><<<grid_for(bext * p.Mt * p.Nt, 256), 256, 0, c.stream>>>(p);
-    CTM_LAUNCH_CHECK();
-  }
+  if (splitk > 1) splitk_reduce_impl<T>(c, p);
 }
 
 void einsum(Ctx& c, const char* spec, const View& A, const View& B, const View& C, double alpha,

@@ -22,6 +22,7 @@
 
 #include "engine.cuh"
 #include "tc_gemm.cuh"
+#include "tcgen05.cuh"
 
 namespace ctm {
 
@@ -33,131 +34,6 @@ constexpr int kBM = 128;         // rows of A per CTA (MMA M)
 constexpr int kThreads = 256;    // 8 warps: in the epilogue warp w reads TMEM lanes
                                  // 32 (w % 4) .. +31 for half (w / 4) of the columns
 constexpr uint32_t kTmemCols = 256;
-constexpr int64_t kSpinLimit = 4LL * 1000 * 1000;
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count)
-               : "memory");
-}
-
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
-               "r"(bytes)
-               : "memory");
-}
-
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t done;
-  asm volatile(
-      "{\n"
-      " .reg .pred P1;\n"
-      " mbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n"
-      " selp.b32 %0, 1, 0, P1;\n"
-      "}\n"
-      : "=r"(done)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return done != 0;
-}
-
-__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t done;
-  asm volatile(
-      "{\n"
-      " .reg .pred P1;\n"
-      " mbarrier.test_wait.parity.shared::cta.b64 P1, [%1], %2;\n"
-      " selp.b32 %0, 1, 0, P1;\n"
-      "}\n"
-      : "=r"(done)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return done != 0;
-}
-
-// Bounded wait of the single producer / MMA thread on a pipeline barrier:
-// a non-blocking test in a tight loop (no suspension, so the thread resumes
-// as soon as the phase flips); gives up after about 0.1 s.
-__device__ __forceinline__ bool mbar_wait_spin(uint64_t* bar, uint32_t parity) {
-  for (int64_t i = 0; i < 8 * kSpinLimit; ++i)
-    if (mbar_test_wait(bar, parity)) return true;
-  return false;
-}
-
-// Bounded wait on an mbarrier phase; false when the limit expired.  Polls
-// without sleeping for the first few thousand tries (a pipeline stage turns
-// over in about a microsecond), then backs off.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
-  for (int64_t i = 0; i < kSpinLimit; ++i) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if (i > 4096) __nanosleep(64);
-  }
-  return false;
-}
-
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y,
-                                            uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(bar))
-      : "memory");
-}
-
-// Shared-memory matrix descriptor: K-major operand with rows of bk BF16
-// (bk = 64: 128-byte swizzle; bk = 32: 64-byte swizzle), 8-row core-matrix
-// groups 8 * 2 * bk bytes apart.
-__device__ __forceinline__ uint64_t smem_desc(const void* p, int bk) {
-  const uint64_t addr = smem_u32(p);
-  uint64_t d = (addr >> 4) & 0x3FFFull;              // start address
-  d |= uint64_t(1) << 16;                            // leading byte offset (unused when swizzled)
-  d |= uint64_t((16 * bk) >> 4) << 32;               // stride byte offset
-  d |= uint64_t(1) << 46;                            // descriptor version (tcgen05)
-  d |= uint64_t(bk == 64 ? 2 : 4) << 61;             // SWIZZLE_128B / SWIZZLE_64B
-  return d;
-}
-
-// Instruction descriptor of kind::f16: FP32 accumulator, BF16 A and B,
-// both K-major, shape M x N.
-__host__ __device__ constexpr uint32_t idesc_bf16(int m, int n) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(n >> 3) << 17) | (uint32_t(m >> 4) << 24);
-}
-
-__device__ __forceinline__ void mma_bf16(uint32_t tmem, uint64_t a, uint64_t b, uint32_t idesc,
-                                         uint32_t accumulate) {
-  asm volatile(
-      "{\n"
-      " .reg .pred p;\n"
-      " setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
-      "}\n" ::"r"(tmem),
-      "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-__device__ __forceinline__ void mma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                   smem_u32(bar))
-               : "memory");
-}
-
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
-  uint32_t r[16];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
-}
-
 // Row / column offsets of a separable layout.  The indices are decoded in
 // 32-bit arithmetic (M and N are below 2^31, checked at launch; a 64-bit
 // division by a run-time divisor is a long software sequence, and the
@@ -467,10 +343,6 @@ __global__ void __launch_bounds__(kThreads, 1)
                  "r"(kTmemCols)
                  : "memory");
   }
-}
-
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
 __device__ __forceinline__ void epi_bar_sync() {
@@ -924,27 +796,6 @@ __global__ void split_bf16_kernel(const S* src, int64_t rows, int64_t cols, int6
       if (lo != nullptr) lo[c * ld_dst + r] = l;
     }
   }
-}
-
-// cuTensorMapEncodeTiled through the runtime's driver entry point, so the
-// library does not link libcuda (it still loads on machines without a driver).
-using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
-                                   const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                   const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_tiled() {
-  static EncodeTiledFn fn = nullptr;
-  if (fn == nullptr) {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q{};
-    CTM_CUDA(cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000,
-                                              cudaEnableDefault, &q));
-    CTM_REQUIRE(p != nullptr && q == cudaDriverEntryPointSuccess, CTM_ERR_CUDA,
-                "cuTensorMapEncodeTiled is not available from the driver");
-    fn = reinterpret_cast<EncodeTiledFn>(p);
-  }
-  return fn;
 }
 
 void make_map(CUtensorMap* map, const bf16* ptr, int64_t rows, int64_t k, int64_t ld,
