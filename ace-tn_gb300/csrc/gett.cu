@@ -18,15 +18,16 @@ namespace ctm {
 
 namespace {
 
-constexpr int BM = 64, BN = 64, BK = 16, NT = 256;
+constexpr int BK = 16, NT = 256;
 
-// One 64x64 output tile per CTA, 4x4 outputs per thread, K staged through
-// shared memory 16 at a time with a register prefetch of the next step (its
-// global loads are in flight while the current step computes).  Each tile
+// One output tile of 16 kT x 16 kT per CTA, kT x kT outputs per thread, K staged
+// through shared memory 16 at a time with a register prefetch of the next step
+// (its global loads are in flight while the current step computes).  Each tile
 // loader walks whichever of its two index groups has unit stride, so warps
 // read contiguous memory for either operand orientation.
-template <class T>
+template <class T, int kT>
 __global__ void __launch_bounds__(NT) gett_kernel(const GettArgs<T> p) {
+  constexpr int BM = 16 * kT, BN = 16 * kT;
   __shared__ int64_t sAm[BM], sCm[BM], sBn[BN], sCn[BN];
   __shared__ int64_t sAk[2][BK], sBk[2][BK];
   __shared__ T As[BK][BM + 1];
@@ -86,11 +87,11 @@ __global__ void __launch_bounds__(NT) gett_kernel(const GettArgs<T> p) {
     }
   };
 
-  T acc[4][4];
+  T acc[kT][kT];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < kT; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = T(0);
+    for (int j = 0; j < kT; ++j) acc[i][j] = T(0);
 
   const int tx = tid & 15, ty = tid >> 4;
   decode_k(0, 0);
@@ -113,25 +114,25 @@ __global__ void __launch_bounds__(NT) gett_kernel(const GettArgs<T> p) {
     decode_k(st + 2, st & 1);  // buffer st & 1 was last read by load(st)
 #pragma unroll
     for (int kk = 0; kk < BK; ++kk) {
-      T a[4], b[4];
+      T a[kT], b[kT];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[kk][ty + 16 * i];
+      for (int i = 0; i < kT; ++i) a[i] = As[kk][ty + 16 * i];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tx + 16 * j];
+      for (int j = 0; j < kT; ++j) b[j] = Bs[kk][tx + 16 * j];
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < kT; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
+        for (int j = 0; j < kT; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
     }
   }
 
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < kT; ++i) {
     const int mi = ty + 16 * i;
     const int64_t m = m0 + mi;
     if (m >= p.Mt) continue;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < kT; ++j) {
       const int nj = tx + 16 * j;
       const int64_t n = n0 + nj;
       if (n >= p.Nt) continue;
@@ -440,15 +441,44 @@ void einsum_impl(Ctx& c, const char* spec, const ViewT<T>& A, const ViewT<T>& B,
       return;
     }
   }
-  const int64_t tiles = ((p.Mt + BM - 1) / BM) * ((p.Nt + BN - 1) / BN) * bext;
-  int splitk = 1;
-  // split K until the grid holds about one CTA per SM: two per SM measured
-  // slower in the concurrent move (the CTAs of other rows' kernels share the
-  // SMs; the split-K partials double), far fewer lengthens the row
-  const int64_t target = sm_count_linalg();
-  if (tiles < target && p.Kt >= 2 * BK) {
-    splitk = static_cast<int>(std::min<int64_t>((target + tiles - 1) / tiles, p.Kt / BK));
-    splitk = std::max(splitk, 1);
+  const int64_t sms = sm_count_linalg();
+  auto tiles_of = [&](int t) {
+    return ((p.Mt + 16 * t - 1) / (16 * t)) * ((p.Nt + 16 * t - 1) / (16 * t)) * bext;
+  };
+  int tile = 4, splitk = 1;
+  if (sizeof(T) == 4) {
+    // split K until the grid holds about one CTA per SM: two per SM measured
+    // slower in the concurrent move (the CTAs of other rows' kernels share the
+    // SMs; the split-K partials double), far fewer lengthens the row
+    const int64_t tiles = tiles_of(tile);
+    if (tiles < sms && p.Kt >= 2 * BK) {
+      splitk = static_cast<int>(std::min<int64_t>((sms + tiles - 1) / tiles, p.Kt / BK));
+      splitk = std::max(splitk, 1);
+    }
+  } else {
+    // An SM does 1.7 FP64 FMAs per cycle: a 64 x 64 tile costs it 2400 cycles
+    // per K index, so a small contraction has to reach every SM (80 x 80 x 80:
+    // four 64 x 64 tiles in five K ranges 22 us, 75 tiles of 16 x 16 x 32 5 us).
+    // The tile size and K split with the least estimated time: 152 kT^2 cycles
+    // per K index and tile, 2500 per tile, 5000 for the sum of the partials.
+    double least = 0.0;
+    for (int t : {4, 2, 1}) {
+      const int64_t tiles = tiles_of(t);
+      if (t != 4 && tiles > 8 * sms) break;
+      for (int64_t sp = 1; sp <= std::max<int64_t>(1, std::min<int64_t>(p.Kt / BK, 16)); ++sp) {
+        const int64_t ch = ((p.Kt + sp - 1) / sp + BK - 1) / BK * BK;
+        const int64_t ranges = std::max<int64_t>(1, (p.Kt + ch - 1) / ch);
+        if (ranges != sp) continue;
+        const double waves = double((tiles * sp + sms - 1) / sms);
+        const double cost = waves * (152.0 * t * t * double(std::min(ch, p.Kt)) + 2500.0) +
+                            (sp > 1 ? 5000.0 + double(sp) * p.Mt * p.Nt * bext / double(sms) : 0.0);
+        if (least == 0.0 || cost < least) {
+          least = cost;
+          tile = t;
+          splitk = int(sp);
+        }
+      }
+    }
   }
   p.kchunk = ((p.Kt + splitk - 1) / splitk + BK - 1) / BK * BK;
   if (p.Kt == 0) p.kchunk = BK;
@@ -457,7 +487,8 @@ void einsum_impl(Ctx& c, const char* spec, const ViewT<T>& A, const ViewT<T>& B,
   Scope scope(c);
   if (splitk > 1) p.part = c.alloc<T>(size_t(splitk) * bext * p.Mt * p.Nt);
   if (c.sizing()) return;
-  const int64_t mtiles = (p.Mt + BM - 1) / BM, ntiles = (p.Nt + BN - 1) / BN;
+  const int64_t edge = 16 * tile;
+  const int64_t mtiles = (p.Mt + edge - 1) / edge, ntiles = (p.Nt + edge - 1) / edge;
   p.swap_xy = ntiles > 65535 ? 1 : 0;
   dim3 grid(static_cast<unsigned>(p.swap_xy ? ntiles : mtiles),
             static_cast<unsigned>(p.swap_xy ? mtiles : ntiles), static_cast<unsigned>(bext * splitk));
@@ -468,7 +499,12 @@ void einsum_impl(Ctx& c, const char* spec, const ViewT<T>& A, const ViewT<T>& B,
     KernelTimer timer(c.stream, sizeof(T) == 8 ? kTagGettF64 : kTagGettF32, flops);
     KernelTimer kt(c.stream, sizeof(T) == 8 ? "gett_kernel<double>" : "gett_kernel<float>",
                    kUnitFlop, flops);
-    gett_kernel<T><<<grid, NT, 0, c.stream>>>(p);
+    if (tile == 4) {
+      gett_kernel<T, 4><<<grid, NT, 0, c.stream>>>(p);
+    } else if constexpr (sizeof(T) == 8) {
+      if (tile == 2) gett_kernel<T, 2><<<grid, NT, 0, c.stream>>>(p);
+      else gett_kernel<T, 1><<<grid, NT, 0, c.stream>>>(p);
+    }
     CTM_LAUNCH_CHECK();
   }
   if (splitk > 1) splitk_reduce_impl<T>(c, p);
