@@ -17,6 +17,9 @@ void einsum(Ctx& c, const char* spec, const ViewF& A, const ViewF& B, const View
 // Number of SMs of the current device.
 int sm_count_linalg();
 
+// CTAs of the largest cluster with full shared memory (16 or 8).
+int max_cluster_ctas();
+
 void absmax(Ctx& c, const double* x, int64_t n, double* out);
 void sumsq(Ctx& c, const double* x, int64_t n, double* out);
 // x[i] = x[i] / s  (mode 0: s = *scal, mode 1: s = sqrt(*scal)) for i < n.
@@ -35,6 +38,11 @@ void to_f64(Ctx& c, const float* x, double* y, int64_t n);
 // ~u cond^2 after the shifted stage, i.e. about 1e-3 in FP32, for bases that
 // are only multiplied again in lower precision).
 void orthonormalize(Ctx& c, double* Y, int64_t n, int64_t q, double* R, int stages = 3);
+// Householder QR of Y (n x q) in place by one cluster, R (q x q) when not null,
+// with LAPACK's signs (R's diagonal opposite to the pivots), and whether the
+// matrix fits.
+bool householder_cluster_fits(int64_t n, int64_t q);
+void householder_cluster(Ctx& c, double* Y, int64_t n, int64_t q, double* R);
 // Shifted Cholesky-QR3 of Y without the Householder fallback: bit 1 of
 // *failed (device, cleared first) is set when the result is not orthonormal
 // to working precision, and Y and R then mean nothing.

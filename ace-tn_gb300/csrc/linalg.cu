@@ -1271,12 +1271,19 @@ void orthonormalize_impl(Ctx& c, T* Y, int64_t n, int64_t q, T* R, int stages,
   Scope scope(c);
   T* V = c.alloc<T>(size_t(n) * q);
   T* beta = c.alloc<T>(q);
-  // the one-CTA Householder QR for small problems (its cost grows as q^2
-  // barriers); the FP32 slab kernels beat it from q = 32 on
+  // Householder QR for small problems: FP64 in a cluster's shared memory where
+  // it fits, else on one CTA (its cost grows as q^2 barriers; the FP32 slab
+  // kernels beat it from q = 32 on)
   const bool small = (failed != nullptr || (sizeof(T) == 4 && q >= 32))
                          ? false
                          : double(n) * q * q <= 4.0e6;
   if (small) {
+    if constexpr (sizeof(T) == 8) {
+      if (householder_cluster_fits(n, q)) {
+        if (!c.sizing()) householder_cluster(c, Y, n, q, R);
+        return;
+      }
+    }
     if (c.sizing()) return;
     KernelTimer kt(c.stream, "householder_qr_kernel", kUnitFlop, 4.0 * double(n) * q * q);
     householder_qr_kernel<T><<<1, LT, 0, c.stream>>>(Y, n, q, R, V, beta, nullptr, 1);

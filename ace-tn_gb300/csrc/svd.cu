@@ -322,36 +322,6 @@ size_t jacobi_smem(int64_t m, int64_t p, int64_t L) {
   return size_t(4 * m) * size_t(jacobi_row(int(p), int(L))) * sizeof(double);
 }
 
-// CTAs of the largest cluster that this device runs at full shared memory (16
-// where a GPC has that many free SMs, else 8, the portable size).
-int max_cluster_ctas() {
-  static const int n = [] {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(16);
-    cfg.blockDim = dim3(512);
-    cfg.dynamicSmemBytes = kJacobiSmem;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 16;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int clusters = 0;
-    const auto kern = jacobi_cluster_f64_kernel<32>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kJacobiSmem)) !=
-            cudaSuccess ||
-        cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
-            cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess) {
-      cudaGetLastError();
-      return 8;
-    }
-    return clusters > 0 ? 16 : 8;
-  }();
-  return n;
-}
-
 JacobiShape jacobi_shape(int64_t p, int64_t L) {
   JacobiShape best;
   double least = 0.0;
@@ -696,6 +666,36 @@ void jacobi_square(Ctx& c, double* W, double* J, double* norm2, int64_t p, const
 }
 
 }  // namespace
+
+// CTAs of the largest cluster that this device runs at full shared memory (16
+// where a GPC has that many free SMs, else 8, the portable size).
+int max_cluster_ctas() {
+  static const int n = [] {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(16);
+    cfg.blockDim = dim3(512);
+    cfg.dynamicSmemBytes = kJacobiSmem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 16;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    const auto kern = jacobi_cluster_f64_kernel<32>;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kJacobiSmem)) !=
+            cudaSuccess ||
+        cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
+            cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      return 8;
+    }
+    return clusters > 0 ? 16 : 8;
+  }();
+  return n;
+}
 
 void svd_thin(Ctx& c, const double* X, int64_t m, int64_t n, double* U, double* S, double* V) {
   CTM_REQUIRE(m >= 1 && n >= 1, CTM_ERR_INVALID, "svd_thin: empty matrix");
