@@ -56,7 +56,8 @@ void svd_thin(Ctx& c, const double* X, int64_t m, int64_t n, double* U, double* 
 // FP32 one-sided Jacobi on the rows of Mc (q x q): Jc (q x q) the accumulated
 // rotations (orthogonal to FP32 accuracy), norms the final row norms; *flags
 // gets bit 2 when the sweep limit is reached.
-void jacobi_rotations(Ctx& c, const float* Mc, int64_t q, float* Jc, float* norms, int* flags);
+void jacobi_rotations(Ctx& c, const float* Mc, int64_t q, float* Jc, float* norms, int max_sweeps,
+                      int* flags);
 // Thin SVD of B (q x n, q <= min(n, 1024)) for the mixed path, from
 // Bt = B^T (n x q, FP32): R of a shifted Cholesky-QR3 of Bt (B = R^T Qb^T),
 // FP32 one-sided Jacobi on the columns of R with accumulated rotations

@@ -1318,7 +1318,9 @@ void orthonormalize_impl(Ctx& c, T* Y, int64_t n, int64_t q, T* R, int stages,
   // stage's L^-T (forward substitution with L^T) and forms the next Gram
   // matrix in the same pass over the rows; the factorisation forms no inverse
   const bool fast_f32 = sizeof(T) == 4 && q <= 192;
-  const T tol = sizeof(T) == 8 ? T(stages == 3 ? 1e-11 : 1e-6) : T(stages == 3 ? 2e-4 : 5e-2);
+  // (a factorisation that is used without the fallback has to be orthonormal to
+  // working precision)
+  const T tol = sizeof(T) == 8 ? T(failed != nullptr ? 1e-13 : stages == 3 ? 1e-11 : 1e-6) : T(stages == 3 ? 2e-4 : 5e-2);
   auto accumulate_r = [&](int stage) {
     if (R == nullptr) return;
     if (stage == 0) {
@@ -1462,7 +1464,7 @@ __global__ void scale_columns_f32_kernel(float* x, int64_t rows, int cols, const
 // rotations (row j: those of row j), norms = the final row norms.  *flags gets
 // bit 2 when the sweep limit is reached.
 void jacobi_rotations_impl(Ctx& c, const float* Mc, int64_t q, float* Jc, float* norms,
-                           int* flags) {
+                           int max_sweeps, int* flags) {
   Scope scope(c);
   // the Jacobi matrices stay in shared memory up to q = 160, in global
   // memory (L2) beyond
@@ -1502,7 +1504,7 @@ void jacobi_rotations_impl(Ctx& c, const float* Mc, int64_t q, float* Jc, float*
       cfg.attrs = attr;
       cfg.numAttrs = 1;
       CTM_CUDA(cudaLaunchKernelEx(&cfg, kern, static_cast<const float*>(Mc), int(q), b, Jc, norms,
-                                  40, 4e-6f, flags));
+                                  max_sweeps, 4e-6f, flags));
     };
     switch (ldj / (4 * kPairThreads)) {
       case 3: launch(jacobi_cluster_f32_kernel<3, kPairThreads>); break;
@@ -1523,7 +1525,7 @@ void jacobi_rotations_impl(Ctx& c, const float* Mc, int64_t q, float* Jc, float*
     auto launch = [&](auto kern) {
       CTM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(wjac)));
       KernelTimer kt(c.stream, "jacobi_onesided_f32_kernel", kUnitFlop, 0.0);
-      kern<<<1, jthreads, wjac, c.stream>>>(Mc, int(q), int(pp), Jc, norms, 40, 4e-6f,
+      kern<<<1, jthreads, wjac, c.stream>>>(Mc, int(q), int(pp), Jc, norms, max_sweeps, 4e-6f,
                                            flags, nullptr);
     };
     switch (jacobi_ld(int(q)) / 32) {
@@ -1537,7 +1539,7 @@ void jacobi_rotations_impl(Ctx& c, const float* Mc, int64_t q, float* Jc, float*
   } else {
     KernelTimer kt(c.stream, "jacobi_onesided_f32_kernel", kUnitFlop, 0.0);
     jacobi_onesided_f32_kernel<false, 0><<<1, jthreads, 0, c.stream>>>(
-        Mc, int(q), int(pp), Jc, norms, 40, 4e-6f, flags, Wg);
+        Mc, int(q), int(pp), Jc, norms, max_sweeps, 4e-6f, flags, Wg);
   }
   CTM_LAUNCH_CHECK();
 }
@@ -1550,14 +1552,15 @@ void jacobi_left_singular(Ctx& c, const float* Mc, int64_t q, double* Ub, double
   Scope scope(c);
   float* Jc = c.alloc<float>(size_t(q) * q);
   float* norms = c.alloc<float>(q);
-  jacobi_rotations_impl(c, Mc, q, Jc, norms, c.sizing() ? nullptr : status_flags(c));
+  jacobi_rotations_impl(c, Mc, q, Jc, norms, 40, c.sizing() ? nullptr : status_flags(c));
   if (!c.sizing()) sort_singular(c.stream, Jc, norms, q, Ub, S, inv_s);
 }
 
 }  // namespace
 
-void jacobi_rotations(Ctx& c, const float* Mc, int64_t q, float* Jc, float* norms, int* flags) {
-  jacobi_rotations_impl(c, Mc, q, Jc, norms, flags);
+void jacobi_rotations(Ctx& c, const float* Mc, int64_t q, float* Jc, float* norms, int max_sweeps,
+                      int* flags) {
+  jacobi_rotations_impl(c, Mc, q, Jc, norms, max_sweeps, flags);
 }
 
 void svd_via_qr(Ctx& c, const float* Bt, int64_t q, int64_t n, double* Ub, double* S, float* V) {

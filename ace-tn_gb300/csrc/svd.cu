@@ -4,9 +4,13 @@
 //    of up to 16 CTAs (up to about 320 x 320), from the rotations of an FP32
 //    Jacobi when the matrix is square (144 x 144: 2.6 to 4.3 ms, 27 ms as
 //    jacobi_sweeps_kernel; 80 x 80: 1.2 to 2.0 ms against 11 ms).
-//  * A long matrix (L > 6 p) is reduced to its p x p triangular factor first
-//    (shifted Cholesky-QR3): the rotations then work on rows of p instead of
-//    L entries, and the long singular vectors are one product with Q.
+//  * From 32 to 160 columns, and for long matrices, a QR factorisation first: the
+//    rows of the p x p factor R are rotated and the long singular vectors are
+//    one product with Q.  R is graded even when the matrix is not, which is
+//    what one-sided Jacobi needs: a 144 x 144 product of four enlarged corners
+//    (values from 1 to 1e-17) takes ten FP32 and four FP64 sweeps from R, and
+//    14 and 29 without the QR.  Householder in a cluster where it fits (any
+//    rank), else a shifted Cholesky-QR3.
 //  * jacobi_sweeps_kernel: rows in global memory, a cooperative grid with a
 //    bounded grid barrier (Demmel & Veselic, SIAM J. Matrix Anal. Appl. 13
 //    (1992) 1204): matrices beyond the cluster's shared memory, and inputs on
@@ -617,13 +621,13 @@ __global__ void __launch_bounds__(1024) scaled_f32_kernel(const double* X, int n
   }
 }
 
-// Preconditioned Jacobi on the rows of W (p x p), p in [kPreMin, kPreMax]: an
-// FP32 Jacobi finds rotations T that make the rows orthogonal to about 1e-6,
-// T is made orthogonal to FP64 accuracy by two Newton steps
-// T <- (3 T - (T T^T) T) / 2 (its deviation of 1e-6 is squared twice), and the
-// FP64 rotations start from T W and T: two or three sweeps instead of 9 to 20
-// (Drmac and Veselic's preconditioning with an approximate SVD in the place
-// of the QR factor).  At p = 144 an FP64 sweep takes 0.5 ms, an FP32 one 0.1.
+// Preconditioned Jacobi on the rows of W (p x p, mostly a triangular factor), p in
+// [kPreMin, kPreMax]: an FP32 Jacobi finds rotations T that make the rows
+// orthogonal to about 1e-6, T is made orthogonal to FP64 accuracy by two Newton
+// steps T <- (3 T - (T T^T) T) / 2 (its deviation of 1e-6 is squared twice), and
+// the FP64 rotations start from T W and T: three or four sweeps instead of 9 to
+// 20 (Drmac and Veselic's preconditioning, with an approximate SVD after the QR
+// factor).  At p = 144 an FP64 sweep takes 0.5 ms, an FP32 one 0.1.
 constexpr int64_t kPreMin = 16, kPreMax = 256;
 
 void jacobi_square(Ctx& c, double* W, double* J, double* norm2, int64_t p, const int* skip) {
@@ -646,7 +650,8 @@ void jacobi_square(Ctx& c, double* W, double* J, double* norm2, int64_t p, const
     scaled_f32_kernel<<<1, 1024, 0, c.stream>>>(W, int(pp), Wf);
     CTM_LAUNCH_CHECK();
   }
-  jacobi_rotations(c, Wf, p, Jf, nf, unused);
+  // what is left after ten sweeps lies at the FP32 rounding level
+  jacobi_rotations(c, Wf, p, Jf, nf, 10, unused);
   to_f64(c, Jf, T, p * p);
   const View t(T, {p, p}), t2(T2, {p, p}), g(G, {p, p}), w(W, {p, p});
   auto newton = [&](const View& from, const View& to) {
@@ -716,10 +721,14 @@ void svd_thin(Ctx& c, const double* X, int64_t m, int64_t n, double* U, double* 
       CTM_CUDA(cudaMemcpyAsync(W, X, sizeof(double) * m * n, cudaMemcpyDeviceToDevice, c.stream));
   };
   const JacobiShape direct = jacobi_shape(p, L), square = jacobi_shape(p, p);
-  // the triangular factor pays off for long rows once the Cholesky-QR (about
-  // nine launches and three one-SM factorisations) is cheaper than the longer
-  // rotations
-  const bool reduce = L > 6 * p && square.ctas > 0 && double(L) * p * p > 4.0e6;
+  // The one-cluster Householder QR up to the size where the Cholesky-QR (about
+  // 20 launches and three one-SM factorisations) is faster; the latter only
+  // where it saves long rows, as it takes well-conditioned input.  No QR for
+  // small matrices: 22 x 80 takes 250 us in 8 sweeps, about what the QR and the
+  // FP32 stage would.
+  const bool house = householder_cluster_fits(L, p) && double(L) * p * p <= 4.0e6;
+  const bool reduce = square.ctas > 0 && (L > 6 * p || direct.ctas == 0 ||
+                                          (house && p >= 32 && p <= kPreMax));
   if (!reduce) {
     load_w();
     if (p == L && direct.ctas > 0) {
@@ -748,12 +757,15 @@ void svd_thin(Ctx& c, const double* X, int64_t m, int64_t n, double* U, double* 
     else
       copy2d(c, View(X, {m, n}).permute({1, 0}), Y, p);
   }
-  orthonormalize_try(c, Y, L, p, R, failed);
+  if (!house) orthonormalize_try(c, Y, L, p, R, failed);
+  else if (!c.sizing()) householder_cluster(c, Y, L, p, R);
+  const int* const flag = house ? nullptr : failed;
   if (!c.sizing())
     CTM_CUDA(cudaMemcpyAsync(W2, R, sizeof(double) * p * p, cudaMemcpyDeviceToDevice, c.stream));
-  jacobi_square(c, W2, J, norm2, p, failed);
+  jacobi_square(c, W2, J, norm2, p, flag);
   if (!c.sizing()) finish(c, W2, J, norm2, p, p, Xs, S, Vs, nullptr);
   einsum(c, "ik,kj->ij", View(Y, {L, p}), View(Xs, {p, p}), View(Vl, {L, p}));
+  if (house) return;
   // when the Cholesky-QR has failed: the whole matrix again, in global memory
   load_w();
   jacobi_grid(c, W, J, norm2, p, L, failed);
