@@ -81,9 +81,14 @@ void quarter_tensor(Ctx& c, const Site& S, int k, double* Q, int64_t qshape[6]) 
 // ------------------------------------------------------------------ rSVD
 // fused_matmul_svd_lowrank and friends (acetn/linalg/*.py) on a chain of
 // factors F[0] @ F[1] @ ... (each rows x cols, row-major).
+// The digits of a factor's rows and columns (for products with it and with its
+// transpose) are kept for the whole chain when it is large.
 struct Factor {
   const double* p;
   int64_t rows, cols;
+  Digits by_row, by_col;
+  const Digits* row_digits() const { return by_row.rows > 0 ? &by_row : nullptr; }
+  const Digits* col_digits() const { return by_col.rows > 0 ? &by_col : nullptr; }
 };
 
 namespace {
@@ -112,15 +117,33 @@ void product(Ctx& c, const double* A, const double* B, double* C, int64_t M, int
   tc_gemm(c, TcOperand{ah, al, M, K, ld}, TcOperand{bh, bl, N, K, ld}, TcMode::kBf16x3, out);
 }
 
+// Each factor is multiplied niter + 1 to niter + 3 times in either form, and the
+// digits (2 x 16 bytes per entry) take as long to form as one product: 0.25 ms of
+// 0.56 ms at 5184 x 5184 x 160.  At most kKeptDigits bytes of them are kept.
+constexpr double kKeptDigits = 24e9;
+
+void keep_digits(Ctx& c, std::vector<Factor>& F, int64_t q) {
+  double bytes = 0.0;
+  for (const Factor& f : F) bytes += 32.0 * double(f.rows) * double(f.cols);
+  if (bytes > kKeptDigits) return;
+  for (Factor& f : F) {
+    if (!digits_pay(f.rows, q, f.cols)) continue;
+    f.by_row = digit_rows(c, mat(f.p, f.rows, f.cols), 0);
+    f.by_col = digit_rows(c, mat(f.p, f.rows, f.cols), 1);
+  }
+}
+
 // y (f.rows x q) = f @ x (f.cols x q)
 void apply(Ctx& c, const Factor& f, const double* x, double* y, int64_t q, int prec) {
   (void)prec;
-  einsum(c, "ik,kj->ij", mat(f.p, f.rows, f.cols), mat(x, f.cols, q), mat(y, f.rows, q));
+  einsum(c, "ik,kj->ij", mat(f.p, f.rows, f.cols), mat(x, f.cols, q), mat(y, f.rows, q), 1.0, 0.0,
+         f.row_digits());
 }
 // y (f.cols x q) = f^T @ x (f.rows x q)
 void apply_t(Ctx& c, const Factor& f, const double* x, double* y, int64_t q, int prec) {
   (void)prec;
-  einsum(c, "ki,kj->ij", mat(f.p, f.rows, f.cols), mat(x, f.rows, q), mat(y, f.cols, q));
+  einsum(c, "ki,kj->ij", mat(f.p, f.rows, f.cols), mat(x, f.rows, q), mat(y, f.cols, q), 1.0, 0.0,
+         f.col_digits());
 }
 
 }  // namespace
@@ -183,12 +206,13 @@ void rsvd_chain(Ctx& c, const std::vector<Factor>& F, int64_t q, int niter, cons
   {
     int64_t cols = F[0].cols;
     (void)rr_prec;
-    einsum(c, "kq,kj->qj", mat(Y, m, q), mat(F[0].p, F[0].rows, F[0].cols), mat(B, q, cols));
+    einsum(c, "kq,kj->qj", mat(Y, m, q), mat(F[0].p, F[0].rows, F[0].cols), mat(B, q, cols), 1.0,
+           0.0, nullptr, F[0].col_digits());
     double* cur = B;
     double* other = B2;
     for (int i = 1; i < nf; ++i) {
       einsum(c, "qk,kj->qj", mat(cur, q, F[i].rows), mat(F[i].p, F[i].rows, F[i].cols),
-             mat(other, q, F[i].cols));
+             mat(other, q, F[i].cols), 1.0, 0.0, nullptr, F[i].col_digits());
       std::swap(cur, other);
       cols = F[i].cols;
     }
@@ -224,19 +248,23 @@ void truncate_and_project(Ctx& c, double* U, double* V, int64_t m, int64_t n, in
   Vv.stride[0] = ldu;
   if (left2 != nullptr) {
     double* tmp = c.alloc<double>(size_t(left2->cols) * cap);
-    einsum(c, "ki,kz->iz", mat(left2->p, left2->rows, left2->cols), Uv, mat(tmp, left2->cols, cap));
+    einsum(c, "ki,kz->iz", mat(left2->p, left2->rows, left2->cols), Uv, mat(tmp, left2->cols, cap),
+           1.0, 0.0, left2->col_digits());
     einsum(c, "ki,kz->iz", mat(left1.p, left1.rows, left1.cols), mat(tmp, left1.rows, cap),
-           mat(P1f, p1rows, cap));
+           mat(P1f, p1rows, cap), 1.0, 0.0, left1.col_digits());
   } else {
-    einsum(c, "ki,kz->iz", mat(left1.p, left1.rows, left1.cols), Uv, mat(P1f, p1rows, cap));
+    einsum(c, "ki,kz->iz", mat(left1.p, left1.rows, left1.cols), Uv, mat(P1f, p1rows, cap),
+           1.0, 0.0, left1.col_digits());
   }
   if (right2 != nullptr) {
     double* tmp = c.alloc<double>(size_t(right2->rows) * cap);
-    einsum(c, "ik,kz->iz", mat(right2->p, right2->rows, right2->cols), Vv, mat(tmp, right2->rows, cap));
+    einsum(c, "ik,kz->iz", mat(right2->p, right2->rows, right2->cols), Vv,
+           mat(tmp, right2->rows, cap), 1.0, 0.0, right2->row_digits());
     einsum(c, "ik,kz->iz", mat(right1.p, right1.rows, right1.cols), mat(tmp, right1.cols, cap),
-           mat(P2f, p2rows, cap));
+           mat(P2f, p2rows, cap), 1.0, 0.0, right1.row_digits());
   } else {
-    einsum(c, "ik,kz->iz", mat(right1.p, right1.rows, right1.cols), Vv, mat(P2f, p2rows, cap));
+    einsum(c, "ik,kz->iz", mat(right1.p, right1.rows, right1.cols), Vv, mat(P2f, p2rows, cap),
+           1.0, 0.0, right1.row_digits());
   }
   if (o.fixed_width) {
     if (!c.sizing()) {
@@ -324,16 +352,18 @@ void calculate_projectors(Ctx& c, const Site* S[4], int k, const ctm_ctmrg_opts&
   double* Q4 = c.alloc<double>(size_t(r4) * c4);
   quarter(*S[0], k, Q1, sh1);
   quarter(*S[3], k + 3, Q4, sh4);
-  const Factor F1{Q1, r1, c1}, F4{Q4, r4, c4};
+  const Factor F1{Q1, r1, c1, {}, {}}, F4{Q4, r4, c4, {}, {}};
   if (o.projectors == CTM_PROJ_HALF) {
     if (o.svd_type == CTM_SVD_RSVD) {
       const int64_t q = pd.q;
+      std::vector<Factor> F{F1, F4};
+      keep_digits(c, F, q);
       double* U = c.alloc<double>(size_t(r1) * q);
       double* s = c.alloc<double>(q);
       double* V = c.alloc<double>(size_t(c4) * q);
-      rsvd_chain(c, {F1, F4}, q, o.rsvd_niter, omega, U, s, V, prec);
-      truncate_and_project(c, U, V, r1, c4, q, s, q, o, F1, nullptr, F4, nullptr, P1, P2, chi_new,
-                           prec);
+      rsvd_chain(c, F, q, o.rsvd_niter, omega, U, s, V, prec);
+      truncate_and_project(c, U, V, r1, c4, q, s, q, o, F[0], nullptr, F[1], nullptr, P1, P2,
+                           chi_new, prec);
     } else {
       // contract_half_system (projectors.py:62-82): R = Q1 Q4 / max|R|
       const int64_t r = std::min(r1, c4);
@@ -359,14 +389,16 @@ void calculate_projectors(Ctx& c, const Site* S[4], int k, const ctm_ctmrg_opts&
   double* Q3 = c.alloc<double>(size_t(r3) * c3);
   quarter(*S[1], k + 1, Q2, sh2);
   quarter(*S[2], k + 2, Q3, sh3);
-  const Factor F2{Q2, r2, c2}, F3{Q3, r3, c3};
+  const Factor F2{Q2, r2, c2, {}, {}}, F3{Q3, r3, c3, {}, {}};
   if (o.svd_type == CTM_SVD_RSVD) {
     const int64_t q = pd.q;
+    std::vector<Factor> F{F2, F1, F4, F3};
+    keep_digits(c, F, q);
     double* U = c.alloc<double>(size_t(r2) * q);
     double* s = c.alloc<double>(q);
     double* V = c.alloc<double>(size_t(c3) * q);
-    rsvd_chain(c, {F2, F1, F4, F3}, q, o.rsvd_niter, omega, U, s, V, CTM_PREC_FP64);
-    truncate_and_project(c, U, V, r2, c3, q, s, q, o, F1, &F2, F4, &F3, P1, P2, chi_new,
+    rsvd_chain(c, F, q, o.rsvd_niter, omega, U, s, V, CTM_PREC_FP64);
+    truncate_and_project(c, U, V, r2, c3, q, s, q, o, F[1], &F[0], F[2], &F[3], P1, P2, chi_new,
                          CTM_PREC_FP64);
     return;
   }
@@ -389,8 +421,8 @@ void calculate_projectors(Ctx& c, const Site* S[4], int k, const ctm_ctmrg_opts&
   double* s = c.alloc<double>(r);
   double* V = c.alloc<double>(size_t(c3) * r);
   svd_thin(c, Fm, r2, c3, U, s, V);
-  truncate_and_project(c, U, V, r2, c3, r, s, r, om, Factor{R1, r2, c1}, nullptr,
-                       Factor{R2, r4, c3}, nullptr, P1, P2, chi_new, CTM_PREC_FP64);
+  truncate_and_project(c, U, V, r2, c3, r, s, r, om, Factor{R1, r2, c1, {}, {}}, nullptr,
+                       Factor{R2, r4, c3, {}, {}}, nullptr, P1, P2, chi_new, CTM_PREC_FP64);
 }
 
 // ------------------------------------------------------------------ renormalization
@@ -972,7 +1004,9 @@ int ctm_svd_lowrank(const double* a, int64_t m, int64_t n, int64_t q, int32_t ni
                     size_t* ws_bytes, ctm_stream_t stream) {
   return with_workspace(ws, ws_bytes, as_stream(stream), [&](Ctx& c) {
     CTM_REQUIRE(m >= 1 && n >= 1 && niter >= 0, CTM_ERR_INVALID, "bad size");
-    rsvd_chain(c, {Factor{a, m, n}}, q, niter, omega, U, S, V, CTM_PREC_FP64);
+    std::vector<Factor> F{Factor{a, m, n, {}, {}}};
+    if (niter > 0) keep_digits(c, F, q);
+    rsvd_chain(c, F, q, niter, omega, U, S, V, CTM_PREC_FP64);
   });
 }
 
@@ -984,7 +1018,9 @@ int ctm_fused_matmul_svd_lowrank(const double* a, const double* b, int64_t m, in
     CTM_REQUIRE(m >= 1 && n >= 1 && k >= 1 && niter >= 0, CTM_ERR_INVALID, "bad size");
     CTM_REQUIRE(precision == CTM_PREC_FP64 || precision == CTM_PREC_MIXED, CTM_ERR_INVALID,
                 "bad precision");
-    rsvd_chain(c, {Factor{a, m, k}, Factor{b, k, n}}, q, niter, omega, U, S, V, precision);
+    std::vector<Factor> F{Factor{a, m, k, {}, {}}, Factor{b, k, n, {}, {}}};
+    if (niter > 0) keep_digits(c, F, q);
+    rsvd_chain(c, F, q, niter, omega, U, S, V, precision);
   });
 }
 
@@ -996,8 +1032,10 @@ int ctm_fused_3matmul_svd_lowrank(const double* a, const double* b, const double
   return with_workspace(ws, ws_bytes, as_stream(stream), [&](Ctx& c) {
     CTM_REQUIRE(m >= 1 && n >= 1 && k1 >= 1 && k2 >= 1 && k3 >= 1 && niter >= 0, CTM_ERR_INVALID,
                 "bad size");
-    rsvd_chain(c, {Factor{a, m, k1}, Factor{b, k1, k2}, Factor{cc, k2, k3}, Factor{e, k3, n}}, q,
-               niter, omega, U, S, V, CTM_PREC_FP64);
+    std::vector<Factor> F{Factor{a, m, k1, {}, {}}, Factor{b, k1, k2, {}, {}},
+                          Factor{cc, k2, k3, {}, {}}, Factor{e, k3, n, {}, {}}};
+    if (niter > 0) keep_digits(c, F, q);
+    rsvd_chain(c, F, q, niter, omega, U, S, V, CTM_PREC_FP64);
   });
 }
 

@@ -42,7 +42,10 @@ namespace {
 using bf16 = __nv_bfloat16;
 
 constexpr int kDigits = 8;
-constexpr int kBadRow = 0x40000000;  // exponent of a row with a non-finite entry
+// A row's scale is kept as the largest exponent field of its entries: |x| <
+// 2^(row_exponent(field) - 1023).  Field 2047: a non-finite entry, no digits.
+constexpr int kBadField = 2047;
+__device__ __forceinline__ int row_exponent(int field) { return max(field, 1) + 1; }
 
 // ------------------------------------------------------------- splitting
 struct SplitSide {
@@ -52,7 +55,7 @@ struct SplitSide {
   int k_is_s1;     // the contracted group's stride of this operand is s1 (second operand)
   int64_t rows;
   int kfast;       // the contracted index has unit stride (else rows are read fastest)
-  int* exps;       // rows: exponent E with |x| < 2^(E - 1023), or kBadRow
+  int* exps;       // rows: the largest exponent field
   bf16* dig;       // [digit][row][Kp]
 };
 
@@ -104,13 +107,12 @@ __device__ void load_block(const SplitSide& s, const SplitArgs& a, int64_t r0, i
   __syncthreads();
 }
 
-// Largest exponent field of each row of the block, 1 at least; 2047 when an
-// entry is not finite.  Four lanes per row.
+// Largest exponent field of each row of the block.  Four lanes per row.
 __device__ void row_exponents(const SplitArgs& a, int nr, int nk, const double* sx, int* s_e) {
   const int ld = a.kc + 1;
   for (int q = threadIdx.x; q < a.rb * 4; q += blockDim.x) {
     const int r = q >> 2;
-    int e = 1;
+    int e = 0;
     if (r < nr)
       for (int k = q & 3; k < nk; k += 4) e = max(e, exponent_field(sx[r * ld + k]));
     e = max(e, __shfl_xor_sync(0xffffffffu, e, 1));
@@ -141,6 +143,39 @@ __device__ __forceinline__ uint32_t digit_f32(uint32_t w, int byte) {
   return __float_as_uint(__uint_as_float(u) - 8388736.f);  // 2^23 + 128
 }
 
+// The eight digits of eight consecutive entries, 16 bytes per digit plane.
+__device__ __forceinline__ void write_digits(const double (&x)[8], int E, bf16* dst,
+                                             int64_t plane) {
+  uint32_t lo[8], hi[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const long long bits = __double_as_longlong(x[i]);
+    const int ex = int((unsigned long long)bits >> 52) & 0x7ff;
+    const long long mant = (bits & 0xfffffffffffffll) | (ex != 0 ? 0x10000000000000ll : 0ll);
+    const int sh = max(ex, 1) - E + 10;  // x 2^62 / 2^(E - 1023) = mant 2^sh, sh <= 9
+    long long t;
+    if (sh >= 0) t = mant << sh;
+    else if (sh >= -54) t = (mant + (1ll << (-sh - 1))) >> -sh;
+    else t = 0;
+    if (bits < 0) t = -t;
+    const unsigned long long u =
+        ((unsigned long long)t + 0x0080808080808080ull) ^ 0x8000000000000000ull;
+    lo[i] = uint32_t(u);
+    hi[i] = uint32_t(u >> 32);
+  }
+#pragma unroll
+  for (int d = 0; d < kDigits; ++d) {  // digit 0 is the top byte
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t f0 = digit_f32(d < 4 ? hi[2 * i] : lo[2 * i], 3 - (d & 3));
+      const uint32_t f1 = digit_f32(d < 4 ? hi[2 * i + 1] : lo[2 * i + 1], 3 - (d & 3));
+      w[i] = __byte_perm(f0, f1, 0x7632);
+    }
+    *reinterpret_cast<uint4*>(dst + int64_t(d) * plane) = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+}
+
 __global__ void __launch_bounds__(256) split_digits_kernel(const SplitArgs a) {
   extern __shared__ __align__(16) double sx[];
   __shared__ int64_t s_ro[128], s_ko[256];
@@ -153,10 +188,9 @@ __global__ void __launch_bounds__(256) split_digits_kernel(const SplitArgs a) {
   const int nr = int(min(int64_t(a.rb), s.rows - r0)), nk = int(min(int64_t(a.kc), a.K - k0));
   if (a.kblocks == 1) {
     row_exponents(a, nr, nk, sx, s_e);
-    for (int r = threadIdx.x; r < nr; r += blockDim.x)
-      s.exps[r0 + r] = s_e[r] == 2047 ? kBadRow : s_e[r] + 1;
-  } else {  // row_exponent_kernel has left the largest field
-    for (int r = threadIdx.x; r < nr; r += blockDim.x) s_e[r] = max(1, s.exps[r0 + r]);
+    for (int r = threadIdx.x; r < nr; r += blockDim.x) s.exps[r0 + r] = s_e[r];
+  } else {
+    for (int r = threadIdx.x; r < nr; r += blockDim.x) s_e[r] = s.exps[r0 + r];
     __syncthreads();
   }
   const int ld = a.kc + 1;
@@ -167,48 +201,113 @@ __global__ void __launch_bounds__(256) split_digits_kernel(const SplitArgs a) {
     const int pair = q / (a.rb * 2), rest = q - pair * (a.rb * 2);
     const int r = rest >> 1, g = pair * 2 + (rest & 1);
     if (r >= nr || g >= ng) continue;
-    const int E = s_e[r] + 1;
-    uint32_t lo[8], hi[8];
+    const int E = row_exponent(s_e[r]);
+    double x[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const int k = g * 8 + i;
-      const double x = k < nk ? sx[r * ld + k] : 0.0;
-      const long long bits = __double_as_longlong(x);
-      const int ex = int((unsigned long long)bits >> 52) & 0x7ff;
-      long long mant = (bits & 0xfffffffffffffll) | (ex != 0 ? 0x10000000000000ll : 0ll);
-      const int sh = max(ex, 1) - E + 10;  // x 2^62 / 2^(E - 1023) = mant 2^sh, sh <= 9
-      long long t;
-      if (sh >= 0) t = mant << sh;
-      else if (sh >= -54) t = (mant + (1ll << (-sh - 1))) >> -sh;
-      else t = 0;
-      if (bits < 0) t = -t;
-      const unsigned long long u =
-          ((unsigned long long)t + 0x0080808080808080ull) ^ 0x8000000000000000ull;
-      lo[i] = uint32_t(u);
-      hi[i] = uint32_t(u >> 32);
+      x[i] = k < nk ? sx[r * ld + k] : 0.0;
     }
-    bf16* dst = s.dig + (r0 + r) * a.Kp + k0 + g * 8;
-#pragma unroll
-    for (int d = 0; d < kDigits; ++d) {  // digit 0 is the top byte
-      uint32_t w[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const uint32_t f0 = digit_f32(d < 4 ? hi[2 * i] : lo[2 * i], 3 - (d & 3));
-        const uint32_t f1 = digit_f32(d < 4 ? hi[2 * i + 1] : lo[2 * i + 1], 3 - (d & 3));
-        w[i] = __byte_perm(f0, f1, 0x7632);
-      }
-      *reinterpret_cast<uint4*>(dst + int64_t(d) * plane) = make_uint4(w[0], w[1], w[2], w[3]);
-    }
+    write_digits(x, E, s.dig + (r0 + r) * a.Kp + k0 + g * 8, plane);
   }
 }
 
-// The exponents that row_exponent_kernel leaves (largest field, 2047 for
-// non-finite) in the form the products read.
-__global__ void finish_exponents_kernel(int* exps, int64_t n) {
-  const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  if (i < n) {
-    const int e = max(1, exps[i]);
-    exps[i] = e == 2047 ? kBadRow : e + 1;
+// Long rows whose contracted index is one mode (the large matrices of the
+// randomized SVD): the warps read along whichever index has unit stride.
+// 5184 x 5184 by rows: exponents 39 us and digits 94 us (147 + 229 us through the
+// general kernels' shared-memory blocks).
+struct LongRows {
+  const double* x;
+  Group R;
+  int64_t ks;       // stride of the contracted index
+  int64_t rows, K, Kp;
+  int64_t kc;       // contracted indices per CTA of the exponent kernels
+  int* exps;        // zeroed when kc < K
+  bf16* dig;
+};
+
+__device__ __forceinline__ void put_field(const LongRows& a, int64_t r, int e) {
+  if (a.kc < a.K) atomicMax(a.exps + r, e);
+  else a.exps[r] = e;
+}
+
+// Contracted index of unit stride: one warp per row.
+__global__ void __launch_bounds__(256) long_exponents_k_kernel(const LongRows a) {
+  const int lane = threadIdx.x & 31;
+  const int64_t r = blockIdx.x * int64_t(8) + (threadIdx.x >> 5);
+  if (r >= a.rows) return;
+  int64_t ro, t;
+  decode(a.R, r, ro, t);
+  const double* x = a.x + ro;
+  const int64_t k0 = blockIdx.y * a.kc, k1 = min(k0 + a.kc, a.K);
+  int e = 0;
+#pragma unroll 8
+  for (int64_t k = k0 + lane; k < k1; k += 32) e = max(e, exponent_field(x[k * a.ks]));
+  for (int o = 16; o > 0; o >>= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, o));
+  if (lane == 0) put_field(a, r, e);
+}
+
+// Otherwise 32 rows per CTA, its warps share the contracted index.
+__global__ void __launch_bounds__(512) long_exponents_r_kernel(const LongRows a) {
+  __shared__ int s_e[16][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t r = blockIdx.x * int64_t(32) + lane;
+  const int64_t k0 = blockIdx.y * a.kc, k1 = min(k0 + a.kc, a.K);
+  int64_t ro = 0, t;
+  if (r < a.rows) decode(a.R, r, ro, t);
+  int e = 0;
+  if (r < a.rows) {
+#pragma unroll 8
+    for (int64_t k = k0 + warp; k < k1; k += 16) e = max(e, exponent_field(a.x[ro + k * a.ks]));
+  }
+  s_e[warp][lane] = e;
+  __syncthreads();
+  if (warp == 0 && r < a.rows) {
+    for (int w = 1; w < 16; ++w) e = max(e, s_e[w][lane]);
+    put_field(a, r, e);
+  }
+}
+
+// kfast: a warp takes 8 rows x 32 indices, four lanes of eight per row, straight
+// from memory.  Else a CTA takes 32 rows x 64 indices through shared memory; two
+// lanes write 32 contiguous bytes of a row.
+template <bool kfast>
+__global__ void __launch_bounds__(256) long_split_kernel(const LongRows a) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t plane = a.rows * a.Kp;
+  if (kfast) {
+    const int64_t kblocks = (a.Kp + 31) / 32;
+    const int64_t w = blockIdx.x * int64_t(8) + warp;
+    const int64_t r = w / kblocks * 8 + (lane >> 2), k0 = w % kblocks * 32 + (lane & 3) * 8;
+    if (r >= a.rows || k0 >= a.Kp) return;
+    int64_t ro, t;
+    decode(a.R, r, ro, t);
+    double x[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) x[i] = k0 + i < a.K ? a.x[ro + (k0 + i) * a.ks] : 0.0;
+    write_digits(x, row_exponent(a.exps[r]), a.dig + r * a.Kp + k0, plane);
+  } else {
+    __shared__ double sx[32][65];
+    const int64_t rblocks = (a.rows + 31) / 32;
+    const int64_t r0 = int64_t(blockIdx.x) % rblocks * 32, kb = int64_t(blockIdx.x) / rblocks * 64;
+    {
+      const int64_t r = r0 + lane;
+      int64_t ro = 0, t;
+      if (r < a.rows) decode(a.R, r, ro, t);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int64_t k = kb + warp + 8 * i;
+        sx[lane][warp + 8 * i] = r < a.rows && k < a.K ? a.x[ro + k * a.ks] : 0.0;
+      }
+    }
+    __syncthreads();
+    const int rl = (warp & 1) * 16 + (lane >> 1), g = (warp >> 1) * 2 + (lane & 1);
+    const int64_t r = r0 + rl, k0 = kb + g * 8;
+    if (r >= a.rows || k0 >= a.Kp) return;
+    double x[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) x[i] = sx[rl][g * 8 + i];
+    write_digits(x, row_exponent(a.exps[r]), a.dig + r * a.Kp + k0, plane);
   }
 }
 
@@ -543,8 +642,8 @@ __global__ void __launch_bounds__(kDThreads, 1)
           if (off < 0) continue;
           // units of 2^-68 of the scales (digit s of the product: 2^(-12 - 8 s))
           double v;
-          if (((er | e) & kBadRow) != 0) v = chain_dot(p, row, int64_t(n0) + half * kHalf + c, k0, k1);
-          else v = round_96(hi[c], lo[c], er + e - 2 * 1023 - 68);
+          if (er == kBadField || e == kBadField) v = chain_dot(p, row, int64_t(n0) + half * kHalf + c, k0, k1);
+          else v = round_96(hi[c], lo[c], row_exponent(er) + row_exponent(e) - 2 * 1023 - 68);
           if (p.split == 1 && !(p.alpha == 1.0 && p.beta == 0.0)) {
             v *= p.alpha;
             if (p.beta != 0.0) v = fma(p.beta, out[off], v);
@@ -603,6 +702,78 @@ int best_ntile(int64_t n) {
   return best;
 }
 
+Digits alloc_digits(Ctx& c, int64_t rows, int64_t K) {
+  Digits d;
+  d.rows = rows;
+  d.K = K;
+  d.dig = c.alloc<bf16>(size_t(kDigits) * rows * ((K + 7) / 8 * 8));
+  d.exps = c.alloc<int>(size_t(rows));
+  return d;
+}
+
+// Exponents and digits of those of the two sides that are wanted.
+void split_sides(Ctx& c, const SplitSide* side, int want0, int want1, int64_t K, int64_t Kp) {
+  if (c.sizing()) return;
+  int want[2] = {want0, want1};
+  for (int i = 0; i < 2; ++i) {
+    const SplitSide& s = side[i];
+    if (!want[i] || K <= 256 || s.K.n > 1) continue;
+    want[i] = 0;
+    LongRows a{s.x, s.R, s.k_is_s1 ? s.K.m[0].s1 : s.K.m[0].s0, s.rows, K, Kp, K, s.exps, s.dig};
+    // enough CTAs of the exponent kernels to cover the SMs twice
+    const int64_t rb = s.kfast ? 8 : 32, rblocks = (s.rows + rb - 1) / rb;
+    const int64_t least = s.kfast ? 512 : 256, want_ctas = 2 * sm_count_linalg();
+    if (rblocks < want_ctas) a.kc = std::min(K, std::max(least, K * rblocks / want_ctas));
+    const int64_t chunks = (K + a.kc - 1) / a.kc;
+    CTM_REQUIRE(chunks <= 65535, CTM_ERR_UNSUPPORTED, "einsum: grid too large");
+    if (chunks > 1)
+      CTM_CUDA(cudaMemsetAsync(s.exps, 0, sizeof(int) * size_t(s.rows), c.stream));
+    {
+      KernelTimer kt(c.stream, "long_exponents_kernel", kUnitByte, 8.0 * double(s.rows) * K);
+      const dim3 grid(unsigned(rblocks), unsigned(chunks), 1);
+      if (s.kfast) long_exponents_k_kernel<<<grid, 256, 0, c.stream>>>(a);
+      else long_exponents_r_kernel<<<grid, 512, 0, c.stream>>>(a);
+      CTM_LAUNCH_CHECK();
+    }
+    KernelTimer kt(c.stream, "long_split_kernel", kUnitByte, 24.0 * double(s.rows) * K);
+    const int64_t ctas = s.kfast ? ((s.rows + 7) / 8 * ((Kp + 31) / 32) + 7) / 8
+                                 : (s.rows + 31) / 32 * ((Kp + 63) / 64);
+    CTM_REQUIRE(ctas < (int64_t(1) << 31), CTM_ERR_UNSUPPORTED, "einsum: grid too large");
+    if (s.kfast) long_split_kernel<true><<<unsigned(ctas), 256, 0, c.stream>>>(a);
+    else long_split_kernel<false><<<unsigned(ctas), 256, 0, c.stream>>>(a);
+    CTM_LAUNCH_CHECK();
+  }
+  if (!want[0] && !want[1]) return;
+  SplitArgs sa{};
+  sa.s[0] = side[0];
+  sa.s[1] = side[1];
+  sa.K = K;
+  sa.Kp = Kp;
+  sa.kblocks = (K + 255) / 256;
+  sa.kc = int(sa.kblocks == 1 ? Kp : 256);
+  sa.rb = sa.kc <= 64 ? 128 : sa.kc <= 128 ? 64 : 32;
+  auto blocks_of = [&](int i) {
+    return want[i] ? (side[i].rows + sa.rb - 1) / sa.rb * sa.kblocks : int64_t(0);
+  };
+  sa.blocks0 = blocks_of(0);
+  const int64_t blocks = sa.blocks0 + blocks_of(1);
+  const size_t ssm = size_t(sa.rb) * (sa.kc + 1) * sizeof(double);
+  const double entries = ((want[0] ? side[0].rows : 0) + (want[1] ? side[1].rows : 0)) * double(K);
+  if (sa.kblocks > 1) {
+    for (int i = 0; i < 2; ++i)
+      if (want[i])
+        CTM_CUDA(cudaMemsetAsync(side[i].exps, 0, sizeof(int) * size_t(side[i].rows), c.stream));
+    CTM_CUDA(cudaFuncSetAttribute(row_exponent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ssm)));
+    KernelTimer kt(c.stream, "row_exponent_kernel", kUnitByte, 8.0 * entries);
+    row_exponent_kernel<<<unsigned(blocks), 256, ssm, c.stream>>>(sa);
+    CTM_LAUNCH_CHECK();
+  }
+  CTM_CUDA(cudaFuncSetAttribute(split_digits_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ssm)));
+  KernelTimer kt(c.stream, "split_digits_kernel", kUnitByte, 24.0 * entries);
+  split_digits_kernel<<<unsigned(blocks), 256, ssm, c.stream>>>(sa);
+  CTM_LAUNCH_CHECK();
+}
+
 bool unit_stride(const Group& g, bool second) {
   return g.n > 0 && (second ? g.m[g.n - 1].s1 : g.m[g.n - 1].s0) == 1;
 }
@@ -612,13 +783,35 @@ bool unit_stride(const Group& g, bool second) {
 // From about 2e7 multiply-adds on the digit form is the faster one: 256^3 takes
 // 40 us in the FP64 GETT, 400^3 (6.4e7) 70 us in digits and about 150 in the
 // GETT; 5184 x 5184 x 144 takes 0.33 ms against 11 ms.
-bool digits_pay(const GettArgs<double>& p) {
-  if (p.bext != 1 || p.Kt < 1) return false;
-  const double mnk = double(p.Mt) * double(p.Nt) * double(p.Kt);
-  return mnk >= 2.0e7 && p.Kt >= 16 && std::min(p.Mt, p.Nt) >= 16;
+bool digits_pay(int64_t rows, int64_t columns, int64_t K) {
+  return double(rows) * double(columns) * double(K) >= 2.0e7 && K >= 16 &&
+         std::min(rows, columns) >= 16;
 }
 
-void digit_contract(Ctx& c, const GettArgs<double>& p) {
+bool digits_pay(const GettArgs<double>& p) {
+  return p.bext == 1 && digits_pay(p.Mt, p.Nt, p.Kt);
+}
+
+Digits digit_rows(Ctx& c, const View& x, int row_dim) {
+  CTM_REQUIRE(x.nd == 2, CTM_ERR_INVALID, "digit_rows: expects a 2-D view");
+  const int kd = 1 - row_dim;
+  Digits d = alloc_digits(c, x.shape[row_dim], x.shape[kd]);
+  SplitSide s{};
+  s.x = x.p;
+  s.R.n = 1;
+  s.R.m[0] = Mode{x.shape[row_dim], x.stride[row_dim], 0};
+  s.K.n = 1;
+  s.K.m[0] = Mode{x.shape[kd], x.stride[kd], 0};
+  s.rows = d.rows;
+  s.kfast = x.stride[kd] == 1 && x.stride[row_dim] != 1 ? 1 : 0;
+  s.exps = d.exps;
+  s.dig = d.dig;
+  const SplitSide side[2] = {s, s};
+  split_sides(c, side, 1, 0, d.K, (d.K + 7) / 8 * 8);
+  return d;
+}
+
+void digit_contract(Ctx& c, const GettArgs<double>& p, const Digits* pre_a, const Digits* pre_b) {
   const int64_t K = p.Kt, Kp = (K + 7) / 8 * 8;
   const int sms = sm_count_linalg();
   // which operand's rows lie on the tensor-memory lanes: fewer waves of tiles,
@@ -634,9 +827,11 @@ void digit_contract(Ctx& c, const GettArgs<double>& p) {
   const int64_t M = swap ? p.Nt : p.Mt, N = swap ? p.Mt : p.Nt;
   const int nt = best_ntile(N);
   Scope scope(c);
-  bf16* da = c.alloc<bf16>(size_t(kDigits) * M * Kp);
-  bf16* db = c.alloc<bf16>(size_t(kDigits) * N * Kp);
-  int* ex = c.alloc<int>(size_t(M + N));
+  const Digits* pre_m = swap ? pre_b : pre_a;
+  const Digits* pre_n = swap ? pre_a : pre_b;
+  const bool ready_a = pre_m != nullptr, ready_b = pre_n != nullptr;
+  const Digits da = ready_a ? *pre_m : alloc_digits(c, M, K);
+  const Digits db = ready_b ? *pre_n : alloc_digits(c, N, K);
   const int64_t m_tiles = (M + kM - 1) / kM, n_tiles = (N + nt - 1) / nt;
   const int64_t tiles = m_tiles * n_tiles;
   const int64_t stages = (K + kStageK - 1) / kStageK;
@@ -652,44 +847,20 @@ void digit_contract(Ctx& c, const GettArgs<double>& p) {
   if (c.sizing()) return;
   CTM_REQUIRE(tiles * split < (int64_t(1) << 31), CTM_ERR_UNSUPPORTED, "einsum: grid too large");
 
-  SplitArgs sa{};
-  auto side = [&](SplitSide& s, bool first, int64_t rows, int* exps, bf16* dig) {
+  SplitSide side[2];
+  auto fill = [&](SplitSide& s, bool first, int64_t rows, const Digits& d) {
     s.x = first ? p.A : p.B;
     s.R = first ? p.M : p.N;
     s.K = p.K;
     s.k_is_s1 = first ? 0 : 1;
     s.rows = rows;
     s.kfast = unit_stride(p.K, !first) && !unit_stride(s.R, false) ? 1 : 0;
-    s.exps = exps;
-    s.dig = dig;
+    s.exps = d.exps;
+    s.dig = d.dig;
   };
-  side(sa.s[0], !swap, M, ex, da);
-  side(sa.s[1], swap, N, ex + M, db);
-  sa.K = K;
-  sa.Kp = Kp;
-  sa.kblocks = (K + 255) / 256;
-  sa.kc = int(sa.kblocks == 1 ? Kp : 256);
-  sa.rb = sa.kc <= 64 ? 128 : sa.kc <= 128 ? 64 : 32;
-  sa.blocks0 = (M + sa.rb - 1) / sa.rb * sa.kblocks;
-  const int64_t blocks = sa.blocks0 + (N + sa.rb - 1) / sa.rb * sa.kblocks;
-  const size_t ssm = size_t(sa.rb) * (sa.kc + 1) * sizeof(double);
-  if (sa.kblocks > 1) {
-    CTM_CUDA(cudaMemsetAsync(ex, 0, sizeof(int) * size_t(M + N), c.stream));
-    CTM_CUDA(cudaFuncSetAttribute(row_exponent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ssm)));
-    KernelTimer kt(c.stream, "row_exponent_kernel", kUnitByte, 8.0 * double(M + N) * K);
-    row_exponent_kernel<<<unsigned(blocks), 256, ssm, c.stream>>>(sa);
-    CTM_LAUNCH_CHECK();
-  }
-  {
-    CTM_CUDA(cudaFuncSetAttribute(split_digits_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ssm)));
-    KernelTimer kt(c.stream, "split_digits_kernel", kUnitByte, 24.0 * double(M + N) * K);
-    split_digits_kernel<<<unsigned(blocks), 256, ssm, c.stream>>>(sa);
-    CTM_LAUNCH_CHECK();
-  }
-  if (sa.kblocks > 1) {
-    finish_exponents_kernel<<<unsigned((M + N + 255) / 256), 256, 0, c.stream>>>(ex, M + N);
-    CTM_LAUNCH_CHECK();
-  }
+  fill(side[0], !swap, M, da);
+  fill(side[1], swap, N, db);
+  split_sides(c, side, ready_a ? 0 : 1, ready_b ? 0 : 1, K, Kp);
 
   DigitArgs d{};
   d.M = M;
@@ -697,8 +868,8 @@ void digit_contract(Ctx& c, const GettArgs<double>& p) {
   d.K = K;
   d.GM = swap ? p.N : p.M;
   d.GN = swap ? p.M : p.N;
-  d.ea = ex;
-  d.eb = ex + M;
+  d.ea = da.exps;
+  d.eb = db.exps;
   d.C = split > 1 ? part : p.C;
   d.ldm = swap ? 1 : p.Nt;
   d.ldn = swap ? p.Nt : 1;
@@ -721,8 +892,8 @@ void digit_contract(Ctx& c, const GettArgs<double>& p) {
   d.FK = p.K;
   d.swapped = swap ? 1 : 0;
   CUtensorMap tA, tB;
-  digit_map(&tA, da, M, Kp, kM);
-  digit_map(&tB, db, N, Kp, uint32_t(nt));
+  digit_map(&tA, da.dig, M, Kp, kM);
+  digit_map(&tB, db.dig, N, Kp, uint32_t(nt));
   const size_t smem = 1024 + size_t(kStages) * (kABytes + size_t(kDigits) * nt * kStageK * 2) + 128;
   const unsigned grid = unsigned(std::min<int64_t>(tiles * split, sms));
   auto launch = [&](auto kern) {

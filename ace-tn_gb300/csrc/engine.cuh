@@ -1,14 +1,30 @@
 // Internal operations of the CTMRG library (FP64 engine and helpers).
 #pragma once
+#include <cuda_bf16.h>
+
 #include "ctm_common.cuh"
 
 namespace ctm {
 
+// Digits of an operand's rows for FP64 products on the tensor cores (digits.cu),
+// kept by a caller that multiplies with the same matrix several times.
+struct Digits {
+  __nv_bfloat16* dig = nullptr;
+  int* exps = nullptr;
+  int64_t rows = 0, K = 0;
+};
+// Of a 2-D view whose dimension row_dim is kept and the other contracted.
+Digits digit_rows(Ctx& c, const View& x, int row_dim);
+// Whether a product of rows x columns over K takes the digit form.
+bool digits_pay(int64_t rows, int64_t columns, int64_t K);
+
 // C = alpha * einsum(spec, A, B) + beta * C for two-operand contractions whose
 // labels split into batch / row / column / contracted groups (no traces, no
 // outer-only labels).  All views are strided; nothing is copied.
+// da, db: digits of A's and B's rows (one kept and one contracted index each).
 void einsum(Ctx& c, const char* spec, const View& A, const View& B, const View& C,
-            double alpha = 1.0, double beta = 0.0);
+            double alpha = 1.0, double beta = 0.0, const Digits* da = nullptr,
+            const Digits* db = nullptr);
 // The same contraction in FP32 (FP32 FMAs, FP32 accumulation).
 void einsum(Ctx& c, const char* spec, const ViewF& A, const ViewF& B, const ViewF& C,
             double alpha = 1.0, double beta = 0.0);

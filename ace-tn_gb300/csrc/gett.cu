@@ -318,7 +318,8 @@ void splitk_reduce(Ctx& c, const GettArgs<double>& p) { splitk_reduce_impl<doubl
 
 template <class T>
 void einsum_impl(Ctx& c, const char* spec, const ViewT<T>& A, const ViewT<T>& B, const ViewT<T>& C,
-                 double alpha, double beta) {
+                 double alpha, double beta, const Digits* da = nullptr,
+                 const Digits* db = nullptr) {
   std::string s(spec);
   const size_t comma = s.find(','), arrow = s.find("->");
   CTM_REQUIRE(comma != std::string::npos && arrow != std::string::npos, CTM_ERR_INVALID,
@@ -437,7 +438,10 @@ void einsum_impl(Ctx& c, const char* spec, const ViewT<T>& A, const ViewT<T>& B,
   }
   if constexpr (std::is_same<T, double>::value) {
     if (digits_pay(p)) {
-      digit_contract(c, p);
+      CTM_REQUIRE((da == nullptr || (da->rows == p.Mt && da->K == p.Kt && p.K.n <= 1)) &&
+                      (db == nullptr || (db->rows == p.Nt && db->K == p.Kt && p.K.n <= 1)),
+                  CTM_ERR_INVALID, "einsum: digits of another operand in " + s);
+      digit_contract(c, p, da, db);
       return;
     }
   }
@@ -511,8 +515,8 @@ void einsum_impl(Ctx& c, const char* spec, const ViewT<T>& A, const ViewT<T>& B,
 }
 
 void einsum(Ctx& c, const char* spec, const View& A, const View& B, const View& C, double alpha,
-            double beta) {
-  einsum_impl<double>(c, spec, A, B, C, alpha, beta);
+            double beta, const Digits* da, const Digits* db) {
+  einsum_impl<double>(c, spec, A, B, C, alpha, beta, da, db);
 }
 
 void einsum(Ctx& c, const char* spec, const ViewF& A, const ViewF& B, const ViewF& C, double alpha,

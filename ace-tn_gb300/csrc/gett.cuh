@@ -58,7 +58,8 @@ __device__ __forceinline__ void decode(const Group& g, int64_t idx, int64_t& o0,
 // C = alpha A B + beta C by exact digit products on the tensor cores (no batch
 // mode), and whether that is the faster form for this contraction.
 bool digits_pay(const GettArgs<double>& p);
-void digit_contract(Ctx& c, const GettArgs<double>& p);
+void digit_contract(Ctx& c, const GettArgs<double>& p, const Digits* pre_a = nullptr,
+                    const Digits* pre_b = nullptr);
 // Sum of the split-K partials p.part into p.C.
 void splitk_reduce(Ctx& c, const GettArgs<double>& p);
 
