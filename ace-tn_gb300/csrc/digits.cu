@@ -32,20 +32,11 @@
 
 #include <algorithm>
 
-#include "gett.cuh"
-#include "tcgen05.cuh"
+#include "digits.cuh"
 
 namespace ctm {
 
 namespace {
-
-using bf16 = __nv_bfloat16;
-
-constexpr int kDigits = 8;
-// A row's scale is kept as the largest exponent field of its entries: |x| <
-// 2^(row_exponent(field) - 1023).  Field 2047: a non-finite entry, no digits.
-constexpr int kBadField = 2047;
-__device__ __forceinline__ int row_exponent(int field) { return max(field, 1) + 1; }
 
 // ------------------------------------------------------------- splitting
 struct SplitSide {
@@ -66,10 +57,6 @@ struct SplitArgs {
   int64_t blocks0;       // CTAs of side 0
   int64_t kblocks;       // K blocks (1: exponents are found here)
 };
-
-__device__ __forceinline__ int exponent_field(double x) {
-  return int((unsigned long long)__double_as_longlong(x) >> 52) & 0x7ff;
-}
 
 // Loads the CTA's rows x indices block into shared memory (row stride kc + 1);
 // walks whichever index has unit stride across the lanes.
@@ -134,46 +121,6 @@ __global__ void __launch_bounds__(256) row_exponent_kernel(const SplitArgs a) {
   const int nr = int(min(int64_t(a.rb), s.rows - r0)), nk = int(min(int64_t(a.kc), a.K - k0));
   row_exponents(a, nr, nk, sx, s_e);
   for (int r = threadIdx.x; r < nr; r += blockDim.x) atomicMax(s.exps + r0 + r, s_e[r]);
-}
-
-// Digit b (0..7, 0 the least significant) of the biased word w as BF16 bits in
-// the upper half: the byte minus 128, exact.
-__device__ __forceinline__ uint32_t digit_f32(uint32_t w, int byte) {
-  const uint32_t u = __byte_perm(w, 0x4B000000u, 0x7650u | uint32_t(byte));
-  return __float_as_uint(__uint_as_float(u) - 8388736.f);  // 2^23 + 128
-}
-
-// The eight digits of eight consecutive entries, 16 bytes per digit plane.
-__device__ __forceinline__ void write_digits(const double (&x)[8], int E, bf16* dst,
-                                             int64_t plane) {
-  uint32_t lo[8], hi[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const long long bits = __double_as_longlong(x[i]);
-    const int ex = int((unsigned long long)bits >> 52) & 0x7ff;
-    const long long mant = (bits & 0xfffffffffffffll) | (ex != 0 ? 0x10000000000000ll : 0ll);
-    const int sh = max(ex, 1) - E + 10;  // x 2^62 / 2^(E - 1023) = mant 2^sh, sh <= 9
-    long long t;
-    if (sh >= 0) t = mant << sh;
-    else if (sh >= -54) t = (mant + (1ll << (-sh - 1))) >> -sh;
-    else t = 0;
-    if (bits < 0) t = -t;
-    const unsigned long long u =
-        ((unsigned long long)t + 0x0080808080808080ull) ^ 0x8000000000000000ull;
-    lo[i] = uint32_t(u);
-    hi[i] = uint32_t(u >> 32);
-  }
-#pragma unroll
-  for (int d = 0; d < kDigits; ++d) {  // digit 0 is the top byte
-    uint32_t w[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const uint32_t f0 = digit_f32(d < 4 ? hi[2 * i] : lo[2 * i], 3 - (d & 3));
-      const uint32_t f1 = digit_f32(d < 4 ? hi[2 * i + 1] : lo[2 * i + 1], 3 - (d & 3));
-      w[i] = __byte_perm(f0, f1, 0x7632);
-    }
-    *reinterpret_cast<uint4*>(dst + int64_t(d) * plane) = make_uint4(w[0], w[1], w[2], w[3]);
-  }
 }
 
 __global__ void __launch_bounds__(256) split_digits_kernel(const SplitArgs a) {
@@ -333,87 +280,8 @@ struct DigitArgs {
   int stages_per_split; // multiple of kChunkStages
   int stages_total;
   int* status;
-  // operands, for rows and columns without digits
-  const double* a;
-  const double* b;
-  Group FM, FN, FK;     // FM.m[].s0, FN.m[].s0, FK: (row operand, column operand) strides
-  int swapped;          // the row operand is the contraction's second one
+  ChainArgs chain;
 };
-
-// (hi 2^32 + lo) 2^e rounded to nearest even.
-__device__ __forceinline__ double round_96(long long hi, uint32_t lo, int e) {
-  const bool neg = hi < 0;
-  if (neg) {
-    lo = 0u - lo;
-    hi = ~hi + (lo == 0u ? 1 : 0);
-  }
-  if (hi == 0 && lo == 0u) return 0.0;
-  const int lz = hi != 0 ? __clzll(hi) : 64 + __clz(int(lo));
-  unsigned long long m;
-  uint32_t rest = 0u;
-  if (lz >= 64) {
-    m = (unsigned long long)lo << (lz - 32);
-  } else if (lz >= 32) {
-    m = ((unsigned long long)hi << lz) | ((unsigned long long)lo << (lz - 32));
-  } else {
-    m = ((unsigned long long)hi << lz) | (((unsigned long long)lo << lz) >> 32);
-    rest = lo << lz;
-  }
-  unsigned long long r = m >> 11;  // 53 bits
-  const uint32_t low = uint32_t(m) & 0x7ffu;
-  if (low > 0x400u || (low == 0x400u && (rest != 0u || (r & 1ull) != 0ull))) ++r;
-  const int ef = 95 - lz + e + 1023;  // exponent field of the leading bit
-  double v;
-  if (ef >= 1 && ef < 2046)
-    v = __longlong_as_double((long long)(((unsigned long long)(ef - 1) << 52) + r));
-  else  // overflow and gradual underflow
-    v = scalbn(double((long long)r), ef - 1023 - 52);
-  return neg ? -v : v;
-}
-
-// One output by the FMA chain, for rows and columns with non-finite entries.
-__device__ __noinline__ double chain_dot(const DigitArgs& p, int64_t m, int64_t n, int64_t k0,
-                                         int64_t k1) {
-  int64_t mo, no, t0, t1;
-  decode(p.FM, m, mo, t0);
-  decode(p.FN, n, no, t0);
-  double v = 0.0;
-  for (int64_t k = k0; k < k1; ++k) {
-    decode(p.FK, k, t0, t1);
-    v = fma(p.a[mo + (p.swapped ? t1 : t0)], p.b[no + (p.swapped ? t0 : t1)], v);
-  }
-  return v;
-}
-
-__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z,
-                                            uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(smem_u32(dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
-      : "memory");
-}
-
-__device__ __forceinline__ void tmem_ld4(uint32_t taddr, float (&v)[4]) {
-  uint32_t r[4];
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(taddr));
-#pragma unroll
-  for (int i = 0; i < 4; ++i) v[i] = __uint_as_float(r[i]);
-}
-
-// Integer value of f, |f| < 2^22 (an FP32 addition; the conversion unit does
-// 16 values per cycle and SM, these adders 128).
-__device__ __forceinline__ int int_small(float f) {
-  return __float_as_int(f + 12582912.f) - 0x4B400000;
-}
-// The same for |f| < 2^25: multiples of 8 and the rest.
-__device__ __forceinline__ int int_wide(float f) {
-  const float t = f + 100663296.f;  // 1.5 2^26: unit 8
-  const float r = f - (t - 100663296.f);
-  return 8 * (__float_as_int(t) - 0x4CC00000) + int_small(r);
-}
 
 // Tiles of 128 rows x ntile columns, persistent over blockIdx.x.  The eight
 // accumulators of a tile fill tensor memory (8 x 64 columns).  One stage holds
@@ -610,15 +478,9 @@ __global__ void __launch_bounds__(kDThreads, 1)
             for (int j = 0; j < 4; ++j) asm volatile("" : "+f"(f[s][j]));
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            const int g01 = int_small(f[0][j]) * 256 + int_small(f[1][j]);
-            const int g23 = int_wide(f[2][j]) * 256 + int_wide(f[3][j]);
-            const long long h = (long long)g01 * 65536 + g23;
-            long long l = (long long)int_wide(f[4][j]) * 16777216 + lo[c + j];
-            l += (long long)__float2int_rn(f[5][j]) * 65536;
-            l += (long long)__float2int_rn(f[6][j]) * 256;
-            l += __float2int_rn(f[7][j]);
-            lo[c + j] = uint32_t(l);
-            hi[c + j] += h + (l >> 32);
+            const float v[kDigits] = {f[0][j], f[1][j], f[2][j], f[3][j],
+                                      f[4][j], f[5][j], f[6][j], f[7][j]};
+            add_groups(v, hi[c + j], lo[c + j]);
           }
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -642,7 +504,7 @@ __global__ void __launch_bounds__(kDThreads, 1)
           if (off < 0) continue;
           // units of 2^-68 of the scales (digit s of the product: 2^(-12 - 8 s))
           double v;
-          if (er == kBadField || e == kBadField) v = chain_dot(p, row, int64_t(n0) + half * kHalf + c, k0, k1);
+          if (er == kBadField || e == kBadField) v = chain_dot(p.chain, row, int64_t(n0) + half * kHalf + c, k0, k1);
           else v = round_96(hi[c], lo[c], row_exponent(er) + row_exponent(e) - 2 * 1023 - 68);
           if (p.split == 1 && !(p.alpha == 1.0 && p.beta == 0.0)) {
             v *= p.alpha;
@@ -811,7 +673,28 @@ Digits digit_rows(Ctx& c, const View& x, int row_dim) {
   return d;
 }
 
+Digits operand_digits(Ctx& c, const GettArgs<double>& p, bool first) {
+  const Digits d = alloc_digits(c, first ? p.Mt : p.Nt, p.Kt);
+  SplitSide s{};
+  s.x = first ? p.A : p.B;
+  s.R = first ? p.M : p.N;
+  s.K = p.K;
+  s.k_is_s1 = first ? 0 : 1;
+  s.rows = d.rows;
+  s.kfast = unit_stride(p.K, !first) && !unit_stride(s.R, false) ? 1 : 0;
+  s.exps = d.exps;
+  s.dig = d.dig;
+  const SplitSide side[2] = {s, s};
+  split_sides(c, side, 1, 0, d.K, (d.K + 7) / 8 * 8);
+  return d;
+}
+
 void digit_contract(Ctx& c, const GettArgs<double>& p, const Digits* pre_a, const Digits* pre_b) {
+  bool stream_swap = false;
+  if (pre_a == nullptr && pre_b == nullptr && stream_fits(p, stream_swap)) {
+    stream_contract(c, p, stream_swap);
+    return;
+  }
   const int64_t K = p.Kt, Kp = (K + 7) / 8 * 8;
   const int sms = sm_count_linalg();
   // which operand's rows lie on the tensor-memory lanes: fewer waves of tiles,
@@ -885,12 +768,7 @@ void digit_contract(Ctx& c, const GettArgs<double>& p, const Digits* pre_a, cons
   d.stages_per_split = int(per);
   d.stages_total = int(stages);
   d.status = status_flags(c);
-  d.a = swap ? p.B : p.A;
-  d.b = swap ? p.A : p.B;
-  d.FM = d.GM;
-  d.FN = d.GN;
-  d.FK = p.K;
-  d.swapped = swap ? 1 : 0;
+  d.chain = chain_args(p, swap);
   CUtensorMap tA, tB;
   digit_map(&tA, da.dig, M, Kp, kM);
   digit_map(&tB, db.dig, N, Kp, uint32_t(nt));

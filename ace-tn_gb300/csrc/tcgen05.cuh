@@ -82,7 +82,7 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
 }
 
 // Shared-memory matrix descriptor: K-major operand with rows of bk BF16
-// (bk = 64: 128-byte swizzle; bk = 32: 64-byte swizzle), 8-row core-matrix
+// (bk = 64: 128-byte swizzle; 32: 64-byte; 16: 32-byte), 8-row core-matrix
 // groups 8 * 2 * bk bytes apart.
 __device__ __forceinline__ uint64_t smem_desc(const void* p, int bk) {
   const uint64_t addr = smem_u32(p);
@@ -90,7 +90,7 @@ __device__ __forceinline__ uint64_t smem_desc(const void* p, int bk) {
   d |= uint64_t(1) << 16;                            // leading byte offset (unused when swizzled)
   d |= uint64_t((16 * bk) >> 4) << 32;               // stride byte offset
   d |= uint64_t(1) << 46;                            // descriptor version (tcgen05)
-  d |= uint64_t(bk == 64 ? 2 : 4) << 61;             // SWIZZLE_128B / SWIZZLE_64B
+  d |= uint64_t(bk == 64 ? 2 : bk == 32 ? 4 : 6) << 61;  // SWIZZLE_128B / 64B / 32B
   return d;
 }
 

@@ -129,3 +129,43 @@ def test_strided_operands():
         mine = gb.ProjectorCalculator.make_quarter_tensor(s, k)[0]
         # chains of 40, 40, 16 and 32 terms in either order: 1e-13 of the largest
         assert float((mine - q / q.abs().max()).abs().max()) < 1e-13
+
+
+# long side, small side, contracted: the streaming kernel's groups of columns
+# (16, 32, 48, 64 wide), blocks of 16 indices, one and several phases
+STREAM = [(80000, 16, 16), (8192, 128, 20), (12001, 72, 36), (17000, 32, 37), (9000, 64, 48),
+          (9999, 33, 64), (12800, 17, 96), (8200, 36, 72), (8193, 48, 81), (10000, 49, 49),
+          (8192, 96, 33), (8300, 100, 129), (9001, 128, 64), (8192, 65, 176), (8320, 16, 191),
+          (12288, 40, 192), (30000, 24, 30)]
+
+
+@pytest.mark.parametrize("long,short,k", STREAM)
+@pytest.mark.parametrize("second", [False, True])
+def test_long_operands(long, short, k, second):
+    assert long * short * k >= 2e7 and long >= 8192  # the streaming route
+    rng = np.random.default_rng(long + short + k)
+    a = rng.standard_normal((long, k)) * 2.0 ** rng.integers(-30, 30, (long, 1))
+    b = rng.standard_normal((k, short))
+    a[7] = 0.0
+    rows = np.unique(np.concatenate([np.arange(140), rng.integers(0, long, 200),
+                                     np.arange(long - 140, long)]))
+    c = run(np.ascontiguousarray(b.T), np.ascontiguousarray(a.T)).T if second else run(a, b)
+    check(a[rows], b, c[rows], splits=0)
+    scale = np.abs(a).max(1)[:, None] * np.abs(b).max(0)[None, :]  # and every entry loosely
+    assert np.all(np.abs(c - a @ b) <= k * 2.0 ** -50 * scale)
+
+
+def test_long_operand_non_finite_and_extreme():
+    rng = np.random.default_rng(9)
+    a, b = rng.standard_normal((9000, 50)), rng.standard_normal((50, 60))
+    a[5, 3], a[8999, 49], b[7, 59] = np.inf, np.nan, -np.inf
+    b[3, 10] = 0.0
+    c, ref = run(a, b), a @ b
+    assert np.array_equal(np.isnan(c), np.isnan(ref)) and np.array_equal(np.isinf(c), np.isinf(ref))
+    fine = np.isfinite(ref)
+    assert np.abs(c[fine] - ref[fine]).max() < 1e-12
+    x = -sum(128 * 256.0 ** -i for i in range(1, 8)) * 2.0 ** -6
+    for k in (36, 192):
+        a, b = np.full((8192, k), x), np.full((k, 80), x)
+        a[:, 0], b[0] = 0.999, 0.999
+        check(a[:200], b, run(a, b)[:200], splits=0)
