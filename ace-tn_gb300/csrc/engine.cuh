@@ -59,6 +59,12 @@ void orthonormalize(Ctx& c, double* Y, int64_t n, int64_t q, double* R, int stag
 // matrix fits.
 bool householder_cluster_fits(int64_t n, int64_t q);
 void householder_cluster(Ctx& c, double* Y, int64_t n, int64_t q, double* R);
+// L^-1 (lower) and, when not null, L^T (upper) of G + shift_factor tr(G) I = L L^T
+// (q x q) by one cluster, and whether q fits.  A pivot that is not positive gives
+// a zero row of both and sets bit 1 of *flags.
+bool cholesky_cluster_fits(int64_t q);
+void cholesky_cluster(Ctx& c, const double* G, int64_t q, double shift_factor, double* Linv,
+                      double* Lt, int* flags);
 // Shifted Cholesky-QR3 of Y without the Householder fallback: bit 1 of
 // *failed (device, cleared first) is set when the result is not orthonormal
 // to working precision, and Y and R then mean nothing.

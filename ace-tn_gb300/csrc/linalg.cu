@@ -1350,7 +1350,17 @@ void orthonormalize_impl(Ctx& c, T* Y, int64_t n, int64_t q, T* R, int stages,
     for (int stage = 0; stage < stages; ++stage) {
       einsum(c, "ia,ib->ab", ViewT<T>(cur, {n, q}), ViewT<T>(cur, {n, q}), ViewT<T>(G, {q, q}));
       const int mode = stage < shifted_stages ? (sizeof(T) == 8 ? 1 : 2) : 0;
-      if (!c.sizing())
+      bool done = false;
+      if constexpr (sizeof(T) == 8) {
+        // 11 (n q + q (q + 1)) u tr(G) in the shifted stage
+        const double f = mode == 1 ? 11.0 * (double(n) * q + double(q) * (q + 1)) *
+                                         1.1102230246251565e-16
+                                   : 0.0;
+        done = cholesky_cluster_fits(q);
+        if (done && !c.sizing())
+          cholesky_cluster(c, G, q, f, Li, R != nullptr ? Lt : nullptr, flags);
+      }
+      if (!done && !c.sizing())
         cholesky<T>(c.stream, G, q, n, mode, Wk, Ek, nullptr, Li, R != nullptr ? Lt : nullptr,
                     flags);
       // nxt = cur @ Linv^T
