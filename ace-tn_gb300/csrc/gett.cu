@@ -501,12 +501,13 @@ void einsum_impl(Ctx& c, const char* spec, const ViewT<T>& A, const ViewT<T>& B,
   {
     const double flops = 2.0 * double(p.Mt) * p.Nt * p.Kt * bext;
     KernelTimer timer(c.stream, sizeof(T) == 8 ? kTagGettF64 : kTagGettF32, flops);
-    KernelTimer kt(c.stream, sizeof(T) == 8 ? "gett_kernel<double>" : "gett_kernel<float>",
+    KernelTimer kt(c.stream, sizeof(T) == 8 ? "gett_kernel<double>" : "gett_f32_kernel",
                    kUnitFlop, flops);
-    if (tile == 4) {
-      gett_kernel<T, 4><<<grid, NT, 0, c.stream>>>(p);
-    } else if constexpr (sizeof(T) == 8) {
-      if (tile == 2) gett_kernel<T, 2><<<grid, NT, 0, c.stream>>>(p);
+    if constexpr (sizeof(T) == 4) {
+      gett_f32(c, p);
+    } else {
+      if (tile == 4) gett_kernel<T, 4><<<grid, NT, 0, c.stream>>>(p);
+      else if (tile == 2) gett_kernel<T, 2><<<grid, NT, 0, c.stream>>>(p);
       else gett_kernel<T, 1><<<grid, NT, 0, c.stream>>>(p);
     }
     CTM_LAUNCH_CHECK();

@@ -60,6 +60,8 @@ __device__ __forceinline__ void decode(const Group& g, int64_t idx, int64_t& o0,
 bool digits_pay(const GettArgs<double>& p);
 void digit_contract(Ctx& c, const GettArgs<double>& p, const Digits* pre_a = nullptr,
                     const Digits* pre_b = nullptr);
+// One FP32 contraction (p.splitk and p.kchunk set).
+void gett_f32(Ctx& c, GettArgs<float>& p);
 // Sum of the split-K partials p.part into p.C.
 void splitk_reduce(Ctx& c, const GettArgs<double>& p);
 
