@@ -597,6 +597,131 @@ __global__ void __launch_bounds__(kCh > 0 ? 128 * kCh : 1024) jacobi_onesided_f3
   }
 }
 
+// jacobi_onesided_f32_kernel for matrices beyond one CTA's shared memory: the same
+// pairs in the same rounds with the same arithmetic (bit for bit), but row r lives
+// in the shared memory of CTA r mod P of a cluster instead of global memory, and
+// pair k of a round is rotated by CTA k mod P through distributed shared memory.
+// kCh > 0: ld = 32 kCh, the two data rows held in registers; 0: any ld.
+// (q = 272: 27 ms on one CTA from L2, about 12 us for each of 271 rounds a sweep.)
+template <int kCh>
+__global__ void __launch_bounds__(kCh > 0 ? 160 : 512)
+    jacobi_spread_f32_kernel(const float* Mc_g, int q, int pp, float* Jc_g, float* norms,
+                             int max_sweeps, float tol, int* flags) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int P = int(cluster.num_blocks()), me = int(cluster.block_rank());
+  extern __shared__ __align__(16) float spm[];  // own rows: ld of Mc, then ld of Jc
+  const int ld = jacobi_ld(q), RS = 2 * ld;
+  __shared__ int s_rot[64];
+  const int mine = (q - me + P - 1) / P;
+  for (int idx = threadIdx.x; idx < mine * ld; idx += blockDim.x) {
+    const int l = idx / ld, c = idx - l * ld, r = l * P + me;
+    spm[l * RS + c] = c < q ? Mc_g[size_t(r) * q + c] : 0.f;
+    spm[l * RS + ld + c] = (r == c) ? 1.f : 0.f;
+  }
+  for (int i = threadIdx.x; i < 64; i += blockDim.x) s_rot[i] = 0;
+  const int npairs = pp / 2;
+  const int g = threadIdx.x >> 3, sub = threadIdx.x & 7;
+  const int ngroups = blockDim.x >> 3;
+  const int nchunk = kCh > 0 ? kCh : ld / 32;
+  const int trips = ((npairs + P - 1) / P + ngroups - 1) / ngroups;
+  cluster.sync();
+  int sweep = 0;
+  for (; sweep < max_sweeps; ++sweep) {
+    for (int r = 0; r < pp - 1; ++r) {
+      for (int trip = 0; trip < trips; ++trip) {
+        const int k = (trip * ngroups + g) * P + me;
+        int i = 0, j = q;
+        if (k < npairs) {
+          const int i0 = k == 0 ? 0 : ((k - 1 + r) % (pp - 1)) + 1;
+          const int k2 = pp - 1 - k;
+          const int j0 = k2 == 0 ? 0 : ((k2 - 1 + r) % (pp - 1)) + 1;
+          i = min(i0, j0);
+          j = max(i0, j0);
+        }
+        const bool active = j < q;
+        const int jj = active ? j : i;
+        float* ra = cluster.map_shared_rank(spm, i % P) + (i / P) * RS;
+        float* rb = cluster.map_shared_rank(spm, jj % P) + (jj / P) * RS;
+        float4* a = reinterpret_cast<float4*>(ra) + sub;
+        float4* b = reinterpret_cast<float4*>(rb) + sub;
+        constexpr int kR = kCh > 0 ? kCh : 1;
+        float4 xa[kR], xb[kR];
+        float al = 0.f, be = 0.f, ga = 0.f;
+        if (active) {
+          if (kCh > 0) {
+#pragma unroll
+            for (int m = 0; m < kR; ++m) {
+              xa[m] = a[8 * m];
+              xb[m] = b[8 * m];
+            }
+          }
+#pragma unroll
+          for (int m = 0; m < (kCh > 0 ? kR : nchunk); ++m) {
+            const float4 x = kCh > 0 ? xa[m % kR] : a[8 * m], y = kCh > 0 ? xb[m % kR] : b[8 * m];
+            al = fmaf(x.x, x.x, fmaf(x.y, x.y, fmaf(x.z, x.z, fmaf(x.w, x.w, al))));
+            be = fmaf(y.x, y.x, fmaf(y.y, y.y, fmaf(y.z, y.z, fmaf(y.w, y.w, be))));
+            ga = fmaf(x.x, y.x, fmaf(x.y, y.y, fmaf(x.z, y.z, fmaf(x.w, y.w, ga))));
+          }
+        }
+        for (int o = 4; o > 0; o >>= 1) {
+          al += __shfl_xor_sync(0xffffffffu, al, o);
+          be += __shfl_xor_sync(0xffffffffu, be, o);
+          ga += __shfl_xor_sync(0xffffffffu, ga, o);
+        }
+        if (!active || al == 0.f || be == 0.f || !(fabsf(ga) > tol * sqrtf(al) * sqrtf(be)))
+          continue;
+        const float zeta = (be - al) / (2.f * ga);
+        const float t = copysignf(1.f, zeta) / (fabsf(zeta) + sqrtf(1.f + zeta * zeta));
+        const float cs = 1.f / sqrtf(1.f + t * t), sn = cs * t, tau = sn / (1.f + cs);
+        float4* ja = reinterpret_cast<float4*>(ra + ld) + sub;
+        float4* jb = reinterpret_cast<float4*>(rb + ld) + sub;
+        auto rot = [&](float4* pa, float4* pb, const float4 x, const float4 y) {
+          *pa = make_float4(fmaf(-sn, fmaf(tau, x.x, y.x), x.x), fmaf(-sn, fmaf(tau, x.y, y.y), x.y),
+                            fmaf(-sn, fmaf(tau, x.z, y.z), x.z), fmaf(-sn, fmaf(tau, x.w, y.w), x.w));
+          *pb = make_float4(fmaf(sn, fmaf(-tau, y.x, x.x), y.x), fmaf(sn, fmaf(-tau, y.y, x.y), y.y),
+                            fmaf(sn, fmaf(-tau, y.z, x.z), y.z), fmaf(sn, fmaf(-tau, y.w, x.w), y.w));
+        };
+        if (kCh > 0) {
+          float4 u[kR], v[kR];
+#pragma unroll
+          for (int m = 0; m < kR; ++m) {
+            u[m] = ja[8 * m];
+            v[m] = jb[8 * m];
+          }
+#pragma unroll
+          for (int m = 0; m < kR; ++m) {
+            rot(a + 8 * m, b + 8 * m, xa[m], xb[m]);
+            rot(ja + 8 * m, jb + 8 * m, u[m], v[m]);
+          }
+        } else {
+          for (int m = 0; m < nchunk; ++m) {
+            rot(a + 8 * m, b + 8 * m, a[8 * m], b[8 * m]);
+            rot(ja + 8 * m, jb + 8 * m, ja[8 * m], jb[8 * m]);
+          }
+        }
+        if (sub == 0) s_rot[sweep] = 1;
+      }
+      cluster.sync();
+    }
+    int any = 0;
+    for (int k = 0; k < P; ++k) any |= *cluster.map_shared_rank(&s_rot[sweep], k);
+    if (any == 0) break;  // every CTA reads the same words: all leave together
+  }
+  if (threadIdx.x == 0 && me == 0 && sweep == max_sweeps) atomicOr(flags, 2);
+  for (int l = threadIdx.x; l < mine; l += blockDim.x) {
+    const float* row = spm + l * RS;
+    float nn = 0.f;
+    for (int t = 0; t < q; ++t) nn = fmaf(row[t], row[t], nn);
+    norms[l * P + me] = sqrtf(nn);
+  }
+  for (int idx = threadIdx.x; idx < mine * q; idx += blockDim.x) {
+    const int l = idx / q, c = idx - l * q;
+    Jc_g[size_t(l * P + me) * q + c] = spm[l * RS + ld + c];
+  }
+  cluster.sync();  // no CTA leaves while others can still read its shared memory
+}
+
 // One plane rotation of the one-sided Jacobi on a pair of rows (ra, rb) of
 // kCh float4 chunks per thread, kTP threads per pair (thread sub owns chunks
 // sub + kTP m); the accumulated-rotation rows follow at ra + ld, rb + ld.
@@ -1476,11 +1601,15 @@ __global__ void scale_columns_f32_kernel(float* x, int64_t rows, int cols, const
 void jacobi_rotations_impl(Ctx& c, const float* Mc, int64_t q, float* Jc, float* norms,
                            int max_sweeps, int* flags) {
   Scope scope(c);
-  // the Jacobi matrices stay in shared memory up to q = 160, in global
-  // memory (L2) beyond
+  // the Jacobi matrices stay in shared memory up to q = 160
   const size_t wjac = size_t(2) * q * jacobi_ld(int(q)) * sizeof(float);
   const bool jac_smem = wjac <= (227 - 1) * 1024;
-  float* Wg = jac_smem ? nullptr : c.alloc<float>(size_t(2) * q * jacobi_ld(int(q)));
+  // beyond that and the block form below: rows spread over a cluster (q <= 640 with 16
+  // CTAs), in global memory (L2) beyond
+  const int ctas = max_cluster_ctas();
+  const size_t sp = size_t((q + ctas - 1) / ctas) * 2 * jacobi_ld(int(q)) * sizeof(float);
+  const bool spread = !jac_smem && sp <= size_t(224) * 1024;
+  float* Wg = jac_smem || spread ? nullptr : c.alloc<float>(size_t(2) * q * jacobi_ld(int(q)));
   const int64_t pp = q + (q & 1);
   if (c.sizing()) return;
   // q >= 96: the block Jacobi on a cluster of kJacobiCluster CTAs with
@@ -1546,6 +1675,29 @@ void jacobi_rotations_impl(Ctx& c, const float* Mc, int64_t q, float* Jc, float*
       case 5: launch(jacobi_onesided_f32_kernel<true, 5>); break;
       default: launch(jacobi_onesided_f32_kernel<true, 0>); break;
     }
+  } else if (spread) {
+    auto launch = [&](auto kern) {
+      CTM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sp)));
+      CTM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+      KernelTimer kt(c.stream, "jacobi_spread_f32_kernel", kUnitFlop, 0.0);
+      const int64_t pairs = (pp / 2 + ctas - 1) / ctas;
+      cudaLaunchConfig_t cfg{};
+      cfg.gridDim = dim3(unsigned(ctas));
+      cfg.blockDim = dim3(unsigned(std::min<int64_t>(512, (pairs * 8 + 31) / 32 * 32)));
+      cfg.dynamicSmemBytes = sp;
+      cfg.stream = c.stream;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = unsigned(ctas);
+      attr[0].val.clusterDim.y = 1;
+      attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      CTM_CUDA(cudaLaunchKernelEx(&cfg, kern, Mc, int(q), int(pp), Jc, norms, max_sweeps, 4e-6f,
+                                  flags));
+    };
+    if (jacobi_ld(int(q)) / 32 == 9) launch(jacobi_spread_f32_kernel<9>);
+    else launch(jacobi_spread_f32_kernel<0>);
   } else {
     KernelTimer kt(c.stream, "jacobi_onesided_f32_kernel", kUnitFlop, 0.0);
     jacobi_onesided_f32_kernel<false, 0><<<1, jthreads, 0, c.stream>>>(
