@@ -556,10 +556,13 @@ void site_rdm_chain(Ctx& c, const ViewT<T>& c1, const ViewT<T>& c2, const ViewT<
   const int64_t E3 = e3.shape[0];
   T* t1b = c.alloc<T>(size_t(C4) * D * D * E3 * D * D);
   einsum(c, "aclL,eadD->clLedD", V(t1a, {A4, C4, D, D}), e3, V(t1b, {C4, D, D, E3, D, D}));
-  // einsum("clLedD,LURDP->cledURP", tmp1, conj(a1))
+  // einsum("clLedD,LURDP->cledURP", tmp1, conj(a1)), stored as eRcUldP: the last
+  // contraction sums over e, R, c, U in that order and takes all of ldP at each step,
+  // so it reads this operand once, front to back.  (As cledURP every pass over c and U
+  // fetched 8 of 48 bytes.)
   T* t1c = c.alloc<T>(size_t(C4) * D * E3 * D * D * D * d);
-  einsum(c, "clLedD,LURDP->cledURP", V(t1b, {C4, D, D, E3, D, D}), a1,
-         V(t1c, {C4, D, E3, D, D, D, d}));
+  einsum(c, "clLedD,LURDP->eRcUldP", V(t1b, {C4, D, D, E3, D, D}), a1,
+         V(t1c, {E3, D, C4, D, D, D, d}));
   // tmp2 = einsum("ab,bcuU->acuU", c1, e1)
   const int64_t A1 = c1.shape[0], C1 = e1.shape[1];
   T* t2 = c.alloc<T>(size_t(A1) * C1 * D * D);
@@ -578,8 +581,8 @@ void site_rdm_chain(Ctx& c, const ViewT<T>& c1, const ViewT<T>& c2, const ViewT<
          V(t3c, {B3, D, D, A1, D, D}));
   // tmp3 = einsum("erRcuU,cledURP->ruldP", tmp3, tmp1)
   T* t3d = c.alloc<T>(size_t(D) * D * D * D * d);
-  einsum(c, "erRcuU,cledURP->ruldP", V(t3c, {B3, D, D, A1, D, D}),
-         V(t1c, {C4, D, E3, D, D, D, d}), V(t3d, {D, D, D, D, d}));
+  einsum(c, "erRcuU,eRcUldP->ruldP", V(t3c, {B3, D, D, A1, D, D}),
+         V(t1c, {E3, D, C4, D, D, D, d}), V(t3d, {D, D, D, D, d}));
   // rdm = einsum("ruldP,lurdp->Pp", tmp3, a1)
   einsum(c, "ruldP,lurdp->Pp", V(t3d, {D, D, D, D, d}), a1, V(out, {d, d}));
 }

@@ -53,25 +53,24 @@ struct SplitSide {
 struct SplitArgs {
   SplitSide s[2];
   int64_t K, Kp;
-  int rb, kc;            // rows and contracted indices per CTA
+  int rb, kc;            // rows per CTA; Kp
   int64_t blocks0;       // CTAs of side 0
-  int64_t kblocks;       // K blocks (1: exponents are found here)
 };
 
-// Loads the CTA's rows x indices block into shared memory (row stride kc + 1);
-// walks whichever index has unit stride across the lanes.
-__device__ void load_block(const SplitSide& s, const SplitArgs& a, int64_t r0, int64_t k0,
-                           double* sx, int64_t* s_ro, int64_t* s_ko) {
+// Loads the CTA's rows into shared memory (row stride kc + 1); walks whichever
+// index has unit stride across the lanes.
+__device__ void load_block(const SplitSide& s, const SplitArgs& a, int64_t r0, double* sx,
+                           int64_t* s_ro, int64_t* s_ko) {
   const int tid = threadIdx.x, nth = blockDim.x, lane = tid & 31, warp = tid >> 5;
   const int nwarps = nth >> 5;
-  const int nr = int(min(int64_t(a.rb), s.rows - r0)), nk = int(min(int64_t(a.kc), a.K - k0));
+  const int nr = int(min(int64_t(a.rb), s.rows - r0)), nk = int(a.K);
   for (int i = tid; i < nr + nk; i += nth) {
     int64_t o0, o1;
     if (i < nr) {
       decode(s.R, r0 + i, o0, o1);
       s_ro[i] = o0;
     } else {
-      decode(s.K, k0 + i - nr, o0, o1);
+      decode(s.K, i - nr, o0, o1);
       s_ko[i - nr] = s.k_is_s1 ? o1 : o0;
     }
   }
@@ -109,20 +108,6 @@ __device__ void row_exponents(const SplitArgs& a, int nr, int nk, const double* 
   __syncthreads();
 }
 
-__global__ void __launch_bounds__(256) row_exponent_kernel(const SplitArgs a) {
-  extern __shared__ __align__(16) double sx[];
-  __shared__ int64_t s_ro[128], s_ko[256];
-  __shared__ int s_e[128];
-  const bool second = int64_t(blockIdx.x) >= a.blocks0;
-  const SplitSide& s = a.s[second ? 1 : 0];
-  const int64_t b = second ? int64_t(blockIdx.x) - a.blocks0 : int64_t(blockIdx.x);
-  const int64_t r0 = b / a.kblocks * a.rb, k0 = b % a.kblocks * a.kc;
-  load_block(s, a, r0, k0, sx, s_ro, s_ko);
-  const int nr = int(min(int64_t(a.rb), s.rows - r0)), nk = int(min(int64_t(a.kc), a.K - k0));
-  row_exponents(a, nr, nk, sx, s_e);
-  for (int r = threadIdx.x; r < nr; r += blockDim.x) atomicMax(s.exps + r0 + r, s_e[r]);
-}
-
 __global__ void __launch_bounds__(256) split_digits_kernel(const SplitArgs a) {
   extern __shared__ __align__(16) double sx[];
   __shared__ int64_t s_ro[128], s_ko[256];
@@ -130,19 +115,14 @@ __global__ void __launch_bounds__(256) split_digits_kernel(const SplitArgs a) {
   const bool second = int64_t(blockIdx.x) >= a.blocks0;
   const SplitSide& s = a.s[second ? 1 : 0];
   const int64_t b = second ? int64_t(blockIdx.x) - a.blocks0 : int64_t(blockIdx.x);
-  const int64_t r0 = b / a.kblocks * a.rb, k0 = b % a.kblocks * a.kc;
-  load_block(s, a, r0, k0, sx, s_ro, s_ko);
-  const int nr = int(min(int64_t(a.rb), s.rows - r0)), nk = int(min(int64_t(a.kc), a.K - k0));
-  if (a.kblocks == 1) {
-    row_exponents(a, nr, nk, sx, s_e);
-    for (int r = threadIdx.x; r < nr; r += blockDim.x) s.exps[r0 + r] = s_e[r];
-  } else {
-    for (int r = threadIdx.x; r < nr; r += blockDim.x) s_e[r] = s.exps[r0 + r];
-    __syncthreads();
-  }
+  const int64_t r0 = b * a.rb;
+  load_block(s, a, r0, sx, s_ro, s_ko);
+  const int nr = int(min(int64_t(a.rb), s.rows - r0)), nk = int(a.K);
+  row_exponents(a, nr, nk, sx, s_e);
+  for (int r = threadIdx.x; r < nr; r += blockDim.x) s.exps[r0 + r] = s_e[r];
   const int ld = a.kc + 1;
   // 16-byte groups of 8 digits; two lanes cover 32 contiguous bytes of a row
-  const int ng = int((min(a.Kp - k0, int64_t(a.kc)) + 7) / 8), ng2 = (ng + 1) / 2;
+  const int ng = a.kc / 8, ng2 = (ng + 1) / 2;
   const int64_t plane = s.rows * a.Kp;
   for (int q = threadIdx.x; q < ng2 * a.rb * 2; q += blockDim.x) {
     const int pair = q / (a.rb * 2), rest = q - pair * (a.rb * 2);
@@ -155,61 +135,92 @@ __global__ void __launch_bounds__(256) split_digits_kernel(const SplitArgs a) {
       const int k = g * 8 + i;
       x[i] = k < nk ? sx[r * ld + k] : 0.0;
     }
-    write_digits(x, E, s.dig + (r0 + r) * a.Kp + k0 + g * 8, plane);
+    write_digits(x, E, s.dig + (r0 + r) * a.Kp + g * 8, plane);
   }
 }
 
-// Long rows whose contracted index is one mode (the large matrices of the
-// randomized SVD): the warps read along whichever index has unit stride.
-// 5184 x 5184 by rows: exponents 39 us and digits 94 us (147 + 229 us through the
-// general kernels' shared-memory blocks).
+// Rows of more than 256 entries: the warps read along whichever index has unit
+// stride.  One contracted mode (kMulti false): 5184 x 5184 by rows, exponents 39 us
+// and digits 94 us (147 + 229 us through blocks in shared memory).  Several: their
+// offsets are tabled in shared memory, or stepped: 36 and 72 rows of 746496 entries,
+// exponents 93 + 97 us and digits 142 + 276 us (555 and 892 us through the blocks).
 struct LongRows {
   const double* x;
-  Group R;
-  int64_t ks;       // stride of the contracted index
+  Group R, Kg;      // strides in s0
   int64_t rows, K, Kp;
   int64_t kc;       // contracted indices per CTA of the exponent kernels
   int* exps;        // zeroed when kc < K
   bf16* dig;
 };
 
+__device__ __forceinline__ int64_t k_offset(const LongRows& a, int64_t k) {
+  int64_t o0, o1;
+  decode(a.Kg, k, o0, o1);
+  return o0;
+}
+
 __device__ __forceinline__ void put_field(const LongRows& a, int64_t r, int e) {
   if (a.kc < a.K) atomicMax(a.exps + r, e);
   else a.exps[r] = e;
 }
 
+// The largest exponent field of x[offset of k], k = k0 + first, + step, .. < k1 (all
+// threads of the CTA take part; live: this thread has a row).
+template <bool kMulti>
+__device__ __forceinline__ int largest_field(const LongRows& a, const double* x, bool live,
+                                             int64_t k0, int64_t k1, int first, int step) {
+  int e = 0;
+  if (!kMulti) {
+    const int64_t ks = a.Kg.m[0].s0;
+    if (live) {
+#pragma unroll 8
+      for (int64_t k = k0 + first; k < k1; k += step) e = max(e, exponent_field(x[k * ks]));
+    }
+  } else {
+    constexpr int kTable = 512;
+    __shared__ int64_t s_ko[kTable];
+    for (int64_t kb = k0; kb < k1; kb += kTable) {
+      const int n = int(min(int64_t(kTable), k1 - kb));
+      __syncthreads();
+      for (int i = threadIdx.x; i < n; i += blockDim.x) s_ko[i] = k_offset(a, kb + i);
+      __syncthreads();
+      if (live) {
+#pragma unroll 8
+        for (int i = first; i < n; i += step) e = max(e, exponent_field(x[s_ko[i]]));
+      }
+    }
+  }
+  return e;
+}
+
 // Contracted index of unit stride: one warp per row.
+template <bool kMulti>
 __global__ void __launch_bounds__(256) long_exponents_k_kernel(const LongRows a) {
   const int lane = threadIdx.x & 31;
   const int64_t r = blockIdx.x * int64_t(8) + (threadIdx.x >> 5);
-  if (r >= a.rows) return;
-  int64_t ro, t;
-  decode(a.R, r, ro, t);
-  const double* x = a.x + ro;
+  const bool live = r < a.rows;
+  int64_t ro = 0, t;
+  if (live) decode(a.R, r, ro, t);
   const int64_t k0 = blockIdx.y * a.kc, k1 = min(k0 + a.kc, a.K);
-  int e = 0;
-#pragma unroll 8
-  for (int64_t k = k0 + lane; k < k1; k += 32) e = max(e, exponent_field(x[k * a.ks]));
+  int e = largest_field<kMulti>(a, a.x + ro, live, k0, k1, lane, 32);
   for (int o = 16; o > 0; o >>= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, o));
-  if (lane == 0) put_field(a, r, e);
+  if (lane == 0 && live) put_field(a, r, e);
 }
 
 // Otherwise 32 rows per CTA, its warps share the contracted index.
+template <bool kMulti>
 __global__ void __launch_bounds__(512) long_exponents_r_kernel(const LongRows a) {
   __shared__ int s_e[16][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t r = blockIdx.x * int64_t(32) + lane;
   const int64_t k0 = blockIdx.y * a.kc, k1 = min(k0 + a.kc, a.K);
+  const bool live = r < a.rows;
   int64_t ro = 0, t;
-  if (r < a.rows) decode(a.R, r, ro, t);
-  int e = 0;
-  if (r < a.rows) {
-#pragma unroll 8
-    for (int64_t k = k0 + warp; k < k1; k += 16) e = max(e, exponent_field(a.x[ro + k * a.ks]));
-  }
+  if (live) decode(a.R, r, ro, t);
+  int e = largest_field<kMulti>(a, a.x + ro, live, k0, k1, warp, 16);
   s_e[warp][lane] = e;
   __syncthreads();
-  if (warp == 0 && r < a.rows) {
+  if (warp == 0 && live) {
     for (int w = 1; w < 16; ++w) e = max(e, s_e[w][lane]);
     put_field(a, r, e);
   }
@@ -218,33 +229,66 @@ __global__ void __launch_bounds__(512) long_exponents_r_kernel(const LongRows a)
 // kfast: a warp takes 8 rows x 32 indices, four lanes of eight per row, straight
 // from memory.  Else a CTA takes 32 rows x 64 indices through shared memory; two
 // lanes write 32 contiguous bytes of a row.
-template <bool kfast>
+template <bool kfast, bool kMulti>
 __global__ void __launch_bounds__(256) long_split_kernel(const LongRows a) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t plane = a.rows * a.Kp;
   if (kfast) {
     const int64_t kblocks = (a.Kp + 31) / 32;
     const int64_t w = blockIdx.x * int64_t(8) + warp;
-    const int64_t r = w / kblocks * 8 + (lane >> 2), k0 = w % kblocks * 32 + (lane & 3) * 8;
+    // several modes: neighbouring warps take neighbouring rows, whose runs of the
+    // innermost mode often share their sectors
+    const int64_t rblocks = (a.rows + 7) / 8;
+    const int64_t rb = kMulti ? w % rblocks : w / kblocks;
+    const int64_t kb = kMulti ? w / rblocks : w % kblocks;
+    const int64_t r = rb * 8 + (lane >> 2), k0 = kb * 32 + (lane & 3) * 8;
     if (r >= a.rows || k0 >= a.Kp) return;
     int64_t ro, t;
     decode(a.R, r, ro, t);
     double x[8];
+    if (!kMulti) {
+      const int64_t ks = a.Kg.m[0].s0;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) x[i] = k0 + i < a.K ? a.x[ro + (k0 + i) * a.ks] : 0.0;
+      for (int i = 0; i < 8; ++i) x[i] = k0 + i < a.K ? a.x[ro + (k0 + i) * ks] : 0.0;
+    } else {
+      // offsets within the innermost mode are steps; a new decode where it wraps
+      const Mode in = a.Kg.m[a.Kg.n - 1];
+      const uint32_t ext = uint32_t(in.ext);
+      const int64_t st = in.s0;
+      uint32_t left = 0;
+      int64_t off = 0;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        if (left == 0 && k0 + i < a.K) {
+          off = ro + k_offset(a, k0 + i);
+          left = ext - uint32_t(k0 + i) % ext;
+        }
+        x[i] = k0 + i < a.K ? a.x[off] : 0.0;
+        off += st;
+        --left;
+      }
+    }
     write_digits(x, row_exponent(a.exps[r]), a.dig + r * a.Kp + k0, plane);
   } else {
     __shared__ double sx[32][65];
+    __shared__ int64_t s_ko[64];
     const int64_t rblocks = (a.rows + 31) / 32;
     const int64_t r0 = int64_t(blockIdx.x) % rblocks * 32, kb = int64_t(blockIdx.x) / rblocks * 64;
+    if (kMulti) {
+      if (threadIdx.x < 64 && kb + threadIdx.x < a.K)
+        s_ko[threadIdx.x] = k_offset(a, kb + threadIdx.x);
+      __syncthreads();
+    }
     {
       const int64_t r = r0 + lane;
       int64_t ro = 0, t;
       if (r < a.rows) decode(a.R, r, ro, t);
+      const int64_t ks = kMulti ? 0 : a.Kg.m[0].s0;
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const int64_t k = kb + warp + 8 * i;
-        sx[lane][warp + 8 * i] = r < a.rows && k < a.K ? a.x[ro + k * a.ks] : 0.0;
+        const bool ok = r < a.rows && k < a.K;
+        sx[lane][warp + 8 * i] = ok ? a.x[ro + (kMulti ? s_ko[warp + 8 * i] : k * ks)] : 0.0;
       }
     }
     __syncthreads();
@@ -573,15 +617,33 @@ Digits alloc_digits(Ctx& c, int64_t rows, int64_t K) {
   return d;
 }
 
+// The contracted modes as one operand sees them (strides in s0): neighbours joined
+// where they are contiguous in it.
+Group joined(const Group& k, bool second) {
+  Group g{};
+  for (int i = 0; i < k.n; ++i) {
+    const Mode m{k.m[i].ext, second ? k.m[i].s1 : k.m[i].s0, 0};
+    if (g.n > 0 && g.m[g.n - 1].s0 == m.ext * m.s0) {
+      g.m[g.n - 1].ext *= m.ext;
+      g.m[g.n - 1].s0 = m.s0;
+    } else {
+      g.m[g.n++] = m;
+    }
+  }
+  return g;
+}
+
 // Exponents and digits of those of the two sides that are wanted.
 void split_sides(Ctx& c, const SplitSide* side, int want0, int want1, int64_t K, int64_t Kp) {
   if (c.sizing()) return;
   int want[2] = {want0, want1};
   for (int i = 0; i < 2; ++i) {
     const SplitSide& s = side[i];
-    if (!want[i] || K <= 256 || s.K.n > 1) continue;
+    if (!want[i] || K <= 256) continue;
     want[i] = 0;
-    LongRows a{s.x, s.R, s.k_is_s1 ? s.K.m[0].s1 : s.K.m[0].s0, s.rows, K, Kp, K, s.exps, s.dig};
+    // the modes of this operand alone, joined where they are contiguous in it
+    LongRows a{s.x, s.R, joined(s.K, s.k_is_s1 != 0), s.rows, K, Kp, K, s.exps, s.dig};
+    const bool multi = a.Kg.n > 1;
     // enough CTAs of the exponent kernels to cover the SMs twice
     const int64_t rb = s.kfast ? 8 : 32, rblocks = (s.rows + rb - 1) / rb;
     const int64_t least = s.kfast ? 512 : 256, want_ctas = 2 * sm_count_linalg();
@@ -593,16 +655,26 @@ void split_sides(Ctx& c, const SplitSide* side, int want0, int want1, int64_t K,
     {
       KernelTimer kt(c.stream, "long_exponents_kernel", kUnitByte, 8.0 * double(s.rows) * K);
       const dim3 grid(unsigned(rblocks), unsigned(chunks), 1);
-      if (s.kfast) long_exponents_k_kernel<<<grid, 256, 0, c.stream>>>(a);
-      else long_exponents_r_kernel<<<grid, 512, 0, c.stream>>>(a);
+      if (s.kfast) {
+        if (multi) long_exponents_k_kernel<true><<<grid, 256, 0, c.stream>>>(a);
+        else long_exponents_k_kernel<false><<<grid, 256, 0, c.stream>>>(a);
+      } else {
+        if (multi) long_exponents_r_kernel<true><<<grid, 512, 0, c.stream>>>(a);
+        else long_exponents_r_kernel<false><<<grid, 512, 0, c.stream>>>(a);
+      }
       CTM_LAUNCH_CHECK();
     }
     KernelTimer kt(c.stream, "long_split_kernel", kUnitByte, 24.0 * double(s.rows) * K);
     const int64_t ctas = s.kfast ? ((s.rows + 7) / 8 * ((Kp + 31) / 32) + 7) / 8
                                  : (s.rows + 31) / 32 * ((Kp + 63) / 64);
     CTM_REQUIRE(ctas < (int64_t(1) << 31), CTM_ERR_UNSUPPORTED, "einsum: grid too large");
-    if (s.kfast) long_split_kernel<true><<<unsigned(ctas), 256, 0, c.stream>>>(a);
-    else long_split_kernel<false><<<unsigned(ctas), 256, 0, c.stream>>>(a);
+    if (s.kfast) {
+      if (multi) long_split_kernel<true, true><<<unsigned(ctas), 256, 0, c.stream>>>(a);
+      else long_split_kernel<true, false><<<unsigned(ctas), 256, 0, c.stream>>>(a);
+    } else {
+      if (multi) long_split_kernel<false, true><<<unsigned(ctas), 256, 0, c.stream>>>(a);
+      else long_split_kernel<false, false><<<unsigned(ctas), 256, 0, c.stream>>>(a);
+    }
     CTM_LAUNCH_CHECK();
   }
   if (!want[0] && !want[1]) return;
@@ -611,25 +683,15 @@ void split_sides(Ctx& c, const SplitSide* side, int want0, int want1, int64_t K,
   sa.s[1] = side[1];
   sa.K = K;
   sa.Kp = Kp;
-  sa.kblocks = (K + 255) / 256;
-  sa.kc = int(sa.kblocks == 1 ? Kp : 256);
+  sa.kc = int(Kp);
   sa.rb = sa.kc <= 64 ? 128 : sa.kc <= 128 ? 64 : 32;
   auto blocks_of = [&](int i) {
-    return want[i] ? (side[i].rows + sa.rb - 1) / sa.rb * sa.kblocks : int64_t(0);
+    return want[i] ? (side[i].rows + sa.rb - 1) / sa.rb : int64_t(0);
   };
   sa.blocks0 = blocks_of(0);
   const int64_t blocks = sa.blocks0 + blocks_of(1);
   const size_t ssm = size_t(sa.rb) * (sa.kc + 1) * sizeof(double);
   const double entries = ((want[0] ? side[0].rows : 0) + (want[1] ? side[1].rows : 0)) * double(K);
-  if (sa.kblocks > 1) {
-    for (int i = 0; i < 2; ++i)
-      if (want[i])
-        CTM_CUDA(cudaMemsetAsync(side[i].exps, 0, sizeof(int) * size_t(side[i].rows), c.stream));
-    CTM_CUDA(cudaFuncSetAttribute(row_exponent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ssm)));
-    KernelTimer kt(c.stream, "row_exponent_kernel", kUnitByte, 8.0 * entries);
-    row_exponent_kernel<<<unsigned(blocks), 256, ssm, c.stream>>>(sa);
-    CTM_LAUNCH_CHECK();
-  }
   CTM_CUDA(cudaFuncSetAttribute(split_digits_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ssm)));
   KernelTimer kt(c.stream, "split_digits_kernel", kUnitByte, 24.0 * entries);
   split_digits_kernel<<<unsigned(blocks), 256, ssm, c.stream>>>(sa);
