@@ -5,10 +5,9 @@
 // cuTENSOR plans and cuSOLVER potrf/potrs in its optional extension).  Here
 // the contractions go through the strided GETT engine and each least-squares
 // step is one kernel: the symmetrised, shifted system is factorised in one
-// CTA with the matrix in shared memory (right-looking Cholesky, then the two
-// triangular solves with one warp per right-hand side; Gaussian elimination
-// with partial pivoting when a pivot is not positive, the reference's
-// torch.linalg.solve fallback).  The pseudo-inverse method runs the FP64
+// CTA with the matrix in shared memory (Cholesky, then the triangular solves with
+// one warp per right-hand side; Gaussian elimination with partial pivoting when a
+// pivot is not positive, the reference's torch.linalg.solve fallback).  The pseudo-inverse method runs the FP64
 // one-sided Jacobi SVD of the symmetrised system.  The host loop reads the
 // cost once per iteration for the reference's convergence test.
 #include <cmath>
@@ -33,11 +32,14 @@ __device__ double block_max(double v, double* red) {
   return r;
 }
 
-// W (m x m, leading dimension ld) = (R + R^T) / 2 + shift * max|.| * I
-__device__ void load_system(const double* R, int m, int ld, double eps, double* W, double* red) {
+// W (m x m, leading dimension ld; its lower half only if lower) =
+// (R + R^T) / 2 + shift * max|.| * I
+__device__ void load_system(const double* R, int m, int ld, double eps, double* W, double* red,
+                            bool lower) {
   double mx = 0.0;
   for (int idx = threadIdx.x; idx < m * m; idx += blockDim.x) {
     const int i = idx / m, j = idx - i * m;
+    if (lower && j > i) continue;
     const double v = 0.5 * (R[size_t(i) * m + j] + R[size_t(j) * m + i]);
     W[i * ld + j] = v;
     mx = fmax(mx, fabs(v));
@@ -47,23 +49,83 @@ __device__ void load_system(const double* R, int m, int ld, double eps, double* 
   __syncthreads();
 }
 
-// One warp solves L y = b (lower = true: forward, L[i][k] at W[i*ld+k]) or
-// L^T x = y (lower = false: backward, L^T[i][k] = W[k*ld+i]) for column p of
-// the right-hand sides x (m x np, in place), lane-parallel dot products.
-__device__ void tri_solve_warp(const double* W, int m, int ld, double* x, int np, int p,
-                               bool lower) {
-  const int lane = threadIdx.x & 31;
-  for (int s = 0; s < m; ++s) {
-    const int i = lower ? s : m - 1 - s;
-    double acc = 0.0;
-    if (lower) {
-      for (int k = lane; k < i; k += 32) acc += W[i * ld + k] * x[k * np + p];
-    } else {
-      for (int k = i + 1 + lane; k < m; k += 32) acc += W[k * ld + i] * x[k * np + p];
+// W = L D L^T (L with a unit diagonal; column j of W becomes L's times d_j) and x =
+// L^-1 x, false when a d_j is not positive: the pivots of the Cholesky factorisation
+// are the roots of these.  An SM does 1.7 FP64 FMAs per cycle, so the work is its m^3 / 6
+// FMAs on 4 x 8 blocks of the lower half, and each step's chain (column j + 1 updated,
+// 1 / d_{j+1}, the scaled column) runs on warp 0 beside the other warps' updates: one
+// barrier a step, no root or divide.  (m = 72 as m rank-one updates with roots and
+// divides in every thread and two triangular solves of dot products: 266 us, here
+// 97 us.)  g: two scaled columns; u: 1 / d_j.
+__device__ bool factorise(double* W, int m, int ld, double* x, int np, double* g, double* u,
+                          int* s_bad) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int kWarps = kAlsThreads / 32;
+  auto panel = [&](int j) {
+    const double d = W[j * ld + j];
+    const bool ok = d > 0.0;
+    const double r = ok ? positive_reciprocal(d) : 0.0;
+    if (lane == 0) {
+      u[j] = r;
+      if (!ok) *s_bad = j;
     }
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0) x[i * np + p] = (x[i * np + p] - acc) / W[i * ld + i];
-    __syncwarp();
+    double* gj = g + (j & 1) * m;
+    for (int k = j + 1 + lane; k < m; k += 32) gj[k] = W[k * ld + j] * r;
+  };
+  if (threadIdx.x == 0) *s_bad = m;
+  __syncthreads();
+  if (warp == 0) panel(0);
+  for (int j = 0; j < m; ++j) {
+    __syncthreads();
+    if (*s_bad <= j) return false;  // set before this barrier, or to a later step's index
+    const double* gj = g + (j & 1) * m;
+    if (warp == 0) {
+      if (j + 1 < m) {
+        const double gn = gj[j + 1];
+        for (int i = j + 1 + lane; i < m; i += 32) W[i * ld + j + 1] -= W[i * ld + j] * gn;
+        __syncwarp();
+        panel(j + 1);
+      }
+    } else if (warp == kWarps - 1) {
+      for (int idx = lane; idx < (m - j - 1) * np; idx += 32) {
+        const int i = j + 1 + idx / np, p = idx % np;
+        x[i * np + p] -= gj[i] * x[j * np + p];
+      }
+    } else {
+      for (int ib = warp - 1; 4 * ib < m - j - 2; ib += kWarps - 2) {
+        const int i = j + 2 + 4 * ib + (lane >> 3);
+        const double w = i < m ? W[i * ld + j] : 0.0;
+        for (int kb = 0; 8 * kb <= 4 * ib + 3; ++kb) {
+          const int k = j + 2 + 8 * kb + (lane & 7);
+          if (i < m && k <= i) W[i * ld + k] -= w * gj[k];
+        }
+      }
+    }
+  }
+  __syncthreads();
+  return true;
+}
+
+// X column p = L^-T D^-1 x by one warp: x_j = u_j w_j, then w_i -= W[j][i] x_j for i < j.
+__device__ void back_substitute(const double* W, int m, int ld, const double* x, int np, int p,
+                                const double* u, double* X) {
+  const int lane = threadIdx.x & 31;
+  constexpr int kT = kAlsMaxM / 32;
+  double w[kT];
+#pragma unroll
+  for (int t = 0; t < kT; ++t) w[t] = lane + 32 * t < m ? x[(lane + 32 * t) * np + p] : 0.0;
+#pragma unroll
+  for (int t = kT - 1; t >= 0; --t) {
+    for (int l = min(31, m - 1 - 32 * t); l >= 0; --l) {
+      const int j = 32 * t + l;
+      const double xj = __shfl_sync(0xffffffffu, w[t], l) * u[j];
+#pragma unroll
+      for (int s = 0; s <= t; ++s) {
+        const int i = lane + 32 * s;
+        if (i < j) w[s] -= W[j * ld + i] * xj;
+      }
+      if (lane == l) X[j * np + p] = xj;
+    }
   }
 }
 
@@ -74,45 +136,21 @@ __global__ void __launch_bounds__(kAlsThreads) als_cholesky_solve_kernel(
     const double* R, const double* S, int m, int np, double eps, double* X, int* used_lu) {
   extern __shared__ double als_smem[];
   __shared__ double red[32];
-  __shared__ int s_piv;
+  __shared__ int s_piv, s_bad;
   const int ld = m + 1;
   double* W = als_smem;           // m x ld
-  double* x = W + size_t(m) * ld;  // m x np
+  double* x = W + size_t(m) * ld;  // m x np, then 3 m of scaled columns and reciprocals
   const int tid = threadIdx.x, nth = blockDim.x, warp = tid >> 5;
-  load_system(R, m, ld, eps, W, red);
+  load_system(R, m, ld, eps, W, red, true);
   for (int idx = tid; idx < m * np; idx += nth) x[idx] = S[idx];
-  __syncthreads();
-  bool ok = true;
-  for (int j = 0; j < m; ++j) {
-    const double d = W[j * ld + j];  // the same value in every thread
-    if (!(d > 0.0)) {
-      ok = false;
-      break;
-    }
-    const double ljj = sqrt(d);
-    for (int i = j + 1 + tid; i < m; i += nth) W[i * ld + j] /= ljj;
-    __syncthreads();
-    if (tid == 0) W[j * ld + j] = ljj;
-    const int t = m - j - 1;
-    for (int idx = tid; idx < t * t; idx += nth) {
-      const int i = j + 1 + idx / t, k = j + 1 + idx % t;
-      if (k <= i) W[i * ld + k] -= W[i * ld + j] * W[k * ld + j];
-    }
-    __syncthreads();
-  }
-  if (ok) {
-    if (warp < np) {
-      tri_solve_warp(W, m, ld, x, np, warp, true);
-      tri_solve_warp(W, m, ld, x, np, warp, false);
-    }
-    __syncthreads();
-    for (int idx = tid; idx < m * np; idx += nth) X[idx] = x[idx];
+  if (factorise(W, m, ld, x, np, x + m * np, x + m * (np + 2), &s_bad)) {
+    if (warp < np) back_substitute(W, m, ld, x, np, warp, x + m * (np + 2), X);
     return;
   }
   // Gaussian elimination with partial pivoting on the shifted system
   __syncthreads();
   if (tid == 0) *used_lu = 1;
-  load_system(R, m, ld, eps, W, red);
+  load_system(R, m, ld, eps, W, red, false);
   for (int idx = tid; idx < m * np; idx += nth) x[idx] = S[idx];
   __syncthreads();
   for (int j = 0; j < m; ++j) {
@@ -260,7 +298,7 @@ void als_solve_ar(Ctx& c, const AlsDims& g, const double* R, const double* S, in
   const int m = int(g.m()), np = int(g.pD);
   if (method == 0) {
     if (c.sizing()) return;
-    const size_t smem = (size_t(m) * (m + 1) + size_t(m) * np) * sizeof(double);
+    const size_t smem = (size_t(m) * (m + 1) + size_t(m) * (np + 3)) * sizeof(double);
     CTM_CUDA(cudaFuncSetAttribute(als_cholesky_solve_kernel,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     KernelTimer kt(c.stream, "als_cholesky_solve_kernel", kUnitFlop, double(m) * m * m / 3.0);

@@ -43,23 +43,6 @@ inline size_t chol_smem(int64_t q8, int64_t P) {
           size_t(local) * kNb + kNb * kNb) * sizeof(double);
 }
 
-// 1 / d for a positive normal d, within about an ulp.
-__device__ __forceinline__ double reciprocal(double d) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(d);
-  const int ex = int(b >> 52) - 1023;
-  if (ex < -1000 || ex > 1000) return 1.0 / d;
-  const double x = __longlong_as_double((long long)(b - ((unsigned long long)(long long)ex << 52)));
-  const float m = __uint_as_float(0x3f800000u | (unsigned(b >> 29) & 0x7fffffu));
-  // (widened by its bits: a conversion takes an FP64 issue slot, 64 cycles)
-  const unsigned u = __float_as_uint(__fdividef(1.f, m));
-  const double r0 = __longlong_as_double(
-      (long long)(((unsigned long long)((u >> 23) + 896u) << 52) |
-                  ((unsigned long long)(u & 0x7fffffu) << 29)));
-  const double e = fma(-x, r0, 1.0);
-  const double r = fma(r0, fma(e, e, e), r0);
-  return __longlong_as_double(__double_as_longlong(r) - ((long long)ex << 52));
-}
-
 __global__ void __launch_bounds__(kCThreads) cholesky_cluster_kernel(const CholArgs a) {
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
@@ -117,7 +100,7 @@ __global__ void __launch_bounds__(kCThreads) cholesky_cluster_kernel(const CholA
       const long long bits = __double_as_longlong(d);  // d > 0 (and no NaN)
       const bool ok = r0 + t < q && bits > 0 && bits <= 0x7ff0000000000000ll;
       fail = fail || (r0 + t < q && !ok);
-      const double rd = ok ? reciprocal(d) : 0.0;
+      const double rd = ok ? positive_reciprocal(d) : 0.0;
       const double y = x[t] * rd;  // lane r: the multiplier of row r
       if (lane == t) {
         piv[(b / P) * kNb + t] = ok ? d : 0.0;
