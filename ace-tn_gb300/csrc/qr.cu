@@ -5,17 +5,18 @@
 // about 1500 cycles), so a column costs one all-reduce and one pass over the
 // rows.  Rows are spread over the CTAs and, inside a CTA, over four warps (one
 // per SM quarter); lanes hold columns.  In column j every CTA needs
-//   d[t] = sum_{i >= j} A[i][j] A[i][t]   (all t, one all-reduce) and row j;
-// with alpha = -sign(A[j][j]) sqrt(d[j]) and v = A[:, j] - alpha e_j, both the
-// products v^T A[:, t] for the trailing columns (t > j) and v^T v_t with the
-// earlier vectors (t < j, stored in place) are w[t] = d[t] - alpha A[j][t].
-// The update of the rows and the sums of the next column's d are one pass.
-// The products with the earlier vectors are the strict upper triangle U of
-// V^T V, and Q = [I; 0] - V M with (diag(1 / beta) + U) M = V_1^T (the compact
-// WY form; V_1: the first q rows of V), one triangular solve and one product
+//   d[t] = sum_{i >= j} A[i][j] A[i][t]   (t >= j, one all-reduce) and row j;
+// with alpha = -sign(A[j][j]) sqrt(d[j]) and v = A[:, j] - alpha e_j, the products
+// v^T A[:, t] for the trailing columns are d[t] - alpha A[j][t].  The update of the
+// rows and the sums of the next column's d are one pass.  Afterwards the strict
+// upper triangle U of V^T V is formed and summed over the CTAs once, and Q = [I; 0] -
+// V M with (diag(1 / beta) + U) M = V_1^T (the compact WY form; V_1: the first q rows
+// of V): one triangular solve, its columns shared among the CTAs, and one product
 // instead of q more all-reduces.
 //
-// 80 x 22: 62 us (783 as householder_qr_kernel, two CTA reductions per column
+// 144 x 144: 909 us (1654 with the sums of d over all columns and the solve on every
+// CTA).
+// 80 x 22: 59 us (783 as householder_qr_kernel, two CTA reductions per column
 // pair on one CTA).
 #include <cooperative_groups.h>
 
@@ -115,6 +116,9 @@ __global__ void __launch_bounds__(kQrThreads) householder_cluster_kernel(const Q
     else __syncthreads();
   };
   sync_all();
+  // more than 32 columns: U is formed at the end (one column chunk has no finished
+  // chunks to skip, and its products with the earlier vectors come with the sums)
+  constexpr bool kLate = NC > 1;
   double g[NC], acc[NC];
   double vj = 0.0;
   for (int j = 0; j <= q; ++j) {
@@ -127,7 +131,8 @@ __global__ void __launch_bounds__(kQrThreads) householder_cluster_kernel(const Q
       double* row = A + i * ld;
       double x[NC];
 #pragma unroll
-      for (int c = 0; c < NC; ++c) x[c] = lane + 32 * c < q ? row[lane + 32 * c] : 0.0;
+      for (int c = 0; c < NC; ++c)
+        x[c] = (!kLate || 32 * c + 31 >= j) && lane + 32 * c < q ? row[lane + 32 * c] : 0.0;
       if (j > 0) {
         const bool pivot = row0 + i == j - 1;
         const double v = pivot ? vj : row[j - 1];
@@ -153,16 +158,17 @@ __global__ void __launch_bounds__(kQrThreads) householder_cluster_kernel(const Q
           if (c == j >> 5) xj = s;
         }
 #pragma unroll
-        for (int c = 0; c < NC; ++c) acc[c] = fma(xj, x[c], acc[c]);
+        for (int c = 0; c < NC; ++c)
+          if (!kLate || 32 * c + 31 >= j) acc[c] = fma(xj, x[c], acc[c]);
       }
     }
     if (j == q) break;
 #pragma unroll
     for (int c = 0; c < NC; ++c)
-      if (lane + 32 * c < q) red[warp * q + lane + 32 * c] = acc[c];
+      if ((!kLate || 32 * c + 31 >= j) && lane + 32 * c < q) red[warp * q + lane + 32 * c] = acc[c];
     __syncthreads();
     double* buf = part + (j & 1) * size_t(P + 1) * q;
-    for (int t = tid; t < q; t += kQrThreads) {
+    for (int t = (kLate ? j : 0) + tid; t < q; t += kQrThreads) {
       double s = red[t];
 #pragma unroll
       for (int w = 1; w < kQrWarps; ++w) s += red[w * q + t];
@@ -177,7 +183,7 @@ __global__ void __launch_bounds__(kQrThreads) householder_cluster_kernel(const Q
     sync_all();
     double d[NC], rj[NC];
     if (NC > 2) {  // each warp sums its share of the columns
-      for (int t = tid; t < q; t += kQrThreads) {
+      for (int t = j + tid; t < q; t += kQrThreads) {
         double s = buf[t];
         for (int r = 1; r < P; ++r) s += buf[r * q + t];
         red[t] = s;
@@ -189,7 +195,7 @@ __global__ void __launch_bounds__(kQrThreads) householder_cluster_kernel(const Q
       const int t = lane + 32 * c;
       d[c] = 0.0;
       rj[c] = 0.0;
-      if (t < q) {
+      if ((!kLate || t >= j) && t < q) {
         if (NC > 2) {
           d[c] = red[t];
         } else {
@@ -212,10 +218,12 @@ __global__ void __launch_bounds__(kQrThreads) householder_cluster_kernel(const Q
     vj = ajj - alpha;
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
-      const int t = lane + 32 * c;
-      const double w = fma(-alpha, rj[c], d[c]);
-      g[c] = beta * w;
-      if (warp == 0 && t < j) S[t * ld + j] = w;
+      g[c] = 0.0;
+      if (!kLate || 32 * c + 31 >= j) {
+        const double w = fma(-alpha, rj[c], d[c]);
+        g[c] = beta * w;
+        if (!kLate && warp == 0 && lane < j) S[lane * ld + j] = w;
+      }
     }
     if (tid == 0) {
       betas[j] = beta;
@@ -233,33 +241,90 @@ __global__ void __launch_bounds__(kQrThreads) householder_cluster_kernel(const Q
     }
   }
   sync_all();
-  // X[j][c] = V[c][j] (c >= j), kept at S[c][j]
-  for (int r = warp; r < q; r += kQrWarps) {
-    const int owner = r / nr;
-    const double* src = (P > 1 ? cluster.map_shared_rank(A, owner) : A) + (r - owner * nr) * ld;
-    for (int t = lane; t <= r; t += 32) S[r * ld + t] = src[t];
-  }
-  __syncthreads();
-  for (int k = q - 1; k > 0; --k) {  // X[j][c] -= U[j][k] beta_k X[k][c], j < k <= c
-    double m[NC];
+  // U = the strict upper triangle of V^T V: every CTA's rows, then row t summed and
+  // handed out by CTA t mod P
+  if (kLate) {
+    for (int t = warp; t < q; t += kQrWarps) {
 #pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      const int t = lane + 32 * c;
-      m[c] = t >= k && t < q ? betas[k] * S[t * ld + k] : 0.0;
+      for (int c = 0; c < NC; ++c) {
+        if (32 * c + 31 <= t) continue;
+        const int u = lane + 32 * c;
+        double w = 0.0;
+        if (u < q)
+          for (int i = 0; i < rows; ++i) w = fma(A[i * ld + t], A[i * ld + u], w);
+        if (u > t && u < q) S[t * ld + u] = w;
+      }
     }
-    for (int j = warp; j < k; j += kQrWarps) {
-      const double u = S[j * ld + k];
+    sync_all();
+    if (P > 1) {
+      for (int t = me; t < q; t += P)
+        for (int u = t + 1 + tid; u < q; u += kQrThreads) {
+          double w = *cluster.map_shared_rank(S + t * ld + u, 0);
+          for (int r = 1; r < P; ++r) w += *cluster.map_shared_rank(S + t * ld + u, r);
+          for (int r = 0; r < P; ++r) *cluster.map_shared_rank(S + t * ld + u, r) = w;
+        }
+      cluster.sync();
+    }
+  }
+  // (diag(1 / beta) + U) M = V_1^T with M[j][c] (c >= j) kept at S[c][j], from X = V_1^T
+  auto row_of_v = [&](int r) {
+    return (P > 1 ? cluster.map_shared_rank(A, r / nr) : A) + (r % nr) * ld;
+  };
+  if (P >= 4) {
+    // a warp per column c, its lanes along j; the CTAs share the columns
+    for (int col = me + P * warp; col < q; col += P * kQrWarps) {
+      const double* src = row_of_v(col);
+      double x[NC];
+#pragma unroll
+      for (int c = 0; c < NC; ++c) x[c] = lane + 32 * c <= col ? src[lane + 32 * c] : 0.0;
+#pragma unroll
+      for (int ck = NC - 1; ck >= 0; --ck) {
+        for (int l = min(31, col - 32 * ck); l >= 0; --l) {
+          const int k = 32 * ck + l;
+          const double m = __shfl_sync(0xffffffffu, x[ck], l) * betas[k];
+          if (lane == l) x[ck] = m;
+#pragma unroll
+          for (int c = 0; c <= ck; ++c) {
+            const int j = lane + 32 * c;
+            if (j < k) x[c] = fma(-S[j * ld + k], m, x[c]);
+          }
+        }
+      }
+      for (int r = 0; r < P; ++r) {
+        double* dst = cluster.map_shared_rank(S, r) + col * ld;
+#pragma unroll
+        for (int c = 0; c < NC; ++c)
+          if (lane + 32 * c <= col) dst[lane + 32 * c] = x[c];
+      }
+    }
+    cluster.sync();
+  } else {
+    for (int r = warp; r < q; r += kQrWarps) {
+      const double* src = row_of_v(r);
+      for (int t = lane; t <= r; t += 32) S[r * ld + t] = src[t];
+    }
+    __syncthreads();
+    for (int k = q - 1; k > 0; --k) {  // X[j][c] -= U[j][k] beta_k X[k][c], j < k <= c
+      double m[NC];
 #pragma unroll
       for (int c = 0; c < NC; ++c) {
         const int t = lane + 32 * c;
-        if (t >= k && t < q) S[t * ld + j] = fma(-u, m[c], S[t * ld + j]);
+        m[c] = t >= k && t < q ? betas[k] * S[t * ld + k] : 0.0;
       }
+      for (int j = warp; j < k; j += kQrWarps) {
+        const double u = S[j * ld + k];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+          const int t = lane + 32 * c;
+          if (t >= k && t < q) S[t * ld + j] = fma(-u, m[c], S[t * ld + j]);
+        }
+      }
+      __syncthreads();
     }
+    for (int r = warp; r < q; r += kQrWarps)
+      for (int t = lane; t <= r; t += 32) S[r * ld + t] *= betas[t];
     __syncthreads();
   }
-  for (int r = warp; r < q; r += kQrWarps)
-    for (int t = lane; t <= r; t += 32) S[r * ld + t] *= betas[t];
-  __syncthreads();
   // Q[i][c] = [i == c] - sum_{k <= c} V[i][k] M[k][c]
   for (int i = warp; i < rows; i += kQrWarps) {
     const int gi = row0 + i;
