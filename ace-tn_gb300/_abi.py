@@ -164,8 +164,10 @@ class _Workspace:
     def __init__(self):
         self.buf = {}
 
-    def get(self, nbytes, device):
-        key = (torch.device(device).index, torch.cuda.current_stream(device).cuda_stream)
+    def get(self, nbytes, device, stream=None):
+        if stream is None:
+            stream = torch.cuda.current_stream(device).cuda_stream
+        key = (torch.device(device).index, stream)
         b = self.buf.get(key)
         if b is None or b.numel() < nbytes:
             size = max(int(nbytes * 1.25), 1 << 20)
@@ -183,11 +185,13 @@ def call(name, args_before_ws, device, key=None, stream=None):
     workspace protocol (size query, then the real call)."""
     lib = load()
     fn = getattr(lib, name)
-    stream = stream_handle(device) if stream is None else stream
+    device = torch.device(device)
+    current = torch.cuda.current_stream(device).cuda_stream
+    stream = ctypes.c_void_p(current) if stream is None else stream
     # workspace sizes depend on the device (its SM count sets the split-K of
     # the tensor-core products), so the cache is keyed by device as well
     if key is not None:
-        key = (torch.device(device).index, key)
+        key = (device.index, key)
     nbytes = _WS_CACHE.get(key) if key is not None else None
     if nbytes is None:
         sz = ctypes.c_size_t(0)
@@ -195,7 +199,7 @@ def call(name, args_before_ws, device, key=None, stream=None):
         nbytes = sz.value
         if key is not None:
             _WS_CACHE[key] = nbytes
-    ws = WORKSPACE.get(nbytes, device)
+    ws = WORKSPACE.get(nbytes, device, current)
     sz = ctypes.c_size_t(ws.numel())
     check(fn(*args_before_ws, ctypes.c_void_p(ws.data_ptr()), ctypes.byref(sz), stream), name)
 
@@ -299,6 +303,18 @@ def device_status(device=None):
     return flags.value
 
 
+_C_NAMES = tuple(f"C[{k}]" for k in range(4))
+_E_NAMES = tuple(f"E[{k}]" for k in range(4))
+
+
+def _widened(t):
+    """``t`` as contiguous float64; the two torch calls are skipped where they would
+    return ``t`` itself (nine tensors a site, and small states are bound by the host)."""
+    if t.dtype == torch.float64 and t.is_contiguous():
+        return t
+    return t.to(torch.float64).contiguous()
+
+
 class SiteRef:
     """A ``CtmSite`` over a site's A, C[0..3], E[0..3] tensors (kept alive)."""
 
@@ -308,29 +324,33 @@ class SiteRef:
         E = site_tensor["E"]
         require_cuda(A, "A", storage=True)
         self.dtype = A.dtype  # storage type of the site (float64 or float32)
-        self.keep = [A.to(torch.float64).contiguous()]
+        self.keep = [_widened(A)]
         self.D = A.shape[0]
         self.d = A.shape[4]
         s = CtmSite()
         s.A = self.keep[0].data_ptr()
+        c_ptr, e_ptr, c_rows, c_cols, e_rows, e_cols = ([0] * 4 for _ in range(6))
         for k in range(4):
             ck = C[k]
             ek = E[k]
-            require_cuda(ck, f"C[{k}]", storage=True)
-            require_cuda(ek, f"E[{k}]", storage=True)
-            ck = ck.to(torch.float64).contiguous()
-            ek = ek.to(torch.float64).contiguous()
+            require_cuda(ck, _C_NAMES[k], storage=True)
+            require_cuda(ek, _E_NAMES[k], storage=True)
+            ck = _widened(ck)
+            ek = _widened(ek)
             self.keep += [ck, ek]
-            s.C[k] = ck.data_ptr()
-            s.E[k] = ek.data_ptr()
-            s.c_rows[k], s.c_cols[k] = ck.shape
-            s.e_rows[k], s.e_cols[k] = ek.shape[0], ek.shape[1]
+            c_ptr[k] = ck.data_ptr()
+            e_ptr[k] = ek.data_ptr()
+            c_rows[k], c_cols[k] = ck.shape
+            e_rows[k], e_cols[k] = ek.shape[:2]
+        s.C[:], s.E[:] = c_ptr, e_ptr
+        s.c_rows[:], s.c_cols[:] = c_rows, c_cols
+        s.e_rows[:], s.e_cols[:] = e_rows, e_cols
         self.s = s
         self.device = A.device
+        self._shapes = (tuple(c_rows), tuple(c_cols), tuple(e_rows), tuple(e_cols), self.D, self.d)
 
     def shapes(self):
-        s = self.s
-        return tuple(tuple(x) for x in (s.c_rows, s.c_cols, s.e_rows, s.e_cols)) + (self.D, self.d)
+        return self._shapes
 
     @property
     def pointer(self):
