@@ -37,6 +37,7 @@ __global__ void __launch_bounds__(NT) gett_kernel(const GettArgs<T> p) {
   const int tid = threadIdx.x;
   const int64_t m0 = static_cast<int64_t>(p.swap_xy ? blockIdx.y : blockIdx.x) * BM;
   const int64_t n0 = static_cast<int64_t>(p.swap_xy ? blockIdx.x : blockIdx.y) * BN;
+  if (p.sym && n0 > m0) return;  // C[m][n] = C[n][m]: written by the tile below the diagonal
   const int64_t z = blockIdx.z;
   const int64_t batch = z % p.bext;
   const int64_t split = z / p.bext;
@@ -137,11 +138,19 @@ __global__ void __launch_bounds__(NT) gett_kernel(const GettArgs<T> p) {
       const int64_t n = n0 + nj;
       if (n >= p.Nt) continue;
       if (p.splitk > 1) {
-        p.part[((split * p.bext + batch) * p.Mt + m) * p.Nt + n] = acc[i][j];
+        T* part = p.part + (split * p.bext + batch) * p.Mt * p.Nt;
+        part[m * p.Nt + n] = acc[i][j];
+        if (p.sym && n0 < m0) part[n * p.Nt + m] = acc[i][j];
       } else {
         T* c = p.C + batch * p.bsc + sCm[mi] + sCn[nj];
         const T v = p.alpha * acc[i][j];
         *c = (p.beta != T(0)) ? fma(p.beta, *c, v) : v;
+        if (p.sym && n0 < m0) {
+          int64_t o, rn, cm;
+          decode(p.M, n, o, rn);
+          decode(p.N, m, o, cm);
+          p.C[rn + cm] = v;
+        }
       }
     }
   }
@@ -298,6 +307,18 @@ Group to_group(std::vector<Mode> v, const char* what) {
   return g;
 }
 
+bool same_rows(const Group& a, const Group& b) {
+  bool same = a.n == b.n;
+  for (int i = 0; same && i < a.n; ++i) same = a.m[i].ext == b.m[i].ext && a.m[i].s0 == b.m[i].s0;
+  return same;
+}
+
+bool one_operand(const Group& k) {
+  bool one = true;
+  for (int i = 0; i < k.n; ++i) one = one && k.m[i].s0 == k.m[i].s1;
+  return one;
+}
+
 int64_t group_size(const Group& g) {
   int64_t s = 1;
   for (int i = 0; i < g.n; ++i) s *= g.m[i].ext;
@@ -446,8 +467,15 @@ void einsum_impl(Ctx& c, const char* spec, const ViewT<T>& A, const ViewT<T>& B,
     }
   }
   const int64_t sms = sm_count_linalg();
+  // a Gram matrix (one operand twice): 3/5 of the tiles of 5 x 5
+  p.sym = sizeof(T) == 8 && p.A == p.B && bext == 1 && p.beta == T(0) && p.Mt == p.Nt &&
+                  same_rows(p.M, p.N) && one_operand(p.K)
+              ? 1
+              : 0;
   auto tiles_of = [&](int t) {
-    return ((p.Mt + 16 * t - 1) / (16 * t)) * ((p.Nt + 16 * t - 1) / (16 * t)) * bext;
+    const int64_t mt = (p.Mt + 16 * t - 1) / (16 * t);
+    if (p.sym) return mt * (mt + 1) / 2;
+    return mt * ((p.Nt + 16 * t - 1) / (16 * t)) * bext;
   };
   int tile = 4, splitk = 1;
   if (sizeof(T) == 4) {
