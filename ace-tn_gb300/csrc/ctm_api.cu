@@ -120,7 +120,7 @@ void product(Ctx& c, const double* A, const double* B, double* C, int64_t M, int
 // Each factor is multiplied niter + 1 to niter + 3 times in either form, and the
 // digits (2 x 16 bytes per entry) take as long to form as one product: 0.25 ms of
 // 0.56 ms at 5184 x 5184 x 160.  At most kKeptDigits bytes of them are kept.
-constexpr double kKeptDigits = 24e9;
+constexpr double kKeptDigits = 4e9;
 
 void keep_digits(Ctx& c, std::vector<Factor>& F, int64_t q) {
   double bytes = 0.0;

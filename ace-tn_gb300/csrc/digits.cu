@@ -751,11 +751,65 @@ Digits operand_digits(Ctx& c, const GettArgs<double>& p, bool first) {
   return d;
 }
 
+namespace {
+
+// The digits take twice their operand's bytes.  Beyond this many bytes for one operand
+// the contraction is done in parts, so that the workspace of any size grows by two
+// gigabytes at most (16384 x 16384 x 272 in five parts: each still fills the SMs, and
+// the small operand's digits are formed again in under 0.1 of a part's time).
+constexpr double kMaxDigitBytes = 1e9;
+
+// p as two contractions over halves of the outermost mode of its rows (0), columns (1)
+// or contracted indices (2); the second half of the latter adds to the first's result.
+bool halves(const GettArgs<double>& p, int which, GettArgs<double>& lo, GettArgs<double>& hi) {
+  lo = hi = p;
+  const Group& g = which == 0 ? p.M : which == 1 ? p.N : p.K;
+  if (g.n == 0 || g.m[0].ext < 2) return false;
+  const Mode m = g.m[0];
+  const int64_t e1 = m.ext / 2, off0 = e1 * m.s0, off1 = e1 * m.s1;
+  auto cut = [&](GettArgs<double>& q, int64_t ext) {
+    Group& h = which == 0 ? q.M : which == 1 ? q.N : q.K;
+    int64_t& total = which == 0 ? q.Mt : which == 1 ? q.Nt : q.Kt;
+    total = total / m.ext * ext;
+    h.m[0].ext = ext;
+    if (ext == 1) {  // no modes of one entry
+      for (int i = 0; i + 1 < h.n; ++i) h.m[i] = h.m[i + 1];
+      --h.n;
+    }
+  };
+  cut(lo, e1);
+  cut(hi, m.ext - e1);
+  if (which == 0) {
+    hi.A += off0;
+    hi.C += off1;
+  } else if (which == 1) {
+    hi.B += off0;
+    hi.C += off1;
+  } else {
+    hi.A += off0;
+    hi.B += off1;
+    hi.beta = 1.0;
+  }
+  return true;
+}
+
+}  // namespace
+
 void digit_contract(Ctx& c, const GettArgs<double>& p, const Digits* pre_a, const Digits* pre_b) {
   bool stream_swap = false;
-  if (pre_a == nullptr && pre_b == nullptr && stream_fits(p, stream_swap)) {
-    stream_contract(c, p, stream_swap);
-    return;
+  if (pre_a == nullptr && pre_b == nullptr) {
+    if (stream_fits(p, stream_swap)) {
+      stream_contract(c, p, stream_swap);
+      return;
+    }
+    const int64_t most = std::max(p.Mt, p.Nt);
+    GettArgs<double> lo, hi;
+    if (16.0 * double(most) * double(p.Kt) > kMaxDigitBytes &&
+        ((most > 512 && halves(p, p.Mt >= p.Nt ? 0 : 1, lo, hi)) || halves(p, 2, lo, hi))) {
+      digit_contract(c, lo);
+      digit_contract(c, hi);
+      return;
+    }
   }
   const int64_t K = p.Kt, Kp = (K + 7) / 8 * 8;
   const int sms = sm_count_linalg();
