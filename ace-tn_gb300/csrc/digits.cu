@@ -840,10 +840,10 @@ void digit_contract(Ctx& c, const GettArgs<double>& p, const Digits* pre_a, cons
   const int64_t m_tiles = (M + kM - 1) / kM, n_tiles = (N + nt - 1) / nt;
   const int64_t tiles = m_tiles * n_tiles;
   const int64_t stages = (K + kStageK - 1) / kStageK;
-  // K ranges when the tiles leave most SMs idle; at least two reads of the
+  // K ranges when the tiles leave most SMs idle; at least one read of the
   // accumulators' worth of stages each
   int64_t split = 1;
-  if (tiles * 2 <= sms) split = std::min<int64_t>(sms / tiles, stages / (2 * kChunkStages));
+  if (tiles * 2 <= sms) split = std::min<int64_t>(sms / tiles, stages / kChunkStages);
   split = std::max<int64_t>(split, 1);
   int64_t per = (stages + split - 1) / split;
   per = (per + kChunkStages - 1) / kChunkStages * kChunkStages;
