@@ -27,7 +27,7 @@
 // times closer to the exact one than the FMA chain's.
 //
 // A row or column with an infinity or a NaN has no digits; outputs on it are
-// formed by the FMA chain in the epilogue.
+// marked and formed by the FMA chain in a kernel of their own (digits_chain.cu).
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -319,12 +319,12 @@ struct DigitArgs {
   int64_t ldm, ldn;     // partial sums: strides of rows and columns (split > 1)
   int64_t part_stride;
   double alpha, beta;
-  int ntile, m_tiles, n_tiles, tiles, n_fast;
+  int m_tiles, n_tiles, tiles, n_fast;
   int split;            // K ranges
   int stages_per_split; // multiple of kChunkStages
   int stages_total;
   int* status;
-  ChainArgs chain;
+  uint32_t* marks;      // split 1: word 2 * column tile + half of row m at word * M + m
 };
 
 // round_96 as a call: inlined once per column it made 30 KB of code that every tile's
@@ -546,22 +546,25 @@ __global__ void __launch_bounds__(kDThreads, 1)
       }
       if (row < p.M) {
         double* out = p.C + ro;
-        const int64_t k0 = int64_t(s0) * kStageK, k1 = min(p.K, int64_t(s1) * kStageK);
+        uint32_t mark = 0;
 #pragma unroll
         for (int c = 0; c < kHalf; ++c) {
           const int64_t off = s_cn[par][half * kHalf + c];
           const int e = s_eb[par][half * kHalf + c];
           if (off < 0) continue;
           // units of 2^-68 of the scales (digit s of the product: 2^(-12 - 8 s))
-          double v;
-          if (er == kBadField || e == kBadField) v = chain_dot(p.chain, row, int64_t(n0) + half * kHalf + c, k0, k1);
-          else v = rounded(hi[c], lo[c], row_exponent(er) + row_exponent(e) - 2 * 1023 - 68);
+          if (p.split == 1 && (er == kBadField || e == kBadField)) {
+            mark |= 1u << c;
+            continue;
+          }
+          double v = rounded(hi[c], lo[c], row_exponent(er) + row_exponent(e) - 2 * 1023 - 68);
           if (p.split == 1 && !(p.alpha == 1.0 && p.beta == 0.0)) {
             v *= p.alpha;
             if (p.beta != 0.0) v = fma(p.beta, out[off], v);
           }
           out[off] = v;
         }
+        if (p.split == 1) p.marks[int64_t(n0 / kHalf + half) * p.M + row] = mark;
       }
     }
   }
@@ -579,6 +582,48 @@ __global__ void __launch_bounds__(kDThreads, 1)
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u)
                  : "memory");
+  }
+}
+
+// Sums the K ranges' partial outputs (in the order of gett_splitk_reduce) into C; a warp
+// takes 32 columns of a row and writes their word of marks.
+struct ReduceArgs {
+  GettArgs<double> p;   // part and splitk set
+  const int* ea;        // of the rows and columns of p
+  const int* eb;
+  uint32_t* marks;
+  int words;
+};
+
+__global__ void __launch_bounds__(256) digit_reduce_kernel(const ReduceArgs a) {
+  const GettArgs<double>& p = a.p;
+  const int lane = threadIdx.x & 31;
+  const int64_t total = p.Mt * a.words, plane = p.Mt * p.Nt;
+  for (int64_t idx = blockIdx.x * int64_t(8) + (threadIdx.x >> 5); idx < total;
+       idx += int64_t(gridDim.x) * 8) {
+    const int64_t m = idx / a.words, w = idx - m * a.words, n = w * 32 + lane;
+    bool mark = false;
+    if (n < p.Nt) {
+      const double* pt = p.part + m * p.Nt + n;
+      double s0 = 0.0, s1 = 0.0;
+      int t = 0;
+      for (; t + 1 < p.splitk; t += 2) {
+        s0 += pt[t * plane];
+        s1 += pt[(t + 1) * plane];
+      }
+      if (t < p.splitk) s0 += pt[t * plane];
+      mark = a.ea[m] == kBadField || a.eb[n] == kBadField;
+      if (!mark) {
+        int64_t am, cm, bn, cn;
+        decode(p.M, m, am, cm);
+        decode(p.N, n, bn, cn);
+        double* c = p.C + cm + cn;
+        const double v = p.alpha * (s0 + s1);
+        *c = p.beta != 0.0 ? fma(p.beta, *c, v) : v;
+      }
+    }
+    const uint32_t word = __ballot_sync(0xffffffffu, mark);
+    if (lane == 0) a.marks[w * p.Mt + m] = word;
   }
 }
 
@@ -849,6 +894,11 @@ void digit_contract(Ctx& c, const GettArgs<double>& p, const Digits* pre_a, cons
   per = (per + kChunkStages - 1) / kChunkStages * kChunkStages;
   split = (stages + per - 1) / per;
   double* part = split > 1 ? c.alloc<double>(size_t(split) * p.Mt * p.Nt) : nullptr;
+  Marks marks;
+  marks.rows = split > 1 ? p.Mt : M;
+  marks.per = split > 1 ? 32 : nt / 2;
+  marks.words = int(split > 1 ? (p.Nt + 31) / 32 : 2 * n_tiles);
+  marks.word = c.alloc<uint32_t>(size_t(marks.rows) * marks.words);
   if (c.sizing()) return;
   CTM_REQUIRE(tiles * split < (int64_t(1) << 31), CTM_ERR_UNSUPPORTED, "einsum: grid too large");
 
@@ -881,7 +931,6 @@ void digit_contract(Ctx& c, const GettArgs<double>& p, const Digits* pre_a, cons
   d.part_stride = p.Mt * p.Nt;
   d.alpha = p.alpha;
   d.beta = p.beta;
-  d.ntile = nt;
   d.m_tiles = int(m_tiles);
   d.n_tiles = int(n_tiles);
   d.tiles = int(tiles);
@@ -890,7 +939,7 @@ void digit_contract(Ctx& c, const GettArgs<double>& p, const Digits* pre_a, cons
   d.stages_per_split = int(per);
   d.stages_total = int(stages);
   d.status = status_flags(c);
-  d.chain = chain_args(p, swap);
+  d.marks = marks.word;
   CUtensorMap tA, tB;
   digit_map(&tA, da.dig, M, Kp, kM);
   digit_map(&tB, db.dig, N, Kp, uint32_t(nt));
@@ -909,10 +958,17 @@ void digit_contract(Ctx& c, const GettArgs<double>& p, const Digits* pre_a, cons
   else launch(digit_gemm_kernel<8>);
   CTM_LAUNCH_CHECK();
   if (split > 1) {
-    GettArgs<double> r = p;
-    r.splitk = int(split);
-    r.part = part;
-    splitk_reduce(c, r);
+    ReduceArgs r{p, swap ? db.exps : da.exps, swap ? da.exps : db.exps, marks.word, marks.words};
+    r.p.splitk = int(split);
+    r.p.part = part;
+    {
+      KernelTimer kt(c.stream, "digit_reduce_kernel", kUnitByte, 8.0 * (split + 1.0) * p.Mt * p.Nt);
+      digit_reduce_kernel<<<grid_for(p.Mt * marks.words, 8), 256, 0, c.stream>>>(r);
+      CTM_LAUNCH_CHECK();
+    }
+    chain_outputs(c, p, chain_args(p, false), p.M, p.N, p.Nt, marks, int(split), part);
+  } else {
+    chain_outputs(c, p, chain_args(p, swap), d.GM, d.GN, N, marks, 1, nullptr);
   }
 }
 

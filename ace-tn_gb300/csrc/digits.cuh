@@ -116,19 +116,19 @@ inline ChainArgs chain_args(const GettArgs<double>& p, bool swap) {
   return c;
 }
 
-// One output by the FMA chain, for rows and columns with non-finite entries.
-static __device__ __noinline__ double chain_dot(const ChainArgs& p, int64_t m, int64_t n, int64_t k0,
-                                         int64_t k1) {
-  int64_t mo, no, t0, t1;
-  decode(p.FM, m, mo, t0);
-  decode(p.FN, n, no, t0);
-  double v = 0.0;
-  for (int64_t k = k0; k < k1; ++k) {
-    decode(p.FK, k, t0, t1);
-    v = fma(p.a[mo + (p.swapped ? t1 : t0)], p.b[no + (p.swapped ? t0 : t1)], v);
-  }
-  return v;
-}
+// Outputs that the products leave to the FMA chain (digits_chain.cu): bit b of
+// marks[w * rows + r] is the one of row r and column w * per + b.  Every word is
+// written by the kernel that forms the outputs; marked ones are not stored.
+struct Marks {
+  uint32_t* word = nullptr;
+  int64_t rows = 0;
+  int words = 0, per = 0;
+};
+// The marked outputs of C = alpha A B + beta C; chain, GM and GN (strides in s1) as
+// their rows and columns, part: room for ranges x rows x columns partial sums when
+// the contracted index is to be shared among ranges > 1 CTAs.
+void chain_outputs(Ctx& c, const GettArgs<double>& p, const ChainArgs& chain, const Group& GM,
+                   const Group& GN, int64_t columns, const Marks& marks, int ranges, double* part);
 
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z,
                                             uint64_t* bar) {

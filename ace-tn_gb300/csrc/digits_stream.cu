@@ -44,7 +44,7 @@ struct StreamArgs {
   int nbuf;                       // digit buffers of the long operand
   int64_t tiles;
   int* status;
-  ChainArgs chain;
+  uint32_t* marks;                // word 2 * pass + half of row m at word * M + m
 };
 
 __device__ __forceinline__ bool wait_warp(uint64_t* bar, uint32_t parity) {
@@ -82,10 +82,8 @@ __device__ __forceinline__ long long fixed_point(const float (&f)[kDigits]) {
   return (long long)((unsigned long long)t + ((unsigned long long)top << 32));
 }
 
-// Outside the normal range, zeros, and rows or columns without digits.
-__device__ __noinline__ double rare_value(const ChainArgs& chain, long long t, int er, int ec,
-                                          int unit, int64_t m, int n, int K) {
-  if (er == kBadField || ec == kBadField) return chain_dot(chain, m, n, 0, K);
+// Outside the normal range, and zeros.
+__device__ __noinline__ double rare_value(long long t, int er, int ec, int unit) {
   return round_96(t >> 32, uint32_t(t), row_exponent(er) + row_exponent(ec) - 2 * 1023 - unit);
 }
 
@@ -314,11 +312,12 @@ __global__ void __launch_bounds__(kSThreads, 1)
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const int er = s_er[ring][row];
-        // (er + 1) + (ec + 1) - 2 1023 - unit + 1023; out of range without digits
-        const int ebase = er == kBadField ? -100000 : max(er, 1) + 2 - 1023 - kUnit;
+        // (er + 1) + (ec + 1) - 2 1023 - unit + 1023
+        const int ebase = max(er, 1) + 2 - 1023 - kUnit;
         const uint32_t ta = tmem + (uint32_t(lane_base) << 16) +
                             uint32_t(tb * kDigits * NT + half * kHalf);
         const int n0 = ps * NT + half * kHalf;
+        uint32_t mark = 0;
         // one copy of the body (the roles' code together has to stay in the
         // instruction cache: unrolled, a third of the cycles waited for it)
 #pragma unroll 1
@@ -339,6 +338,10 @@ __global__ void __launch_bounds__(kSThreads, 1)
             const long long fx = fixed_point<kSmallGroups, kUnit>(g);
             if (valid && off >= 0) {
               const int ec = s_eb[n0 + c + j];
+              if (er == kBadField || ec == kBadField) {
+                mark |= 1u << (c + j);
+                continue;
+              }
               const unsigned long long mag = (unsigned long long)(fx < 0 ? -fx : fx);
               const int lz = __clzll((long long)mag);
               const unsigned long long nm = mag << (lz & 63);
@@ -348,13 +351,12 @@ __global__ void __launch_bounds__(kSThreads, 1)
               // the rounding leaves r = 0 in 53 bits and goes through the rare path
               const int ef = ebase + max(ec, 1) + (63 - lz);
               double v;
-              if (nm < 0xfffffffffffffc00ull && unsigned(ef - 1) < 2044u && mag != 0 &&
-                  ec != kBadField)
+              if (nm < 0xfffffffffffffc00ull && unsigned(ef - 1) < 2044u && mag != 0)
                 v = __longlong_as_double(
                     (long long)((((unsigned long long)unsigned(ef - 1)) << 52) + r) |
                     (fx & (long long)0x8000000000000000ull));
               else
-                v = rare_value(p.chain, fx, er, ec, kUnit, m, n0 + c + j, p.K);
+                v = rare_value(fx, er, ec, kUnit);
               if (scaled) {
                 v *= p.alpha;
                 if (p.beta != 0.0) v = fma(p.beta, out[off], v);
@@ -364,6 +366,7 @@ __global__ void __launch_bounds__(kSThreads, 1)
           }
           __syncwarp();
         }
+        if (valid) p.marks[(2 * ps + half) * p.M + m] = mark;
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         if (lane == 0) mbar_arrive(&t_empty[tb]);
       }
@@ -427,13 +430,18 @@ bool stream_fits(const GettArgs<double>& p, bool& swap) {
 void stream_contract(Ctx& c, const GettArgs<double>& p, bool swap) {
   Scope scope(c);
   const Digits db = operand_digits(c, p, swap);
-  if (c.sizing()) return;
   StreamPlan pl;
   StreamArgs a{};
   a.M = swap ? p.Nt : p.Mt;
   a.N = int(swap ? p.Mt : p.Nt);
   a.K = int(p.Kt);
   stream_plan(a.N, a.K, pl);
+  Marks marks;
+  marks.rows = a.M;
+  marks.per = pl.nt / 2;
+  marks.words = 2 * pl.passes;
+  marks.word = c.alloc<uint32_t>(size_t(marks.rows) * marks.words);
+  if (c.sizing()) return;
   a.x = swap ? p.B : p.A;
   a.FX = swap ? p.N : p.M;
   a.FK = p.K;
@@ -451,7 +459,7 @@ void stream_contract(Ctx& c, const GettArgs<double>& p, bool swap) {
   a.nbuf = pl.nbuf;
   a.tiles = (a.M + kTileM - 1) / kTileM;
   a.status = status_flags(c);
-  a.chain = chain_args(p, swap);
+  a.marks = marks.word;
   const int64_t Kp = (p.Kt + 7) / 8 * 8;
   CUtensorMap tB;
   {
@@ -485,6 +493,7 @@ void stream_contract(Ctx& c, const GettArgs<double>& p, bool swap) {
   else if (pl.nt == 48) pick(std::integral_constant<int, 48>());
   else pick(std::integral_constant<int, 64>());
   CTM_LAUNCH_CHECK();
+  chain_outputs(c, p, chain_args(p, swap), a.GM, a.GN, a.N, marks, 1, nullptr);
 }
 
 }  // namespace ctm

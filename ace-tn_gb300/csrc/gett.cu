@@ -328,16 +328,6 @@ int64_t group_size(const Group& g) {
 }  // namespace
 
 template <class T>
-void splitk_reduce_impl(Ctx& c, const GettArgs<T>& p) {
-  KernelTimer kt(c.stream, "gett_splitk_reduce", kUnitByte,
-                 double(sizeof(T)) * (p.splitk + 1.0) * p.bext * p.Mt * p.Nt);
-  gett_splitk_reduce<T><<<grid_for(p.bext * p.Mt * p.Nt, 256), 256, 0, c.stream>>>(p);
-  CTM_LAUNCH_CHECK();
-}
-
-void splitk_reduce(Ctx& c, const GettArgs<double>& p) { splitk_reduce_impl<double>(c, p); }
-
-template <class T>
 void einsum_impl(Ctx& c, const char* spec, const ViewT<T>& A, const ViewT<T>& B, const ViewT<T>& C,
                  double alpha, double beta, const Digits* da = nullptr,
                  const Digits* db = nullptr) {
@@ -540,7 +530,12 @@ void einsum_impl(Ctx& c, const char* spec, const ViewT<T>& A, const ViewT<T>& B,
     }
     CTM_LAUNCH_CHECK();
   }
-  if (splitk > 1) splitk_reduce_impl<T>(c, p);
+  if (splitk > 1) {
+    KernelTimer kt(c.stream, "gett_splitk_reduce", kUnitByte,
+                   double(sizeof(T)) * (splitk + 1.0) * bext * p.Mt * p.Nt);
+    gett_splitk_reduce<T><<<grid_for(bext * p.Mt * p.Nt, 256), 256, 0, c.stream>>>(p);
+    CTM_LAUNCH_CHECK();
+  }
 }
 
 void einsum(Ctx& c, const char* spec, const View& A, const View& B, const View& C, double alpha,

@@ -63,7 +63,5 @@ void digit_contract(Ctx& c, const GettArgs<double>& p, const Digits* pre_a = nul
                     const Digits* pre_b = nullptr);
 // One FP32 contraction (p.splitk and p.kchunk set).
 void gett_f32(Ctx& c, GettArgs<float>& p);
-// Sum of the split-K partials p.part into p.C.
-void splitk_reduce(Ctx& c, const GettArgs<double>& p);
 
 }  // namespace ctm
