@@ -27,12 +27,13 @@
 // times closer to the exact one than the FMA chain's.
 //
 // A row or column with an infinity or a NaN has no digits; outputs on it are
-// marked and formed by the FMA chain in a kernel of their own (digits_chain.cu).
+// marked and formed by the FMA chain after the products (digits_chain.cuh).
 #include <cuda_bf16.h>
 
 #include <algorithm>
 
 #include "digits.cuh"
+#include "digits_chain.cuh"
 
 namespace ctm {
 
@@ -344,7 +345,8 @@ static __device__ __noinline__ double rounded(long long hi, uint32_t lo, int e) 
 template <int kHalf>
 __global__ void __launch_bounds__(kDThreads, 1)
     digit_gemm_kernel(const __grid_constant__ CUtensorMap tA,
-                      const __grid_constant__ CUtensorMap tB, const DigitArgs p) {
+                      const __grid_constant__ CUtensorMap tB,
+                      const DigitArgs p) {
   extern __shared__ uint8_t dyn_smem[];
   uint8_t* base = reinterpret_cast<uint8_t*>(
       (reinterpret_cast<uintptr_t>(dyn_smem) + 1023) & ~uintptr_t(1023));
@@ -359,6 +361,7 @@ __global__ void __launch_bounds__(kDThreads, 1)
   __shared__ int s_fail, s_epi_fail[2];
   __shared__ int64_t s_cn[2][NT];
   __shared__ int s_eb[2][NT];
+  __shared__ uint32_t s_bad[2][2];  // columns without digits, by half
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
@@ -477,6 +480,12 @@ __global__ void __launch_bounds__(kDThreads, 1)
     for (int it = blockIdx.x; it < work; it += gridDim.x, par ^= 1) {
       int m0, n0, s0, s1, sp;
       item(it, m0, n0, s0, s1, sp);
+      if (warp < 6) {  // warp 4 + h: columns of half h
+        const int64_t n = int64_t(n0) + (warp - 4) * kHalf + lane;
+        const bool bad = lane < kHalf && n < p.N && p.eb[n] == kBadField;
+        const uint32_t mask = __ballot_sync(0xffffffffu, bad);
+        if (lane == 0) s_bad[par][warp - 4] = mask;
+      }
       for (int c = etid; c < NT; c += 256) {
         const int64_t n = int64_t(n0) + c;
         int64_t off = -1, t;
@@ -546,21 +555,19 @@ __global__ void __launch_bounds__(kDThreads, 1)
       }
       if (row < p.M) {
         double* out = p.C + ro;
-        uint32_t mark = 0;
+        // marked: the chain's, stored after the products
+        uint32_t mark = s_bad[par][half];
+        if (er == kBadField) mark = low_bits(min(kHalf, int(p.N) - n0 - half * kHalf));
 #pragma unroll
         for (int c = 0; c < kHalf; ++c) {
           const int64_t off = s_cn[par][half * kHalf + c];
           const int e = s_eb[par][half * kHalf + c];
           if (off < 0) continue;
           // units of 2^-68 of the scales (digit s of the product: 2^(-12 - 8 s))
-          if (p.split == 1 && (er == kBadField || e == kBadField)) {
-            mark |= 1u << c;
-            continue;
-          }
           double v = rounded(hi[c], lo[c], row_exponent(er) + row_exponent(e) - 2 * 1023 - 68);
           if (p.split == 1 && !(p.alpha == 1.0 && p.beta == 0.0)) {
             v *= p.alpha;
-            if (p.beta != 0.0) v = fma(p.beta, out[off], v);
+            if (p.beta != 0.0) v = (mark >> c & 1u) ? out[off] : fma(p.beta, out[off], v);
           }
           out[off] = v;
         }
@@ -591,17 +598,16 @@ struct ReduceArgs {
   GettArgs<double> p;   // part and splitk set
   const int* ea;        // of the rows and columns of p
   const int* eb;
-  uint32_t* marks;
-  int words;
+  Marks marks;
 };
 
 __global__ void __launch_bounds__(256) digit_reduce_kernel(const ReduceArgs a) {
   const GettArgs<double>& p = a.p;
   const int lane = threadIdx.x & 31;
-  const int64_t total = p.Mt * a.words, plane = p.Mt * p.Nt;
+  const int64_t total = p.Mt * a.marks.words, plane = p.Mt * p.Nt;
   for (int64_t idx = blockIdx.x * int64_t(8) + (threadIdx.x >> 5); idx < total;
        idx += int64_t(gridDim.x) * 8) {
-    const int64_t m = idx / a.words, w = idx - m * a.words, n = w * 32 + lane;
+    const int64_t m = idx / a.marks.words, w = idx - m * a.marks.words, n = w * 32 + lane;
     bool mark = false;
     if (n < p.Nt) {
       const double* pt = p.part + m * p.Nt + n;
@@ -623,7 +629,41 @@ __global__ void __launch_bounds__(256) digit_reduce_kernel(const ReduceArgs a) {
       }
     }
     const uint32_t word = __ballot_sync(0xffffffffu, mark);
-    if (lane == 0) a.marks[w * p.Mt + m] = word;
+    if (lane == 0) a.marks.word[w * p.Mt + m] = word;
+  }
+}
+
+// The marked outputs, over blockIdx.y's range of the contracted index where part is set.
+// (At the end of digit_gemm_kernel itself this code cost 64 us of 405 at 5184 x 5184 x 144
+// with nothing marked; as a kernel 4 us.)
+__global__ void __launch_bounds__(256) chain_outputs_kernel(
+    const __grid_constant__ ChainOutputs a, int64_t kchunk) {
+  __shared__ __align__(16) uint8_t buf[kChainSmem];
+  const int64_t rblocks = (a.marks.rows + kCRows - 1) / kCRows, items = rblocks * a.marks.words;
+  const int mine = int((items - blockIdx.x + gridDim.x - 1) / gridDim.x);
+  auto where = [&](int b, int64_t& r, int64_t& w) {
+    const int64_t it = blockIdx.x + int64_t(b) * gridDim.x;
+    w = it / rblocks;
+    r = (it - w * rblocks) * kCRows;
+  };
+  const int64_t k0 = blockIdx.y * kchunk;
+  chain_marked<256>(a, mine, where, buf, sizeof(buf), k0, min(a.K, k0 + kchunk));
+}
+
+// The ranges' sums of the marked outputs into C.
+__global__ void __launch_bounds__(256) chain_sum_kernel(ChainOutputs a, int ranges) {
+  const double* part = a.part;
+  a.part = nullptr;
+  const int64_t total = a.marks.rows * a.marks.words;
+  for (int64_t idx = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; idx < total;
+       idx += int64_t(gridDim.x) * blockDim.x) {
+    const int64_t w = idx / a.marks.rows, r = idx - w * a.marks.rows;
+    for (uint32_t left = a.marks.word[idx]; left != 0u; left &= left - 1u) {
+      const int64_t n = w * a.marks.per + __ffs(int(left)) - 1;
+      double v = 0.0;
+      for (int t = 0; t < ranges; ++t) v += part[(t * a.marks.rows + r) * a.columns + n];
+      chain_store(a, r, n, v);
+    }
   }
 }
 
@@ -894,7 +934,7 @@ void digit_contract(Ctx& c, const GettArgs<double>& p, const Digits* pre_a, cons
   per = (per + kChunkStages - 1) / kChunkStages * kChunkStages;
   split = (stages + per - 1) / per;
   double* part = split > 1 ? c.alloc<double>(size_t(split) * p.Mt * p.Nt) : nullptr;
-  Marks marks;
+  Marks marks{};
   marks.rows = split > 1 ? p.Mt : M;
   marks.per = split > 1 ? 32 : nt / 2;
   marks.words = int(split > 1 ? (p.Nt + 31) / 32 : 2 * n_tiles);
@@ -958,17 +998,25 @@ void digit_contract(Ctx& c, const GettArgs<double>& p, const Digits* pre_a, cons
   else launch(digit_gemm_kernel<8>);
   CTM_LAUNCH_CHECK();
   if (split > 1) {
-    ReduceArgs r{p, swap ? db.exps : da.exps, swap ? da.exps : db.exps, marks.word, marks.words};
+    ReduceArgs r{p, swap ? db.exps : da.exps, swap ? da.exps : db.exps, marks};
     r.p.splitk = int(split);
     r.p.part = part;
-    {
-      KernelTimer kt(c.stream, "digit_reduce_kernel", kUnitByte, 8.0 * (split + 1.0) * p.Mt * p.Nt);
-      digit_reduce_kernel<<<grid_for(p.Mt * marks.words, 8), 256, 0, c.stream>>>(r);
-      CTM_LAUNCH_CHECK();
-    }
-    chain_outputs(c, p, chain_args(p, false), p.M, p.N, p.Nt, marks, int(split), part);
-  } else {
-    chain_outputs(c, p, chain_args(p, swap), d.GM, d.GN, N, marks, 1, nullptr);
+    KernelTimer kt(c.stream, "digit_reduce_kernel", kUnitByte, 8.0 * (split + 1.0) * p.Mt * p.Nt);
+    digit_reduce_kernel<<<grid_for(p.Mt * marks.words, 8), 256, 0, c.stream>>>(r);
+    CTM_LAUNCH_CHECK();
+  }
+  ChainOutputs out = chain_outputs(p, split == 1 && swap, marks);
+  // long chains of few outputs in the product's ranges (746496 terms: 190 us by one CTA)
+  const int ranges = K > 16384 ? int(split) : 1;
+  if (ranges > 1) out.part = part;
+  const int64_t blocks = (marks.rows + kCRows - 1) / kCRows * marks.words;
+  KernelTimer kt(c.stream, "chain_outputs_kernel", kUnitByte, 4.0 * double(marks.rows) * marks.words);
+  chain_outputs_kernel<<<dim3(unsigned(std::min<int64_t>(blocks, 4 * sms)), unsigned(ranges)), 256, 0,
+                         c.stream>>>(out, (K + ranges - 1) / ranges);
+  CTM_LAUNCH_CHECK();
+  if (ranges > 1) {
+    chain_sum_kernel<<<grid_for(marks.rows * marks.words, 256), 256, 0, c.stream>>>(out, ranges);
+    CTM_LAUNCH_CHECK();
   }
 }
 

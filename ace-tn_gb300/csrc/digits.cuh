@@ -116,19 +116,42 @@ inline ChainArgs chain_args(const GettArgs<double>& p, bool swap) {
   return c;
 }
 
-// Outputs that the products leave to the FMA chain (digits_chain.cu): bit b of
-// marks[w * rows + r] is the one of row r and column w * per + b.  Every word is
+// Outputs that the products leave to the FMA chain (digits_chain.cuh): bit b of
+// word[w * rows + r] is the one of row r and column w * per + b.  Every word is
 // written by the kernel that forms the outputs; marked ones are not stored.
 struct Marks {
-  uint32_t* word = nullptr;
-  int64_t rows = 0;
-  int words = 0, per = 0;
+  uint32_t* word;
+  int64_t rows;
+  int words, per;
 };
-// The marked outputs of C = alpha A B + beta C; chain, GM and GN (strides in s1) as
-// their rows and columns, part: room for ranges x rows x columns partial sums when
-// the contracted index is to be shared among ranges > 1 CTAs.
-void chain_outputs(Ctx& c, const GettArgs<double>& p, const ChainArgs& chain, const Group& GM,
-                   const Group& GN, int64_t columns, const Marks& marks, int ranges, double* part);
+
+__device__ __forceinline__ uint32_t low_bits(int n) {
+  return n >= 32 ? ~0u : n > 0 ? (1u << n) - 1u : 0u;
+}
+
+struct ChainOutputs {
+  ChainArgs ch;
+  Group GM, GN;         // output strides of rows and columns (m[].s1)
+  Marks marks;
+  int64_t columns, K;
+  double* C;
+  double* part;         // not null: sums of K ranges, [blockIdx.y][row][column]
+  double alpha, beta;
+};
+
+inline ChainOutputs chain_outputs(const GettArgs<double>& p, bool swap, const Marks& marks) {
+  ChainOutputs o{};
+  o.ch = chain_args(p, swap);
+  o.GM = swap ? p.N : p.M;
+  o.GN = swap ? p.M : p.N;
+  o.marks = marks;
+  o.columns = swap ? p.Mt : p.Nt;
+  o.K = p.Kt;
+  o.C = p.C;
+  o.alpha = p.alpha;
+  o.beta = p.beta;
+  return o;
+}
 
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z,
                                             uint64_t* bar) {

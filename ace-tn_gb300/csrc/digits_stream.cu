@@ -18,6 +18,7 @@
 #include <type_traits>
 
 #include "digits.cuh"
+#include "digits_chain.cuh"
 
 namespace ctm {
 
@@ -44,7 +45,7 @@ struct StreamArgs {
   int nbuf;                       // digit buffers of the long operand
   int64_t tiles;
   int* status;
-  uint32_t* marks;                // word 2 * pass + half of row m at word * M + m
+  ChainOutputs out;               // word 2 * pass + half
 };
 
 __device__ __forceinline__ bool wait_warp(uint64_t* bar, uint32_t parity) {
@@ -91,7 +92,8 @@ __device__ __noinline__ double rare_value(long long t, int er, int ec, int unit)
 // (3 2^14 K); 2: K <= 192, the first two.
 template <int NT, int kMode>
 __global__ void __launch_bounds__(kSThreads, 1)
-    digit_stream_kernel(const __grid_constant__ CUtensorMap tB, const StreamArgs p) {
+    digit_stream_kernel(const __grid_constant__ CUtensorMap tB,
+                        const __grid_constant__ StreamArgs p) {
   extern __shared__ uint8_t dyn_smem[];
   uint8_t* base = reinterpret_cast<uint8_t*>(
       (reinterpret_cast<uintptr_t>(dyn_smem) + 1023) & ~uintptr_t(1023));
@@ -112,6 +114,7 @@ __global__ void __launch_bounds__(kSThreads, 1)
   __shared__ int64_t s_ko[kMaxK];
   __shared__ int64_t s_cn[kMaxCols];
   __shared__ int s_eb[kMaxCols];
+  __shared__ uint32_t s_bad[kMaxCols / 8];  // columns without digits, by pass and half
   __shared__ int s_er[8][kTileM];  // tiles in flight: two digit buffers, up to four accumulators
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -143,6 +146,12 @@ __global__ void __launch_bounds__(kSThreads, 1)
     }
     s_cn[n] = off;
     s_eb[n] = e;
+  }
+  if (warp < 2 * p.passes) {  // (16 warps and more: at most 12 words)
+    const int n = warp * (NT / 2) + lane;
+    const bool bad = lane < NT / 2 && n < p.N && p.eb[n] == kBadField;
+    const uint32_t mask = __ballot_sync(0xffffffffu, bad);
+    if (lane == 0) s_bad[warp] = mask;
   }
   if (warp == 16) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
@@ -317,7 +326,9 @@ __global__ void __launch_bounds__(kSThreads, 1)
         const uint32_t ta = tmem + (uint32_t(lane_base) << 16) +
                             uint32_t(tb * kDigits * NT + half * kHalf);
         const int n0 = ps * NT + half * kHalf;
-        uint32_t mark = 0;
+        // marked: the chain's, stored after the products
+        uint32_t mark = s_bad[2 * ps + half];
+        if (er == kBadField) mark = low_bits(min(kHalf, p.N - n0));
         // one copy of the body (the roles' code together has to stay in the
         // instruction cache: unrolled, a third of the cycles waited for it)
 #pragma unroll 1
@@ -338,10 +349,6 @@ __global__ void __launch_bounds__(kSThreads, 1)
             const long long fx = fixed_point<kSmallGroups, kUnit>(g);
             if (valid && off >= 0) {
               const int ec = s_eb[n0 + c + j];
-              if (er == kBadField || ec == kBadField) {
-                mark |= 1u << (c + j);
-                continue;
-              }
               const unsigned long long mag = (unsigned long long)(fx < 0 ? -fx : fx);
               const int lz = __clzll((long long)mag);
               const unsigned long long nm = mag << (lz & 63);
@@ -359,14 +366,14 @@ __global__ void __launch_bounds__(kSThreads, 1)
                 v = rare_value(fx, er, ec, kUnit);
               if (scaled) {
                 v *= p.alpha;
-                if (p.beta != 0.0) v = fma(p.beta, out[off], v);
+                if (p.beta != 0.0) v = (mark >> (c + j) & 1u) ? out[off] : fma(p.beta, out[off], v);
               }
               out[off] = v;
             }
           }
           __syncwarp();
         }
-        if (valid) p.marks[(2 * ps + half) * p.M + m] = mark;
+        if (valid) p.out.marks.word[(2 * ps + half) * p.M + m] = mark;
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         if (lane == 0) mbar_arrive(&t_empty[tb]);
       }
@@ -381,6 +388,17 @@ __global__ void __launch_bounds__(kSThreads, 1)
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u)
                  : "memory");
+  }
+  if (s_fail == 0) {
+    const int words = 2 * p.passes;
+    const int mine = int((p.tiles - blockIdx.x + gridDim.x - 1) / gridDim.x);
+    auto where = [&](int b, int64_t& r, int64_t& w) {
+      const int t = b / words;
+      r = (blockIdx.x + int64_t(t) * gridDim.x) * kTileM;
+      w = b - t * words;
+    };
+    chain_marked<kSThreads>(p.out, mine * words, where, base,
+                            size_t(p.nbuf) * a_bytes, 0, p.K);
   }
 }
 
@@ -436,7 +454,7 @@ void stream_contract(Ctx& c, const GettArgs<double>& p, bool swap) {
   a.N = int(swap ? p.Mt : p.Nt);
   a.K = int(p.Kt);
   stream_plan(a.N, a.K, pl);
-  Marks marks;
+  Marks marks{};
   marks.rows = a.M;
   marks.per = pl.nt / 2;
   marks.words = 2 * pl.passes;
@@ -459,7 +477,7 @@ void stream_contract(Ctx& c, const GettArgs<double>& p, bool swap) {
   a.nbuf = pl.nbuf;
   a.tiles = (a.M + kTileM - 1) / kTileM;
   a.status = status_flags(c);
-  a.marks = marks.word;
+  a.out = chain_outputs(p, swap, marks);
   const int64_t Kp = (p.Kt + 7) / 8 * 8;
   CUtensorMap tB;
   {
@@ -493,7 +511,6 @@ void stream_contract(Ctx& c, const GettArgs<double>& p, bool swap) {
   else if (pl.nt == 48) pick(std::integral_constant<int, 48>());
   else pick(std::integral_constant<int, 64>());
   CTM_LAUNCH_CHECK();
-  chain_outputs(c, p, chain_args(p, swap), a.GM, a.GN, a.N, marks, 1, nullptr);
 }
 
 }  // namespace ctm
