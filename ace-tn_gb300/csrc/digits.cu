@@ -592,24 +592,31 @@ __global__ void __launch_bounds__(kDThreads, 1)
   }
 }
 
-// Sums the K ranges' partial outputs (in the order of gett_splitk_reduce) into C; a warp
-// takes 32 columns of a row and writes their word of marks.
+// Sums the K ranges' partial outputs (in the order of gett_splitk_reduce) into C, eight
+// rows by one word a CTA.  kChain: the marked ones follow at once; else they are left to
+// chain_outputs_kernel.
 struct ReduceArgs {
   GettArgs<double> p;   // part and splitk set
   const int* ea;        // of the rows and columns of p
   const int* eb;
-  Marks marks;
+  ChainOutputs out;
 };
 
-__global__ void __launch_bounds__(256) digit_reduce_kernel(const ReduceArgs a) {
+template <bool kChain>
+__global__ void __launch_bounds__(256) digit_reduce_kernel(const __grid_constant__ ReduceArgs a) {
+  __shared__ uint32_t list[256];
+  __shared__ int s_count;
   const GettArgs<double>& p = a.p;
-  const int lane = threadIdx.x & 31;
-  const int64_t total = p.Mt * a.marks.words, plane = p.Mt * p.Nt;
-  for (int64_t idx = blockIdx.x * int64_t(8) + (threadIdx.x >> 5); idx < total;
-       idx += int64_t(gridDim.x) * 8) {
-    const int64_t m = idx / a.marks.words, w = idx - m * a.marks.words, n = w * 32 + lane;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t words = (p.Nt + 31) / 32, total = (p.Mt + 7) / 8 * words, plane = p.Mt * p.Nt;
+  for (int64_t idx = blockIdx.x; idx < total; idx += gridDim.x) {
+    const int64_t r0 = idx / words * 8, w = idx - r0 / 8 * words, m = r0 + warp, n = w * 32 + lane;
+    if (kChain) {
+      if (threadIdx.x == 0) s_count = 0;
+      __syncthreads();
+    }
     bool mark = false;
-    if (n < p.Nt) {
+    if (m < p.Mt && n < p.Nt) {
       const double* pt = p.part + m * p.Nt + n;
       double s0 = 0.0, s1 = 0.0;
       int t = 0;
@@ -628,10 +635,25 @@ __global__ void __launch_bounds__(256) digit_reduce_kernel(const ReduceArgs a) {
         *c = p.beta != 0.0 ? fma(p.beta, *c, v) : v;
       }
     }
-    const uint32_t word = __ballot_sync(0xffffffffu, mark);
-    if (lane == 0) a.marks.word[w * p.Mt + m] = word;
+    if (kChain) {
+      if (mark) list[atomicAdd(&s_count, 1)] = threadIdx.x;
+      __syncthreads();
+      auto where = [&](int, int64_t& r, int64_t& word) {
+        r = r0;
+        word = w;
+      };
+      chain_listed<256>(a.out, list, s_count, 0, a.out.K, where);
+      __syncthreads();
+    } else {
+      const uint32_t word = __ballot_sync(0xffffffffu, mark);
+      if (lane == 0 && m < p.Mt) a.out.marks.word[w * p.Mt + m] = word;
+    }
   }
 }
+
+// Contracted indices from which the marked outputs of a product in K ranges are summed in
+// ranges too (746496 terms of one output take a CTA 190 us).
+constexpr int64_t kLongChain = 16384;
 
 // The marked outputs, over blockIdx.y's range of the contracted index where part is set.
 // (At the end of digit_gemm_kernel itself this code cost 64 us of 405 at 5184 x 5184 x 144
@@ -997,25 +1019,28 @@ void digit_contract(Ctx& c, const GettArgs<double>& p, const Digits* pre_a, cons
   else if (nt == 32) launch(digit_gemm_kernel<16>);
   else launch(digit_gemm_kernel<8>);
   CTM_LAUNCH_CHECK();
+  ChainOutputs out = chain_outputs(p, split == 1 && swap, marks);
+  const bool ranges = split > 1 && K > kLongChain;
   if (split > 1) {
-    ReduceArgs r{p, swap ? db.exps : da.exps, swap ? da.exps : db.exps, marks};
+    ReduceArgs r{p, swap ? db.exps : da.exps, swap ? da.exps : db.exps, out};
     r.p.splitk = int(split);
     r.p.part = part;
     KernelTimer kt(c.stream, "digit_reduce_kernel", kUnitByte, 8.0 * (split + 1.0) * p.Mt * p.Nt);
-    digit_reduce_kernel<<<grid_for(p.Mt * marks.words, 8), 256, 0, c.stream>>>(r);
+    const int ctas = grid_for((p.Mt + 7) / 8 * marks.words, 1);
+    if (ranges) digit_reduce_kernel<false><<<ctas, 256, 0, c.stream>>>(r);
+    else digit_reduce_kernel<true><<<ctas, 256, 0, c.stream>>>(r);
     CTM_LAUNCH_CHECK();
+    if (!ranges) return;
+    out.part = part;
   }
-  ChainOutputs out = chain_outputs(p, split == 1 && swap, marks);
-  // long chains of few outputs in the product's ranges (746496 terms: 190 us by one CTA)
-  const int ranges = K > 16384 ? int(split) : 1;
-  if (ranges > 1) out.part = part;
   const int64_t blocks = (marks.rows + kCRows - 1) / kCRows * marks.words;
   KernelTimer kt(c.stream, "chain_outputs_kernel", kUnitByte, 4.0 * double(marks.rows) * marks.words);
-  chain_outputs_kernel<<<dim3(unsigned(std::min<int64_t>(blocks, 4 * sms)), unsigned(ranges)), 256, 0,
-                         c.stream>>>(out, (K + ranges - 1) / ranges);
+  chain_outputs_kernel<<<dim3(unsigned(std::min<int64_t>(blocks, 4 * sms)),
+                              unsigned(ranges ? split : 1)),
+                         256, 0, c.stream>>>(out, ranges ? (K + split - 1) / split : K);
   CTM_LAUNCH_CHECK();
-  if (ranges > 1) {
-    chain_sum_kernel<<<grid_for(marks.rows * marks.words, 256), 256, 0, c.stream>>>(out, ranges);
+  if (ranges) {
+    chain_sum_kernel<<<grid_for(marks.rows * marks.words, 256), 256, 0, c.stream>>>(out, int(split));
     CTM_LAUNCH_CHECK();
   }
 }
