@@ -55,11 +55,12 @@ __device__ __forceinline__ bool wait_warp(uint64_t* bar, uint32_t parity) {
 }
 
 // One output's eight accumulators as an integer in units of 2^-kUnit of the
-// scales (the sum of K products below 1 fits in 63 bits): the groups below
+// scales (the sum of K products below 1 fits in 63 bits), to nearest: the groups below
 // kSmallGroups are under 2^22, converted by an FP32 addition each, the others by
-// the conversion unit.  The truncation is at most 2^-55, under the dropped digit
-// products' sqrt(K) 2^-60 in the mean, and 60 instructions per output fewer than
-// 96 bits need: the epilogue's instructions bound these products.
+// the conversion unit.  The rounding is 2^-58, 2^-57 and 2^-56 at most (K <= 36, 80, 192),
+// with a deviation of 2^-59.8 to 2^-57.8 beside the dropped digit products' sqrt(K)
+// 2^-62.2, and 60 instructions per output fewer than 96 bits need: the epilogue's
+// instructions bound these products.
 template <int kSmallGroups, int kUnit>
 __device__ __forceinline__ long long fixed_point(const float (&f)[kDigits]) {
   int g[kDigits];
@@ -71,13 +72,13 @@ __device__ __forceinline__ long long fixed_point(const float (&f)[kDigits]) {
   if (kSmallGroups == kDigits) {
     t = (long long)(g[2] * 256 + g[3]) * (1 << (kUnit - 36));
     t += (long long)(g[4] * 256 + g[5]) * (1 << (kUnit - 52));
-    t += (g[6] * 256 + g[7]) >> (68 - kUnit);
+    t += (g[6] * 256 + g[7] + (1 << (67 - kUnit))) >> (68 - kUnit);
   } else {
     t = (long long)g[2] * (1 << (kUnit - 28));
     t += (long long)g[3] * (1 << (kUnit - 36));
     t += (long long)g[4] * (1 << (kUnit - 44));
     t += (long long)g[5] * (1 << (kUnit - 52));
-    t += ((long long)g[6] * 256 + g[7]) >> (68 - kUnit);
+    t += ((long long)g[6] * 256 + g[7] + (1 << (67 - kUnit))) >> (68 - kUnit);
   }
   const uint32_t top = uint32_t(g[0] * 256 + g[1]) << (kUnit - 52);
   return (long long)((unsigned long long)t + ((unsigned long long)top << 32));
