@@ -26,8 +26,11 @@
 // products for a chain of FMAs: on random operands the result is 10 to 100
 // times closer to the exact one than the FMA chain's.
 //
-// A row or column with an infinity or a NaN has no digits; outputs on it are
-// marked and formed by the FMA chain after the products (digits_chain.cuh).
+// That is the error beside the two rows' scales.  Outputs whose terms all lie far
+// below them (a row graded one way along the contracted index, the column the
+// other; digits.cuh), and those on a row or column with an infinity or a NaN,
+// which has no digits, are marked and formed by the FMA chain after the products
+// (digits_chain.cuh).
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -49,6 +52,7 @@ struct SplitSide {
   int kfast;       // the contracted index has unit stride (else rows are read fastest)
   int* exps;       // rows: the largest exponent field
   bf16* dig;       // [digit][row][Kp]
+  uint32_t* cover;
 };
 
 struct SplitArgs {
@@ -129,14 +133,14 @@ __global__ void __launch_bounds__(256) split_digits_kernel(const SplitArgs a) {
     const int pair = q / (a.rb * 2), rest = q - pair * (a.rb * 2);
     const int r = rest >> 1, g = pair * 2 + (rest & 1);
     if (r >= nr || g >= ng) continue;
-    const int E = row_exponent(s_e[r]);
     double x[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const int k = g * 8 + i;
       x[i] = k < nk ? sx[r * ld + k] : 0.0;
     }
-    write_digits(x, E, s.dig + (r0 + r) * a.Kp + g * 8, plane);
+    write_digits(x, s_e[r], s.dig + (r0 + r) * a.Kp + g * 8, plane,
+                 s.cover + (r0 + r) * cover_stride(a.K) + g);
   }
 }
 
@@ -152,6 +156,7 @@ struct LongRows {
   int64_t kc;       // contracted indices per CTA of the exponent kernels
   int* exps;        // zeroed when kc < K
   bf16* dig;
+  uint32_t* cover;
 };
 
 __device__ __forceinline__ int64_t k_offset(const LongRows& a, int64_t k) {
@@ -269,7 +274,8 @@ __global__ void __launch_bounds__(256) long_split_kernel(const LongRows a) {
         --left;
       }
     }
-    write_digits(x, row_exponent(a.exps[r]), a.dig + r * a.Kp + k0, plane);
+    write_digits(x, a.exps[r], a.dig + r * a.Kp + k0, plane,
+                 a.cover + r * cover_stride(a.K) + k0 / 8);
   } else {
     __shared__ double sx[32][65];
     __shared__ int64_t s_ko[64];
@@ -299,7 +305,8 @@ __global__ void __launch_bounds__(256) long_split_kernel(const LongRows a) {
     double x[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) x[i] = sx[rl][g * 8 + i];
-    write_digits(x, row_exponent(a.exps[r]), a.dig + r * a.Kp + k0, plane);
+    write_digits(x, a.exps[r], a.dig + r * a.Kp + k0, plane,
+                 a.cover + r * cover_stride(a.K) + k0 / 8);
   }
 }
 
@@ -326,6 +333,8 @@ struct DigitArgs {
   int stages_total;
   int* status;
   uint32_t* marks;      // split 1: word 2 * column tile + half of row m at word * M + m
+  int* queued;          // split 1: ChainQueue::count
+  int guard;            // small outputs are marked too
 };
 
 // round_96 as a call: inlined once per column it made 30 KB of code that every tile's
@@ -365,6 +374,7 @@ __global__ void __launch_bounds__(kDThreads, 1)
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
+    if (blockIdx.x == 0 && p.split == 1) *p.queued = 0;
     s_fail = 0;
     s_epi_fail[0] = s_epi_fail[1] = 0;
     for (int s = 0; s < kStages; ++s) {
@@ -564,6 +574,8 @@ __global__ void __launch_bounds__(kDThreads, 1)
           const int e = s_eb[par][half * kHalf + c];
           if (off < 0) continue;
           // units of 2^-68 of the scales (digit s of the product: 2^(-12 - 8 s))
+          constexpr long long kSmall = 1ll << (68 - kCoverBits - 32);
+          if (p.guard && hi[c] < kSmall && hi[c] >= -kSmall) mark |= 1u << c;
           double v = rounded(hi[c], lo[c], row_exponent(er) + row_exponent(e) - 2 * 1023 - 68);
           if (p.split == 1 && !(p.alpha == 1.0 && p.beta == 0.0)) {
             v *= p.alpha;
@@ -615,23 +627,58 @@ __global__ void __launch_bounds__(256) digit_reduce_kernel(const __grid_constant
       if (threadIdx.x == 0) s_count = 0;
       __syncthreads();
     }
-    bool mark = false;
+    bool mark = false, small = false;
+    double sum = 0.0;
     if (m < p.Mt && n < p.Nt) {
       const double* pt = p.part + m * p.Nt + n;
-      double s0 = 0.0, s1 = 0.0;
+      double s0 = 0.0, s1 = 0.0, m0 = 0.0, m1 = 0.0;
       int t = 0;
       for (; t + 1 < p.splitk; t += 2) {
-        s0 += pt[t * plane];
-        s1 += pt[(t + 1) * plane];
+        const double v0 = pt[t * plane], v1 = pt[(t + 1) * plane];
+        s0 += v0;
+        s1 += v1;
+        m0 += fabs(v0);
+        m1 += fabs(v1);
       }
-      if (t < p.splitk) s0 += pt[t * plane];
-      mark = a.ea[m] == kBadField || a.eb[n] == kBadField;
+      if (t < p.splitk) {
+        s0 += pt[t * plane];
+        m0 += fabs(pt[t * plane]);
+      }
+      sum = s0 + s1;
+      const int ea = a.ea[m], eb = a.eb[n];
+      mark = ea == kBadField || eb == kBadField;
+      // (|sums| with a field below the scales' by kCoverBits)
+      small = !mark && !p.beside_scales &&
+              exponent_field(m0 + m1) < row_exponent(ea) + row_exponent(eb) - 1023 - kCoverBits;
+    }
+    const Cover& cv = a.out.cover;
+    if (kChain) {  // a warp each
+      for (uint32_t left = __ballot_sync(0xffffffffu, small); left != 0u; left &= left - 1u) {
+        const int l = __ffs(int(left)) - 1;
+        const bool ok =
+            covered_by<1>(cv.row + m * cv.stride, cv.col + (w * 32 + l) * cv.stride, cv.groups);
+        if (lane == l) mark = !ok;
+      }
+    } else {  // long rows: the CTA each
+      if (threadIdx.x == 0) s_count = 0;
+      __syncthreads();
+      if (small) list[atomicAdd(&s_count, 1)] = threadIdx.x;
+      __syncthreads();
+      for (int i = 0; i < s_count; ++i) {
+        const uint32_t t = list[i];
+        const bool ok = covered_by<8>(cv.row + (r0 + (t >> 5)) * cv.stride,
+                                      cv.col + (w * 32 + (t & 31u)) * cv.stride, cv.groups);
+        if (threadIdx.x == t) mark = !ok;
+      }
+      __syncthreads();
+    }
+    if (m < p.Mt && n < p.Nt) {
       if (!mark) {
         int64_t am, cm, bn, cn;
         decode(p.M, m, am, cm);
         decode(p.N, n, bn, cn);
         double* c = p.C + cm + cn;
-        const double v = p.alpha * (s0 + s1);
+        const double v = p.alpha * sum;
         *c = p.beta != 0.0 ? fma(p.beta, *c, v) : v;
       }
     }
@@ -664,12 +711,26 @@ __global__ void __launch_bounds__(256) chain_outputs_kernel(
   const int64_t rblocks = (a.marks.rows + kCRows - 1) / kCRows, items = rblocks * a.marks.words;
   const int mine = int((items - blockIdx.x + gridDim.x - 1) / gridDim.x);
   auto where = [&](int b, int64_t& r, int64_t& w) {
-    const int64_t it = blockIdx.x + int64_t(b) * gridDim.x;
-    w = it / rblocks;
-    r = (it - w * rblocks) * kCRows;
+    const uint32_t it = blockIdx.x + uint32_t(b) * gridDim.x, rb = uint32_t(rblocks);  // < 2^32
+    const uint32_t q = it / rb;
+    w = q;
+    r = int64_t(it - q * rb) * kCRows;
   };
   const int64_t k0 = blockIdx.y * kchunk;
   chain_marked<256>(a, mine, where, buf, sizeof(buf), k0, min(a.K, k0 + kchunk));
+}
+
+// The queued outputs.  (Where the kernel that finds them forms them too, the CTA that has
+// a row or column of many takes as long as all others together.)
+__global__ void __launch_bounds__(256) chain_queue_kernel(const __grid_constant__ ChainOutputs a) {
+  const int count = min(*a.queue.count, a.queue.cap);
+  // neighbouring outputs go to different SMs
+  const int id = ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32 + (threadIdx.x & 31);
+  chain_each(a, count, id, gridDim.x * 256, 0, a.K, [&](int o, int64_t& r, int64_t& n) {
+    const uint2 e = a.queue.entry[o];
+    r = e.x;
+    n = e.y;
+  });
 }
 
 // The ranges' sums of the marked outputs into C.
@@ -727,6 +788,7 @@ Digits alloc_digits(Ctx& c, int64_t rows, int64_t K) {
   d.K = K;
   d.dig = c.alloc<bf16>(size_t(kDigits) * rows * ((K + 7) / 8 * 8));
   d.exps = c.alloc<int>(size_t(rows));
+  d.cover = c.alloc<uint32_t>(size_t(rows) * size_t(cover_stride(K)));
   return d;
 }
 
@@ -755,7 +817,7 @@ void split_sides(Ctx& c, const SplitSide* side, int want0, int want1, int64_t K,
     if (!want[i] || K <= 256) continue;
     want[i] = 0;
     // the modes of this operand alone, joined where they are contiguous in it
-    LongRows a{s.x, s.R, joined(s.K, s.k_is_s1 != 0), s.rows, K, Kp, K, s.exps, s.dig};
+    LongRows a{s.x, s.R, joined(s.K, s.k_is_s1 != 0), s.rows, K, Kp, K, s.exps, s.dig, s.cover};
     const bool multi = a.Kg.n > 1;
     // enough CTAs of the exponent kernels to cover the SMs twice
     const int64_t rb = s.kfast ? 8 : 32, rblocks = (s.rows + rb - 1) / rb;
@@ -843,6 +905,7 @@ Digits digit_rows(Ctx& c, const View& x, int row_dim) {
   s.kfast = x.stride[kd] == 1 && x.stride[row_dim] != 1 ? 1 : 0;
   s.exps = d.exps;
   s.dig = d.dig;
+  s.cover = d.cover;
   const SplitSide side[2] = {s, s};
   split_sides(c, side, 1, 0, d.K, (d.K + 7) / 8 * 8);
   return d;
@@ -859,6 +922,7 @@ Digits operand_digits(Ctx& c, const GettArgs<double>& p, bool first) {
   s.kfast = unit_stride(p.K, !first) && !unit_stride(s.R, false) ? 1 : 0;
   s.exps = d.exps;
   s.dig = d.dig;
+  s.cover = d.cover;
   const SplitSide side[2] = {s, s};
   split_sides(c, side, 1, 0, d.K, (d.K + 7) / 8 * 8);
   return d;
@@ -961,6 +1025,12 @@ void digit_contract(Ctx& c, const GettArgs<double>& p, const Digits* pre_a, cons
   marks.per = split > 1 ? 32 : nt / 2;
   marks.words = int(split > 1 ? (p.Nt + 31) / 32 : 2 * n_tiles);
   marks.word = c.alloc<uint32_t>(size_t(marks.rows) * marks.words);
+  ChainQueue queue{};
+  if (split == 1) {  // room for half of the outputs, 32 MB at most
+    queue.cap = int(std::min(int64_t(1) << 22, M * N / 2));
+    queue.entry = c.alloc<uint2>(size_t(queue.cap));
+    queue.count = c.alloc<int>(1);
+  }
   if (c.sizing()) return;
   CTM_REQUIRE(tiles * split < (int64_t(1) << 31), CTM_ERR_UNSUPPORTED, "einsum: grid too large");
 
@@ -974,6 +1044,7 @@ void digit_contract(Ctx& c, const GettArgs<double>& p, const Digits* pre_a, cons
     s.kfast = unit_stride(p.K, !first) && !unit_stride(s.R, false) ? 1 : 0;
     s.exps = d.exps;
     s.dig = d.dig;
+    s.cover = d.cover;
   };
   fill(side[0], !swap, M, da);
   fill(side[1], swap, N, db);
@@ -1002,6 +1073,8 @@ void digit_contract(Ctx& c, const GettArgs<double>& p, const Digits* pre_a, cons
   d.stages_total = int(stages);
   d.status = status_flags(c);
   d.marks = marks.word;
+  d.queued = queue.count;
+  d.guard = split == 1 && !p.beside_scales ? 1 : 0;
   CUtensorMap tA, tB;
   digit_map(&tA, da.dig, M, Kp, kM);
   digit_map(&tB, db.dig, N, Kp, uint32_t(nt));
@@ -1020,6 +1093,9 @@ void digit_contract(Ctx& c, const GettArgs<double>& p, const Digits* pre_a, cons
   else launch(digit_gemm_kernel<8>);
   CTM_LAUNCH_CHECK();
   ChainOutputs out = chain_outputs(p, split == 1 && swap, marks);
+  const bool as_d = split == 1 || !swap;  // the outputs' rows are da's
+  out.cover = Cover{as_d ? da.cover : db.cover, as_d ? db.cover : da.cover, cover_stride(K),
+                    int(Kp / 8), 0, 0, 0};
   const bool ranges = split > 1 && K > kLongChain;
   if (split > 1) {
     ReduceArgs r{p, swap ? db.exps : da.exps, swap ? da.exps : db.exps, out};
@@ -1033,12 +1109,18 @@ void digit_contract(Ctx& c, const GettArgs<double>& p, const Digits* pre_a, cons
     if (!ranges) return;
     out.part = part;
   }
+  if (split > 1 || p.beta != 0.0) out.cover.col = nullptr;  // marks are final
+  out.queue = queue;
   const int64_t blocks = (marks.rows + kCRows - 1) / kCRows * marks.words;
   KernelTimer kt(c.stream, "chain_outputs_kernel", kUnitByte, 4.0 * double(marks.rows) * marks.words);
   chain_outputs_kernel<<<dim3(unsigned(std::min<int64_t>(blocks, 4 * sms)),
                               unsigned(ranges ? split : 1)),
                          256, 0, c.stream>>>(out, ranges ? (K + split - 1) / split : K);
   CTM_LAUNCH_CHECK();
+  if (split == 1) {
+    chain_queue_kernel<<<unsigned(4 * sms), 256, 0, c.stream>>>(out);
+    CTM_LAUNCH_CHECK();
+  }
   if (ranges) {
     chain_sum_kernel<<<grid_for(marks.rows * marks.words, 256), 256, 0, c.stream>>>(out, int(split));
     CTM_LAUNCH_CHECK();

@@ -19,6 +19,29 @@ __device__ __forceinline__ int exponent_field(double x) {
   return int((unsigned long long)__double_as_longlong(x) >> 52) & 0x7ff;
 }
 
+// Which outputs the digits may form.  Their error is relative to the product sA sB of the
+// row's and the column's scales, an FMA chain's to S = sum_k |a_k b_k|: where the large
+// entries of a row meet the small ones of a column (or zeros), S is far below sA sB and the
+// digits would lose what the chain keeps.  So an output is left to the chain unless
+// S >= 2^-8.4 sA sB is known: from |C| <= S, from the K ranges' |sums|, or from classes of
+// the entries, large (above 2^-4.2 of the scale) and medium (above 2^-7): one k with two
+// large ones, 8 with a large and a medium one or 48 with two medium ones.  With that the
+// dropped digit products' deviation, sqrt(K) 2^-62.2 sA sB, is at most sqrt(K) 2^-53.8 S.
+// Where no k has two nonzero entries, zero is exact.
+// (Environments at D = 6, chi = 144: 1.4 % of the outputs of 5184 x 5184 x 144 are below
+// 2^-8, 0.05 to 0.1 % fail the classes; none of the products over 36, 72 or 5184 does.)
+//
+// A word tells of eight consecutive entries: bits 0-7 large (|top digit| >= 4), 8-15
+// medium (>= 1), 16-23 nonzero.
+constexpr int kCoverBits = 8;      // |C| >= 2^-8 sA sB: no look at the entries
+constexpr int kCoverSum = 48;      // units of 2^-14
+constexpr uint32_t kBadCover = 1;  // first word of a row without digits
+__host__ __device__ inline int64_t cover_stride(int64_t K) { return (K + 31) / 32 * 4; }
+
+__device__ __forceinline__ bool large_digit(unsigned long long u) {
+  return uint32_t(u >> 56) - 125u > 6u;
+}
+
 // Digit b (0..7, 0 the least significant) of the biased word w as BF16 bits in
 // the upper half: the byte minus 128, exact.
 __device__ __forceinline__ uint32_t digit_f32(uint32_t w, int byte) {
@@ -58,11 +81,18 @@ __device__ __forceinline__ void put_digits(const unsigned long long (&u)[8], Put
   }
 }
 
-__device__ __forceinline__ void write_digits(const double (&x)[8], int E, bf16* dst,
-                                             int64_t plane) {
+__device__ __forceinline__ void write_digits(const double (&x)[8], int field, bf16* dst,
+                                             int64_t plane, uint32_t* cover) {
   unsigned long long u[8];
+  const int E = row_exponent(field);
+  uint32_t c = 0;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) u[i] = digit_word(x[i], E);
+  for (int i = 0; i < 8; ++i) {
+    u[i] = digit_word(x[i], E);
+    c |= (large_digit(u[i]) ? 1u : 0u) << i | (uint32_t(u[i] >> 56) != 128u ? 0x100u : 0u) << i |
+         (x[i] != 0.0 ? 0x10000u : 0u) << i;
+  }
+  *cover = field == kBadField ? kBadCover : c;
   put_digits(u, [&](int d, uint4 w) { *reinterpret_cast<uint4*>(dst + int64_t(d) * plane) = w; });
 }
 
@@ -118,7 +148,8 @@ inline ChainArgs chain_args(const GettArgs<double>& p, bool swap) {
 
 // Outputs that the products leave to the FMA chain (digits_chain.cuh): bit b of
 // word[w * rows + r] is the one of row r and column w * per + b.  Every word is
-// written by the kernel that forms the outputs; marked ones are not stored.
+// written by the kernel that forms the outputs.  Marked ones are not to be relied on
+// (with beta = 0 they may be stored like the others) unless Cover says so.
 struct Marks {
   uint32_t* word;
   int64_t rows;
@@ -129,8 +160,29 @@ __device__ __forceinline__ uint32_t low_bits(int n) {
   return n >= 32 ? ~0u : n > 0 ? (1u << n) - 1u : 0u;
 }
 
+// Whether a candidate's digits may stand: words of rows and columns (null: they may not).
+struct Cover {
+  const uint32_t* row;
+  const uint32_t* col;
+  int64_t stride;
+  int groups;           // words of a row
+  // rows of the streaming kernel: [4 phase + 2 half + {large, nonzero}][row], bits 8 q of
+  // its block q of 16 entries; phases 0: as the columns
+  int phases, per_phase, blocks;
+};
+
+// Marked outputs (row, column) for a kernel of their own; cap entries, others are formed
+// where they are found.  count is zeroed before.
+struct ChainQueue {
+  uint2* entry;         // null: no queue
+  int* count;
+  int cap;
+};
+
 struct ChainOutputs {
   ChainArgs ch;
+  Cover cover;
+  ChainQueue queue;
   Group GM, GN;         // output strides of rows and columns (m[].s1)
   Marks marks;
   int64_t columns, K;

@@ -45,6 +45,8 @@ struct StreamArgs {
   int nbuf;                       // digit buffers of the long operand
   int64_t tiles;
   int* status;
+  int guard;                      // small outputs are marked too
+  uint32_t* cover;                // of the long operand's rows (Cover::row)
   ChainOutputs out;               // word 2 * pass + half
 };
 
@@ -195,12 +197,25 @@ __global__ void __launch_bounds__(kSThreads, 1)
                           : 0ull;
           }
       };
-      auto words = [&](int E) {
+      // phase ph's entries into words, and which of them are large or nonzero
+      auto words = [&](int e, int ph, int count, bool note) {
+        const int E = row_exponent(e);
+        uint32_t large = 0u, nonzero = 0u;
 #pragma unroll
-        for (int q = 0; q < kGroups; ++q)
+        for (int q = 0; q < kGroups; ++q) {
+          if (q >= count) continue;
 #pragma unroll
-          for (int i = 0; i < 8; ++i)
+          for (int i = 0; i < 8; ++i) {
+            nonzero |= (u[q][i] << 1 != 0ull ? 1u : 0u) << (8 * q + i);
             u[q][i] = digit_word(__longlong_as_double((long long)u[q][i]), E);
+            large |= (large_digit(u[q][i]) ? 1u : 0u) << (8 * q + i);
+          }
+        }
+        if (note && valid) {
+          uint32_t* c = p.cover + int64_t(4 * ph + 2 * half) * p.M + m;
+          c[0] = e == kBadField ? 1u : large;
+          c[p.M] = e == kBadField ? 0u : nonzero;
+        }
       };
       int e = 0;
       if (p.phases == 1) {
@@ -216,14 +231,13 @@ __global__ void __launch_bounds__(kSThreads, 1)
       s_half[half][row] = e;
       asm volatile("bar.sync 2, 256;" ::: "memory");  // the eight splitting warps
       e = max(e, s_half[half ^ 1][row]);
-      const int E = row_exponent(e);
-      if (p.phases == 1) words(E);
+      if (p.phases == 1) words(e, 0, p.blocks, true);
       for (int f = 0; f < refills; ++f, ++fill) {
         const int first = (f % p.phases) * p.per_phase;
         const int count = min(p.per_phase, p.blocks - first);
         if (p.phases > 1) {
           load(first, count);
-          words(E);
+          words(e, f % p.phases, count, f < p.phases);
         }
         const int b = int(fill) % p.nbuf;
         ok = ok && wait_warp(&a_empty[b], ((fill / uint32_t(p.nbuf)) & 1u) ^ 1u);
@@ -304,6 +318,7 @@ __global__ void __launch_bounds__(kSThreads, 1)
     constexpr int kHalf = NT / 2;
     constexpr int kSmallGroups = kMode == 0 ? 8 : kMode == 1 ? 4 : 2;
     constexpr int kUnit = kMode == 0 ? 57 : kMode == 1 ? 56 : 55;
+    const unsigned long long small = p.guard ? 1ull << (kUnit - kCoverBits) : 0ull;
     const bool scaled = !(p.alpha == 1.0 && p.beta == 0.0);
     const int lane_base = (warp & 3) * 32, half = (warp - 8) >> 2;
     const int row = lane_base + lane;
@@ -351,6 +366,7 @@ __global__ void __launch_bounds__(kSThreads, 1)
             if (valid && off >= 0) {
               const int ec = s_eb[n0 + c + j];
               const unsigned long long mag = (unsigned long long)(fx < 0 ? -fx : fx);
+              if (mag < small) mark |= 1u << (c + j);
               const int lz = __clzll((long long)mag);
               const unsigned long long nm = mag << (lz & 63);
               // 53 bits, to nearest even
@@ -460,6 +476,7 @@ void stream_contract(Ctx& c, const GettArgs<double>& p, bool swap) {
   marks.per = pl.nt / 2;
   marks.words = 2 * pl.passes;
   marks.word = c.alloc<uint32_t>(size_t(marks.rows) * marks.words);
+  a.cover = c.alloc<uint32_t>(size_t(4 * pl.phases) * size_t(a.M));
   if (c.sizing()) return;
   a.x = swap ? p.B : p.A;
   a.FX = swap ? p.N : p.M;
@@ -478,7 +495,10 @@ void stream_contract(Ctx& c, const GettArgs<double>& p, bool swap) {
   a.nbuf = pl.nbuf;
   a.tiles = (a.M + kTileM - 1) / kTileM;
   a.status = status_flags(c);
+  a.guard = p.beside_scales ? 0 : 1;
   a.out = chain_outputs(p, swap, marks);
+  a.out.cover = Cover{a.cover, p.beta != 0.0 ? nullptr : db.cover, cover_stride(p.Kt),
+                      int((p.Kt + 7) / 8), pl.phases, pl.per_phase, pl.blocks};
   const int64_t Kp = (p.Kt + 7) / 8 * 8;
   CUtensorMap tB;
   {

@@ -11,6 +11,7 @@ namespace ctm {
 struct Digits {
   __nv_bfloat16* dig = nullptr;
   int* exps = nullptr;
+  uint32_t* cover = nullptr;  // which entries are large, by eight (digits.cuh)
   int64_t rows = 0, K = 0;
 };
 // Of a 2-D view whose dimension row_dim is kept and the other contracted.
@@ -22,9 +23,11 @@ bool digits_pay(int64_t rows, int64_t columns, int64_t K);
 // labels split into batch / row / column / contracted groups (no traces, no
 // outer-only labels).  All views are strided; nothing is copied.
 // da, db: digits of A's and B's rows (one kept and one contracted index each).
+// beside_scales: an error of 2^-60 of the largest entries of an output's row and column
+// does no harm, however small their products are (digits.cuh).
 void einsum(Ctx& c, const char* spec, const View& A, const View& B, const View& C,
             double alpha = 1.0, double beta = 0.0, const Digits* da = nullptr,
-            const Digits* db = nullptr);
+            const Digits* db = nullptr, bool beside_scales = false);
 // The same contraction in FP32 (FP32 FMAs, FP32 accumulation).
 void einsum(Ctx& c, const char* spec, const ViewF& A, const ViewF& B, const ViewF& C,
             double alpha = 1.0, double beta = 0.0);

@@ -330,7 +330,7 @@ int64_t group_size(const Group& g) {
 template <class T>
 void einsum_impl(Ctx& c, const char* spec, const ViewT<T>& A, const ViewT<T>& B, const ViewT<T>& C,
                  double alpha, double beta, const Digits* da = nullptr,
-                 const Digits* db = nullptr) {
+                 const Digits* db = nullptr, bool beside_scales = false) {
   std::string s(spec);
   const size_t comma = s.find(','), arrow = s.find("->");
   CTM_REQUIRE(comma != std::string::npos && arrow != std::string::npos, CTM_ERR_INVALID,
@@ -414,6 +414,7 @@ void einsum_impl(Ctx& c, const char* spec, const ViewT<T>& A, const ViewT<T>& B,
   p.bext = bext; p.bsa = bsa; p.bsb = bsb; p.bsc = bsc;
   p.alpha = T(alpha);
   p.beta = T(beta);
+  p.beside_scales = beside_scales ? 1 : 0;
   if (p.Mt == 0 || p.Nt == 0) return;
   // loaders walk K fastest when K, not the row / column group, is unit-stride
   p.kfa = (p.K.n > 0 && p.K.m[p.K.n - 1].s0 == 1 &&
@@ -539,8 +540,8 @@ void einsum_impl(Ctx& c, const char* spec, const ViewT<T>& A, const ViewT<T>& B,
 }
 
 void einsum(Ctx& c, const char* spec, const View& A, const View& B, const View& C, double alpha,
-            double beta, const Digits* da, const Digits* db) {
-  einsum_impl<double>(c, spec, A, B, C, alpha, beta, da, db);
+            double beta, const Digits* da, const Digits* db, bool beside_scales) {
+  einsum_impl<double>(c, spec, A, B, C, alpha, beta, da, db, beside_scales);
 }
 
 void einsum(Ctx& c, const char* spec, const ViewF& A, const ViewF& B, const ViewF& C, double alpha,

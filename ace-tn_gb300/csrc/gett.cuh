@@ -32,6 +32,7 @@ struct GettArgs {
   T* part;
   int kfa, kfb;  // tile loaders walk K fastest (K is the unit-stride mode of A / B)
   int swap_xy;   // grid x runs over column tiles (more than 65535 of them)
+  int beside_scales;  // outputs need only be exact beside their row's and column's largest entries
   int sym;       // A and B are one operand (a Gram matrix): tiles above the diagonal are mirrored
 };
 

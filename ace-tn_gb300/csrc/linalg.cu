@@ -1388,6 +1388,31 @@ void slab_gram(Ctx& c, const float* Y, int64_t n, int64_t q, const float* Lt, fl
   CTM_LAUNCH_CHECK();
 }
 
+// Columns of Y (n x q) and G = Y^T Y scaled by powers of two, column norms to [1, 2)
+// (the exponents, from G's diagonal, to e; Gs: the scaled G).
+__global__ void __launch_bounds__(256) equilibrate_kernel(double* Y, const double* G, int64_t n,
+                                                          int q, double* Gs, int* e) {
+  extern __shared__ double s_scale[];
+  for (int k = threadIdx.x; k < q; k += blockDim.x) {
+    const int f = int((unsigned long long)__double_as_longlong(G[size_t(k) * q + k]) >> 52);
+    const int d = f > 0 && f < 2047 ? (f - 1023) >> 1 : 0;  // 4^d <= |y|^2 < 4^(d + 1)
+    s_scale[k] = __longlong_as_double((long long)(1023 - d) << 52);
+    if (blockIdx.x == 0) e[k] = d;
+  }
+  __syncthreads();
+  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n * q;
+       i += int64_t(gridDim.x) * blockDim.x)
+    Y[i] *= s_scale[i % q];
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < q * q; i += gridDim.x * blockDim.x)
+    Gs[i] = G[i] * s_scale[i / q] * s_scale[i % q];
+}
+
+__global__ void __launch_bounds__(256) scale_r_kernel(const double* Rs, int q, const int* e,
+                                                      double* R) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < q * q; i += gridDim.x * blockDim.x)
+    R[i] = Rs[i] * __longlong_as_double((long long)(1023 + e[i % q]) << 52);
+}
+
 template <class T>
 void orthonormalize_impl(Ctx& c, T* Y, int64_t n, int64_t q, T* R, int stages,
                          int* failed = nullptr) {
@@ -1443,6 +1468,13 @@ void orthonormalize_impl(Ctx& c, T* Y, int64_t n, int64_t q, T* R, int stages,
   // stage's L^-T (forward substitution with L^T) and forms the next Gram
   // matrix in the same pass over the rows; the factorisation forms no inverse
   const bool fast_f32 = sizeof(T) == 4 && q <= 192;
+  // FP64 with digit products: the columns are scaled to equal norms by powers of two
+  // first (graded ones, as a randomized SVD's B^T has, would meet an oppositely graded
+  // L^-1, and their products go through FMA chains: 1 ms at 5184 x 160).  Then a small
+  // entry of Q may lose bits beside its row's largest: no more than the Gram matrix's
+  // rounding has cost already, so the product need not look after it.
+  const bool equal = sizeof(T) == 8 && digits_pay(n, q, q) && q <= 4096;
+  int* expo = c.alloc<int>(size_t(q));
   // (a factorisation that is used without the fallback has to be orthonormal to
   // working precision)
   const T tol = sizeof(T) == 8 ? T(failed != nullptr ? 1e-13 : stages == 3 ? 1e-11 : 1e-6) : T(stages == 3 ? 2e-4 : 5e-2);
@@ -1473,7 +1505,16 @@ void orthonormalize_impl(Ctx& c, T* Y, int64_t n, int64_t q, T* R, int stages,
     }
   } else {
     for (int stage = 0; stage < stages; ++stage) {
+      T* Gs = equal && stage == 0 ? Rt2 : G;
       einsum(c, "ia,ib->ab", ViewT<T>(cur, {n, q}), ViewT<T>(cur, {n, q}), ViewT<T>(G, {q, q}));
+      if constexpr (sizeof(T) == 8) {
+        if (Gs != G && !c.sizing()) {
+          KernelTimer kt(c.stream, "equilibrate_kernel", kUnitByte, 16.0 * double(n) * q);
+          equilibrate_kernel<<<grid_for(n * q, 1024), 256, size_t(q) * sizeof(double), c.stream>>>(
+              cur, G, n, int(q), Gs, expo);
+          CTM_LAUNCH_CHECK();
+        }
+      }
       const int mode = stage < shifted_stages ? (sizeof(T) == 8 ? 1 : 2) : 0;
       bool done = false;
       if constexpr (sizeof(T) == 8) {
@@ -1483,13 +1524,15 @@ void orthonormalize_impl(Ctx& c, T* Y, int64_t n, int64_t q, T* R, int stages,
                                    : 0.0;
         done = cholesky_cluster_fits(q);
         if (done && !c.sizing())
-          cholesky_cluster(c, G, q, f, Li, R != nullptr ? Lt : nullptr, flags);
+          cholesky_cluster(c, Gs, q, f, Li, R != nullptr ? Lt : nullptr, flags);
       }
       if (!done && !c.sizing())
-        cholesky<T>(c.stream, G, q, n, mode, Wk, Ek, nullptr, Li, R != nullptr ? Lt : nullptr,
+        cholesky<T>(c.stream, Gs, q, n, mode, Wk, Ek, nullptr, Li, R != nullptr ? Lt : nullptr,
                     flags);
       // nxt = cur @ Linv^T
-      einsum(c, "ia,ba->ib", ViewT<T>(cur, {n, q}), ViewT<T>(Li, {q, q}), ViewT<T>(nxt, {n, q}));
+      const ViewT<T> x(cur, {n, q}), l(Li, {q, q}), y(nxt, {n, q});
+      if constexpr (sizeof(T) == 8) einsum(c, "ia,ba->ib", x, l, y, 1.0, 0.0, nullptr, nullptr, equal);
+      else einsum(c, "ia,ba->ib", x, l, y);
       accumulate_r(stage);
       std::swap(cur, nxt);
     }
@@ -1506,8 +1549,14 @@ void orthonormalize_impl(Ctx& c, T* Y, int64_t n, int64_t q, T* R, int stages,
   }
   if (cur != Y)
     CTM_CUDA(cudaMemcpyAsync(Y, cur, sizeof(T) * n * q, cudaMemcpyDeviceToDevice, c.stream));
-  if (R != nullptr)
+  if (R != nullptr && !equal)
     CTM_CUDA(cudaMemcpyAsync(R, Rt, sizeof(T) * q * q, cudaMemcpyDeviceToDevice, c.stream));
+  if constexpr (sizeof(T) == 8) {
+    if (R != nullptr && equal) {
+      scale_r_kernel<<<grid_for(q * q, 1024), 256, 0, c.stream>>>(Rt, int(q), expo, R);
+      CTM_LAUNCH_CHECK();
+    }
+  }
   if (failed != nullptr) return;  // the caller looks at the flag
   // when flagged: Y = the saved input, then its Householder QR
   householder_qr_kernel<T><<<1, LT, 0, c.stream>>>(Y, n, q, R, hv, beta, flags, 1, V);
