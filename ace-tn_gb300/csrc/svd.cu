@@ -57,8 +57,9 @@ __device__ double block_sum(double v, double* sh) {
 //    orthogonal map up to rounding for any h as long as s = 2 h / (1 + h^2)
 //    holds in FP64, so that the angle itself may be an FP32 number;
 //  * the angle and the convergence test in FP32 on mantissas and exponents
-//    taken from the FP64 bit patterns by integer instructions (any scale of
-//    the input, no FP64 division, square root or conversion);
+//    taken from the FP64 bit patterns by integer instructions (no FP64
+//    division, square root or conversion; norms and dot products have to be
+//    normal numbers, which svd_thin's scaling provides);
 //  * squared row norms kept and updated (5 instructions) instead of two more
 //    dot products per pair, and recomputed at the start of every sweep;
 //  * two pairs per warp (kTP = 16 lanes each) where that fills the four SM
@@ -510,14 +511,65 @@ __global__ void __launch_bounds__(LT) row_norms_kernel(const double* W, int64_t 
   if (threadIdx.x == 0) norm2[blockIdx.x] = part;
 }
 
+// The input is scaled by a power of two that puts its largest entry's exponent at kTop:
+// squared norms stay below 2^1023 and the dot products of rows 2^-900 as long are still
+// normal numbers.  (Exact, so the result has the same bits wherever none underflowed.)
+constexpr int kTop = 440;
+
+// Largest exponent field of the finite entries; *top zeroed where the grid has several CTAs.
+__global__ void __launch_bounds__(1024) top_field_kernel(const double* X, int64_t n, int* top) {
+  int e = 0;
+  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n;
+       i += int64_t(gridDim.x) * blockDim.x) {
+    const int f = int((unsigned long long)__double_as_longlong(X[i]) >> 52) & 0x7ff;
+    if (f != 0x7ff) e = max(e, f);
+  }
+  for (int o = 16; o > 0; o >>= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, o));
+  __shared__ int s_top;
+  if (threadIdx.x == 0) s_top = 0;
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) atomicMax(&s_top, e);
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  if (gridDim.x == 1) *top = s_top;
+  else atomicMax(top, s_top);
+}
+
+__device__ __forceinline__ double pow2(int e) {
+  return __longlong_as_double((long long)(e + 1023) << 52);
+}
+
+// x 2^e in two steps, the first of them exact where the second is not.
+__device__ __forceinline__ double scaled(double x, int e) {
+  return x * pow2(e / 2) * pow2(e - e / 2);
+}
+
+// Exponent of the scaling (even: the halves of the exponents that a square root sees stay).
+__device__ __forceinline__ int scale_exponent(int top) {
+  return (kTop + 1023 - max(top, 1)) & ~1;
+}
+
+// dst[r][c] = X[r s0 + c s1] 2^e, rows x cols.
+__global__ void __launch_bounds__(256) scaled_copy_kernel(const double* X, int64_t rows,
+                                                          int64_t cols, int64_t s0, int64_t s1,
+                                                          const int* top, double* dst) {
+  const int e = scale_exponent(*top);
+  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < rows * cols;
+       i += int64_t(gridDim.x) * blockDim.x) {
+    const int64_t r = i / cols, q = i - r * cols;
+    dst[i] = scaled(X[r * s0 + q * s1], e);
+  }
+}
+
 // Sorts the Jacobi result by descending row norm and writes the singular
 // values and vectors, one CTA per row j: rank r of row j (strictly larger
-// norms, ties by index), S[r] = |W_j|, the short side's vectors
+// norms, ties by index), S[r] = |W_j| without the scaling, the short side's vectors
 // Vs[t][r] = J_j[t] (p x p), the long side's Vl[t][r] = W_j[t] / S[r] (L x p).
 __global__ void __launch_bounds__(LT) jacobi_finish_kernel(const double* W, const double* J,
                                                            const double* norm2, int64_t p,
                                                            int64_t L, double* Vs, double* S,
-                                                           double* Vl, const int* only_if) {
+                                                           double* Vl, const int* top,
+                                                           const int* only_if) {
   if (only_if != nullptr && (*only_if & 1) == 0) return;
   const int64_t j = blockIdx.x;
   __shared__ int s_rank;
@@ -534,7 +586,7 @@ __global__ void __launch_bounds__(LT) jacobi_finish_kernel(const double* W, cons
   const int64_t rk = s_rank;
   const double sj = sqrt(nj2);
   const double inv = sj > 0.0 ? 1.0 / sj : 0.0;
-  if (threadIdx.x == 0) S[rk] = sj;
+  if (threadIdx.x == 0) S[rk] = scaled(sj, -scale_exponent(*top));
   for (int64_t t = threadIdx.x; t < p; t += blockDim.x) Vs[t * p + rk] = J[j * p + t];
   for (int64_t t = threadIdx.x; t < L; t += blockDim.x) Vl[t * p + rk] = W[j * L + t] * inv;
 }
@@ -547,9 +599,9 @@ __global__ void identity_kernel(double* X, int64_t p, const int* only_if) {
 }
 
 void finish(Ctx& c, const double* W, const double* J, const double* norm2, int64_t p, int64_t L,
-            double* Vs, double* S, double* Vl, const int* only_if) {
+            double* Vs, double* S, double* Vl, const int* top, const int* only_if) {
   KernelTimer kt(c.stream, "jacobi_finish_kernel", kUnitByte, 16.0 * double(p) * (p + L));
-  jacobi_finish_kernel<<<unsigned(p), LT, 0, c.stream>>>(W, J, norm2, p, L, Vs, S, Vl, only_if);
+  jacobi_finish_kernel<<<unsigned(p), LT, 0, c.stream>>>(W, J, norm2, p, L, Vs, S, Vl, top, only_if);
   CTM_LAUNCH_CHECK();
 }
 
@@ -713,13 +765,22 @@ void svd_thin(Ctx& c, const double* X, int64_t m, int64_t n, double* U, double* 
   double* W = c.alloc<double>(size_t(p) * L);
   double* J = c.alloc<double>(size_t(p) * p);
   double* norm2 = c.alloc<double>(p);
-  auto load_w = [&] {  // W rows = columns of X (tall) or rows of X
+  int* top = c.alloc<int>(1);
+  // dst = X (rows first) or X^T, scaled
+  auto load = [&](double* dst, bool transposed) {
     if (c.sizing()) return;
-    if (tall)
-      copy2d(c, View(X, {m, n}).permute({1, 0}), W, L);
-    else
-      CTM_CUDA(cudaMemcpyAsync(W, X, sizeof(double) * m * n, cudaMemcpyDeviceToDevice, c.stream));
+    KernelTimer kt(c.stream, "scaled_copy_kernel", kUnitByte, 16.0 * double(m) * n);
+    scaled_copy_kernel<<<grid_for(m * n, 256), 256, 0, c.stream>>>(
+        X, transposed ? n : m, transposed ? m : n, transposed ? 1 : n, transposed ? n : 1, top, dst);
+    CTM_LAUNCH_CHECK();
   };
+  auto load_w = [&] { load(W, tall); };  // W rows = columns of X (tall) or rows of X
+  if (!c.sizing()) {
+    const int ctas = int(std::min<int64_t>(sm_count_linalg(), (m * n + 32767) / 32768));
+    if (ctas > 1) CTM_CUDA(cudaMemsetAsync(top, 0, sizeof(int), c.stream));
+    top_field_kernel<<<ctas, 1024, 0, c.stream>>>(X, m * n, top);
+    CTM_LAUNCH_CHECK();
+  }
   const JacobiShape direct = jacobi_shape(p, L), square = jacobi_shape(p, p);
   // The one-cluster Householder QR up to the size where the Cholesky-QR (about
   // 20 launches and three one-SM factorisations) is faster; the latter only
@@ -739,7 +800,7 @@ void svd_thin(Ctx& c, const double* X, int64_t m, int64_t n, double* U, double* 
     } else {
       jacobi_grid(c, W, J, norm2, p, L, nullptr);
     }
-    if (!c.sizing()) finish(c, W, J, norm2, p, L, Vs, S, Vl, nullptr);
+    if (!c.sizing()) finish(c, W, J, norm2, p, L, Vs, S, Vl, top, nullptr);
     return;
   }
   // long side = Y R.  The rows of R are rotated, R = J^T W: the short side's
@@ -751,25 +812,20 @@ void svd_thin(Ctx& c, const double* X, int64_t m, int64_t n, double* U, double* 
   double* W2 = c.alloc<double>(size_t(p) * p);
   double* Xs = c.alloc<double>(size_t(p) * p);
   int* failed = c.alloc<int>(1);
-  if (!c.sizing()) {
-    if (tall)
-      CTM_CUDA(cudaMemcpyAsync(Y, X, sizeof(double) * m * n, cudaMemcpyDeviceToDevice, c.stream));
-    else
-      copy2d(c, View(X, {m, n}).permute({1, 0}), Y, p);
-  }
+  load(Y, !tall);
   if (!house) orthonormalize_try(c, Y, L, p, R, failed);
   else if (!c.sizing()) householder_cluster(c, Y, L, p, R);
   const int* const flag = house ? nullptr : failed;
   if (!c.sizing())
     CTM_CUDA(cudaMemcpyAsync(W2, R, sizeof(double) * p * p, cudaMemcpyDeviceToDevice, c.stream));
   jacobi_square(c, W2, J, norm2, p, flag);
-  if (!c.sizing()) finish(c, W2, J, norm2, p, p, Xs, S, Vs, nullptr);
+  if (!c.sizing()) finish(c, W2, J, norm2, p, p, Xs, S, Vs, top, nullptr);
   einsum(c, "ik,kj->ij", View(Y, {L, p}), View(Xs, {p, p}), View(Vl, {L, p}));
   if (house) return;
   // when the Cholesky-QR has failed: the whole matrix again, in global memory
   load_w();
   jacobi_grid(c, W, J, norm2, p, L, failed);
-  if (!c.sizing()) finish(c, W, J, norm2, p, L, Vs, S, Vl, failed);
+  if (!c.sizing()) finish(c, W, J, norm2, p, L, Vs, S, Vl, top, failed);
 }
 
 }  // namespace ctm
