@@ -563,7 +563,8 @@ __global__ void __launch_bounds__(256) scaled_copy_kernel(const double* X, int64
 
 // Sorts the Jacobi result by descending row norm and writes the singular
 // values and vectors, one CTA per row j: rank r of row j (strictly larger
-// norms, ties by index), S[r] = |W_j| without the scaling, the short side's vectors
+// norms, ties by index; NaNs, whose bits are above an infinity's, come first and
+// so have ranks of their own: every output is written), S[r] = |W_j| without the scaling, the short side's vectors
 // Vs[t][r] = J_j[t] (p x p), the long side's Vl[t][r] = W_j[t] / S[r] (L x p).
 __global__ void __launch_bounds__(LT) jacobi_finish_kernel(const double* W, const double* J,
                                                            const double* norm2, int64_t p,
@@ -574,12 +575,14 @@ __global__ void __launch_bounds__(LT) jacobi_finish_kernel(const double* W, cons
   const int64_t j = blockIdx.x;
   __shared__ int s_rank;
   const double nj2 = norm2[j];
+  auto key = [](double v) { return __double_as_longlong(v) & 0x7fffffffffffffffll; };
+  const long long kj = key(nj2);
   if (threadIdx.x == 0) s_rank = 0;
   __syncthreads();
   int cnt = 0;
   for (int64_t i = threadIdx.x; i < p; i += blockDim.x) {
-    const double ni2 = norm2[i];
-    if (i != j && (ni2 > nj2 || (ni2 == nj2 && i < j))) ++cnt;
+    const long long ki = key(norm2[i]);
+    if (i != j && (ki > kj || (ki == kj && i < j))) ++cnt;
   }
   if (cnt != 0) atomicAdd(&s_rank, cnt);
   __syncthreads();
