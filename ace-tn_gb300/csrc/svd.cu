@@ -122,9 +122,15 @@ struct ClusterJacobi {
   const int* skip;  // nothing to do when (*skip & 1)
 };
 
-// Doubles per row in shared memory: the row, its rotations, its squared norm
-// (an even number: block moves are 16-byte copies).
-__host__ __device__ inline int jacobi_row(int p, int L) { return (L + p + 2) & ~1; }
+// Doubles per row in shared memory: the row, its rotations, its squared norm and the first
+// sweep's (an even number: block moves are 16-byte copies).
+__host__ __device__ inline int jacobi_row(int p, int L) { return (L + p + 3) & ~1; }
+
+// A row this much shorter than at first (squares) is what is left of a linear combination of
+// the others, a rounding error 2^-53 of its first length and smaller by 2^-23 after each
+// sweep: it becomes zero.  (Otherwise it is rotated until it underflows: with the input
+// scaled to 2^440, more than 60 sweeps.)
+constexpr double kCollapsed = 0x1p-150;
 
 // One rotation of rows x and y (L entries, then p of the accumulated rotations,
 // then the squared norm) by the kTP lanes of a group; returns whether it was
@@ -244,7 +250,15 @@ __global__ void __launch_bounds__(512) jacobi_cluster_f64_kernel(const ClusterJa
       double v = 0.0;
       for (int t = lane; t < L; t += 32) v = fma(s[t], s[t], v);
       v = warp_sum(v);
-      if (lane == 0) s[L + p] = v;
+      if (sweep > 0 && v < kCollapsed * s[L + p + 1]) {
+        for (int t = lane; t < L; t += 32) s[t] = 0.0;
+        v = 0.0;
+      }
+      __syncwarp();
+      if (lane == 0) {
+        s[L + p] = v;
+        if (sweep == 0) s[L + p + 1] = v;
+      }
     }
     __syncthreads();
     bool rotated = false;
@@ -399,6 +413,7 @@ struct JacobiArgs {
   int64_t p, L;
   int64_t pp;     // p rounded up to even
   double tol;
+  const double* first;  // p: squared norms before the sweeps (kCollapsed)
   int max_sweeps;
   unsigned* bar;  // [0] arrival count, [1] generation, [2] abort, [3..4] sweep flags
   int* flags;
@@ -471,7 +486,9 @@ __global__ void __launch_bounds__(64) jacobi_sweeps_kernel(const JacobiArgs a) {
         al = warp_sum(al);
         be = warp_sum(be);
         ga = warp_sum(ga);
-        if (al == 0.0 || be == 0.0 || !(fabs(ga) > a.tol * sqrt(al) * sqrt(be))) continue;
+        if (al <= kCollapsed * a.first[i] || be <= kCollapsed * a.first[j] ||
+            !(fabs(ga) > a.tol * sqrt(al) * sqrt(be)))
+          continue;
         const double zeta = (be - al) / (2.0 * ga);
         const double t = copysign(1.0, zeta) / (fabs(zeta) + sqrt(fma(zeta, zeta, 1.0)));
         const double cs = 1.0 / sqrt(fma(t, t, 1.0));
@@ -499,15 +516,20 @@ __global__ void __launch_bounds__(64) jacobi_sweeps_kernel(const JacobiArgs a) {
   if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(a.flags, 2);
 }
 
-// Squared norms of the rows of W (p x L), one CTA per row.
-__global__ void __launch_bounds__(LT) row_norms_kernel(const double* W, int64_t L, double* norm2,
-                                                       const int* only_if) {
+// Squared norms of the rows of W (p x L), one CTA per row; with those before the sweeps,
+// collapsed rows become zero.
+__global__ void __launch_bounds__(LT) row_norms_kernel(double* W, int64_t L, double* norm2,
+                                                       const double* first, const int* only_if) {
   if (only_if != nullptr && (*only_if & 1) == 0) return;
   __shared__ double sh[LT / 32];
-  const double* w = W + int64_t(blockIdx.x) * L;
+  double* w = W + int64_t(blockIdx.x) * L;
   double part = 0.0;
   for (int64_t t = threadIdx.x; t < L; t += blockDim.x) part = fma(w[t], w[t], part);
   part = block_sum(part, sh);
+  if (first != nullptr && part < kCollapsed * first[blockIdx.x]) {
+    for (int64_t t = threadIdx.x; t < L; t += blockDim.x) w[t] = 0.0;
+    part = 0.0;
+  }
   if (threadIdx.x == 0) norm2[blockIdx.x] = part;
 }
 
@@ -594,6 +616,99 @@ __global__ void __launch_bounds__(LT) jacobi_finish_kernel(const double* W, cons
   for (int64_t t = threadIdx.x; t < L; t += blockDim.x) Vl[t * p + rk] = W[j * L + t] * inv;
 }
 
+// Short side's vectors from the rows of a factor R, V (p x p), S sorted: where R has no full
+// rank in exact arithmetic, the rotations shrink its last rows towards zero, and what is left
+// of them, normalised, is a rounding error, or nothing.  These two kernels put vectors
+// orthogonal to the others in such places.
+//
+// loose[r]: whether column r, of a value below 1e-8 of the largest, is not orthonormal to the
+// others.  One CTA per column (2 us without small values).
+__global__ void __launch_bounds__(LT) loose_columns_kernel(const double* V, const double* S, int p,
+                                                           int* loose) {
+  const int r = blockIdx.x, tid = threadIdx.x;
+  if (!(S[r] < 1e-8 * S[0] || S[r] == 0.0)) {
+    if (tid == 0) loose[r] = 0;
+    return;
+  }
+  const double tol = 16.0 * 2.220446049250313e-16 * sqrt(double(p));
+  extern __shared__ double s_col[];
+  for (int t = tid; t < p; t += LT) s_col[t] = V[size_t(t) * p + r];
+  __syncthreads();
+  bool bad = false;
+  for (int k = tid; k < p; k += LT) {
+    double d = k == r ? -1.0 : 0.0;
+    for (int t = 0; t < p; ++t) d = fma(s_col[t], V[size_t(t) * p + k], d);
+    bad = bad || fabs(d) > tol;
+  }
+  bad = __syncthreads_or(bad);
+  if (tid == 0) loose[r] = bad ? 1 : 0;
+}
+
+// The loose columns, orthogonalised twice against the others (from the unit vector e_t
+// farthest from their span, whose squared distance is 1 minus the sum of squares of their
+// entries t, where little of the column is left).  One CTA; returns at once without any.
+__global__ void __launch_bounds__(LT) tighten_columns_kernel(double* V, int p, int* loose) {
+  extern __shared__ double s_dot[];  // p coefficients, then p flags
+  int* s_loose = reinterpret_cast<int*>(s_dot + p);
+  __shared__ double sh[LT / 32];
+  __shared__ int s_at;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  bool any = false;
+  for (int k = tid; k < p; k += LT) {
+    s_loose[k] = loose[k];
+    any = any || s_loose[k] != 0;
+  }
+  if (!__syncthreads_or(any)) return;
+  for (int r = 0; r < p; ++r) {
+    if (s_loose[r] == 0) continue;
+    // column r without its part in the span, to norm 1; its norm before that
+    auto pass = [&] {
+      __syncthreads();
+      for (int k = warp; k < p; k += LT / 32) {
+        double d = 0.0;
+        if (s_loose[k] == 0)
+          for (int t = lane; t < p; t += 32) d = fma(V[size_t(t) * p + k], V[size_t(t) * p + r], d);
+        d = warp_sum(d);
+        if (lane == 0) s_dot[k] = d;
+      }
+      __syncthreads();
+      double part = 0.0;
+      for (int t = tid; t < p; t += LT) {
+        double v = V[size_t(t) * p + r];
+        for (int k = 0; k < p; ++k)
+          if (s_loose[k] == 0) v = fma(-s_dot[k], V[size_t(t) * p + k], v);
+        V[size_t(t) * p + r] = v;
+        part = fma(v, v, part);
+      }
+      const double norm = sqrt(block_sum(part, sh)), inv = norm > 0.0 ? 1.0 / norm : 0.0;
+      for (int t = tid; t < p; t += LT) V[size_t(t) * p + r] *= inv;
+      return norm;
+    };
+    if (!(pass() > 0.5)) {
+      for (int t = warp; t < p; t += LT / 32) {
+        double d = 0.0;
+        for (int k = lane; k < p; k += 32)
+          if (s_loose[k] == 0) d = fma(V[size_t(t) * p + k], V[size_t(t) * p + k], d);
+        d = warp_sum(d);
+        if (lane == 0) s_dot[t] = d;
+      }
+      __syncthreads();
+      if (tid == 0) {
+        s_at = 0;
+        for (int t = 1; t < p; ++t)
+          if (s_dot[t] < s_dot[s_at]) s_at = t;
+      }
+      __syncthreads();
+      for (int t = tid; t < p; t += LT) V[size_t(t) * p + r] = t == s_at ? 1.0 : 0.0;
+      pass();
+    }
+    pass();
+    __syncthreads();
+    if (tid == 0) s_loose[r] = 0;
+    __syncthreads();
+  }
+}
+
 __global__ void identity_kernel(double* X, int64_t p, const int* only_if) {
   if (only_if != nullptr && (*only_if & 1) == 0) return;
   for (int64_t idx = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; idx < p * p;
@@ -613,7 +728,10 @@ void jacobi_grid(Ctx& c, double* W, double* J, double* norm2, int64_t p, int64_t
                  const int* only_if) {
   Scope scope(c);
   unsigned* bar = c.alloc<unsigned>(8);
+  double* first = c.alloc<double>(size_t(p));
   if (c.sizing()) return;
+  row_norms_kernel<<<unsigned(p), LT, 0, c.stream>>>(W, L, first, nullptr, only_if);
+  CTM_LAUNCH_CHECK();
   identity_kernel<<<grid_for(p * p, 256), 256, 0, c.stream>>>(J, p, only_if);
   CTM_LAUNCH_CHECK();
   CTM_CUDA(cudaMemsetAsync(bar, 0, 8 * sizeof(unsigned), c.stream));
@@ -624,6 +742,7 @@ void jacobi_grid(Ctx& c, double* W, double* J, double* norm2, int64_t p, int64_t
   a.L = L;
   a.pp = p + (p & 1);
   a.tol = 2.220446049250313e-16 * std::sqrt(double(L));
+  a.first = first;
   a.max_sweeps = 60;
   a.bar = bar;
   a.flags = status_flags(c);
@@ -646,7 +765,7 @@ void jacobi_grid(Ctx& c, double* W, double* J, double* norm2, int64_t p, int64_t
                                          dim3(unsigned(blocks)), dim3(threads), args, 0, c.stream));
     CTM_LAUNCH_CHECK();
   }
-  row_norms_kernel<<<unsigned(p), LT, 0, c.stream>>>(W, L, norm2, only_if);
+  row_norms_kernel<<<unsigned(p), LT, 0, c.stream>>>(W, L, norm2, first, only_if);
   CTM_LAUNCH_CHECK();
 }
 
@@ -815,6 +934,7 @@ void svd_thin(Ctx& c, const double* X, int64_t m, int64_t n, double* U, double* 
   double* W2 = c.alloc<double>(size_t(p) * p);
   double* Xs = c.alloc<double>(size_t(p) * p);
   int* failed = c.alloc<int>(1);
+  int* loose = c.alloc<int>(p);
   load(Y, !tall);
   if (!house) orthonormalize_try(c, Y, L, p, R, failed);
   else if (!c.sizing()) householder_cluster(c, Y, L, p, R);
@@ -822,7 +942,16 @@ void svd_thin(Ctx& c, const double* X, int64_t m, int64_t n, double* U, double* 
   if (!c.sizing())
     CTM_CUDA(cudaMemcpyAsync(W2, R, sizeof(double) * p * p, cudaMemcpyDeviceToDevice, c.stream));
   jacobi_square(c, W2, J, norm2, p, flag);
-  if (!c.sizing()) finish(c, W2, J, norm2, p, p, Xs, S, Vs, top, nullptr);
+  if (!c.sizing()) {
+    finish(c, W2, J, norm2, p, p, Xs, S, Vs, top, nullptr);
+    KernelTimer kt(c.stream, "loose_columns_kernel", kUnitByte, 8.0 * double(p) * p);
+    loose_columns_kernel<<<unsigned(p), LT, size_t(p) * sizeof(double), c.stream>>>(Vs, S, int(p),
+                                                                                   loose);
+    CTM_LAUNCH_CHECK();
+    tighten_columns_kernel<<<1, LT, size_t(p) * (sizeof(double) + sizeof(int)), c.stream>>>(
+        Vs, int(p), loose);
+    CTM_LAUNCH_CHECK();
+  }
   einsum(c, "ik,kj->ij", View(Y, {L, p}), View(Xs, {p, p}), View(Vl, {L, p}));
   if (house) return;
   // when the Cholesky-QR has failed: the whole matrix again, in global memory
