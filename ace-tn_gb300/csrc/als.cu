@@ -13,6 +13,7 @@
 #include <cmath>
 
 #include "engine.cuh"
+#include "seeded.cuh"
 
 namespace ctm {
 namespace {

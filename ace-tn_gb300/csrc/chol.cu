@@ -14,6 +14,7 @@
 #include <cooperative_groups.h>
 
 #include "engine.cuh"
+#include "seeded.cuh"
 
 namespace ctm {
 

@@ -145,21 +145,4 @@ int* status_flags(Ctx& c);
 // (the Householder fallback ran), read by ctm_qr_fallbacks().
 unsigned long long* qr_fallback_counter();
 
-// 1 / d for a positive normal d, within about an ulp.
-__device__ __forceinline__ double positive_reciprocal(double d) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(d);
-  const int ex = int(b >> 52) - 1023;
-  if (ex < -1000 || ex > 1000) return 1.0 / d;
-  const double x = __longlong_as_double((long long)(b - ((unsigned long long)(long long)ex << 52)));
-  const float m = __uint_as_float(0x3f800000u | (unsigned(b >> 29) & 0x7fffffu));
-  // (widened by its bits: a conversion takes an FP64 issue slot, 64 cycles)
-  const unsigned u = __float_as_uint(__fdividef(1.f, m));
-  const double r0 = __longlong_as_double(
-      (long long)(((unsigned long long)((u >> 23) + 896u) << 52) |
-                  ((unsigned long long)(u & 0x7fffffu) << 29)));
-  const double e = fma(-x, r0, 1.0);
-  const double r = fma(r0, fma(e, e, e), r0);
-  return __longlong_as_double(__double_as_longlong(r) - ((long long)ex << 52));
-}
-
 }  // namespace ctm

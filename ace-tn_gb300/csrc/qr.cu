@@ -23,6 +23,7 @@
 #include <algorithm>
 
 #include "engine.cuh"
+#include "seeded.cuh"
 
 namespace ctm {
 
@@ -45,53 +46,6 @@ inline size_t qr_smem(int64_t nr, int64_t q, int64_t P) {
   // rows; U and M; partial sums and row j by parity; warp sums; betas, diagonals
   return (size_t(nr) * ld + size_t(q) * ld + 2 * size_t(P + 1) * q + size_t(kQrWarps) * q +
           2 * size_t(q)) * sizeof(double);
-}
-
-__device__ __forceinline__ bool mantissa_f64(double x, float& m, int& e) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-  const int ex = int(b >> 52) & 0x7ff;
-  m = __uint_as_float(0x3f800000u | (unsigned(b >> 29) & 0x7fffffu));
-  e = ex - 1023;
-  return ex != 0 && ex != 2047;
-}
-
-__device__ __forceinline__ double times_pow2(double x, int e) {  // results stay normal
-  return __longlong_as_double(__double_as_longlong(x) + ((long long)e << 52));
-}
-
-// alpha = -sign(a) sqrt(d) and beta = 2 / |v|^2 = 1 / (d - alpha a), d >= a^2,
-// from FP32 seeds with one cubic step each (relative errors below 2^-52); both
-// 0 for a zero column, NaN for a non-finite one.
-__device__ __forceinline__ void reflector(double d, double a, double& alpha, double& beta) {
-  float m;
-  int e;
-  if (!mantissa_f64(d, m, e)) {
-    const bool finite = ((unsigned long long)__double_as_longlong(d) << 1) < 0xffe0000000000000ull;
-    alpha = beta = finite ? 0.0 : __longlong_as_double(0x7ff8000000000000ll);
-    return;
-  }
-  const int odd = e & 1, half = (e - odd) / 2;
-  const double x = times_pow2(d, -(e - odd));  // in [1, 4)
-  const double y = double(rsqrtf(odd ? 2.f * m : m));
-  const double h = x * y;
-  const double r = fma(-h, y, 1.0);
-  const double z = fma(y * r, fma(r, 0.375, 0.5), y);
-  double s = x * z;
-  s = fma(0.5 * z, fma(-s, s, x), s);
-  s = times_pow2(s, half);  // sqrt(d)
-  alpha = a >= 0.0 ? -s : s;
-  const double v = fma(-alpha, a, d);
-  float mv;
-  int ev;
-  if (!mantissa_f64(v, mv, ev)) {
-    beta = 1.0 / v;
-    return;
-  }
-  const double xv = times_pow2(v, -ev);  // in [1, 2)
-  const double r0 = double(__fdividef(1.f, mv));
-  const double e1 = fma(-xv, r0, 1.0);
-  const double b = fma(r0, fma(e1, e1, e1), r0);
-  beta = ev > -1000 && ev < 1000 ? times_pow2(b, -ev) : scalbn(b, -ev);
 }
 
 template <int NC>  // column chunks of 32 lanes
@@ -347,6 +301,15 @@ __global__ void __launch_bounds__(kQrThreads) householder_cluster_kernel(const Q
   if (P > 1) cluster.sync();  // remote reads of V are over
 }
 
+// Test hook's: 1 / x, then alpha and beta of (x, y).
+__global__ void seeded_kernel(const double* x, const double* y, int64_t n, double* out) {
+  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n;
+       i += int64_t(gridDim.x) * blockDim.x) {
+    out[i] = positive_reciprocal(x[i]);
+    reflector(x[i], y[i], out[n + i], out[2 * n + i]);
+  }
+}
+
 }  // namespace
 
 // CTAs of the cluster for an n x q matrix, 0 when it does not fit.
@@ -414,3 +377,12 @@ void householder_cluster(Ctx& c, double* Y, int64_t n, int64_t q, double* R) {
 }
 
 }  // namespace ctm
+
+// Test hook, not part of the plugin interface (no declaration in the public header): the
+// functions of seeded.cuh on n pairs; out: n reciprocals, n alphas, n betas.
+extern "C" int ctm_test_seeded(const double* x, const double* y, int64_t n, double* out,
+                               void* stream) {
+  ctm::seeded_kernel<<<ctm::grid_for(n, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(x, y, n,
+                                                                                           out);
+  return int(cudaGetLastError());
+}

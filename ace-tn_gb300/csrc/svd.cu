@@ -22,6 +22,7 @@
 #include <cmath>
 
 #include "engine.cuh"
+#include "seeded.cuh"
 
 namespace ctm {
 
@@ -74,28 +75,6 @@ __device__ double block_sum(double v, double* sh) {
 // 0 stays, the others advance by one) and one cluster barrier follows.  (A
 // first form that moved two rows after every round of pairs spent about 2500
 // cycles per round in the cluster barrier and its remote stores.)
-
-// |x| = m 2^e with m in [1, 2) as FP32 (truncated to 24 bits); false for zero,
-// subnormals and non-finite values.
-__device__ __forceinline__ bool split_f64(double x, float& m, int& e) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-  const unsigned hi = unsigned(b >> 32) & 0x7fffffffu;
-  const int ex = int(hi >> 20);
-  m = __uint_as_float(0x3f800000u | (unsigned(b >> 29) & 0x7fffffu));
-  e = ex - 1023;
-  return ex != 0 && ex != 2047;
-}
-
-// FP32 value (normal) times 2^e as FP64, by bit patterns; 0 below the range.
-__device__ __forceinline__ double join_f64(float v, int e) {
-  const unsigned u = __float_as_uint(v);
-  const int ex = int((u >> 23) & 0xffu) - 127 + 1023 + e;
-  if (((u >> 23) & 0xffu) == 0u || ex < 1) return 0.0;
-  const unsigned long long b = ((unsigned long long)(u & 0x80000000u) << 32) |
-                               ((unsigned long long)ex << 52) |
-                               ((unsigned long long)(u & 0x7fffffu) << 29);
-  return __longlong_as_double((long long)b);
-}
 
 __device__ __forceinline__ double twice(double x) {  // exact, normal x below 2^1023
   return __longlong_as_double(__double_as_longlong(x) + (1ll << 52));
@@ -171,15 +150,12 @@ __device__ __forceinline__ bool rotate_pair(double* x, double* y, int L, int p, 
   }
   if (__double_as_longlong(h) == 0) return false;  // below the range of FP64
   if (!dz && neg) h = negate(h);
-  // s = 2 h / (1 + h^2): FP32 reciprocal and one cubic Newton step
+  // s = 2 h / (1 + h^2)
   const double d = fma(h, h, 1.0);
   float md1;
   int ed1;
   split_f64(d, md1, ed1);  // 1 <= d < 2
-  const double r0 = join_f64(__fdividef(1.f, md1), 0);
-  const double e1 = fma(-d, r0, 1.0);
-  const double e2 = fma(e1, e1, e1);
-  const double s = twice(h) * fma(r0, e2, r0);
+  const double s = twice(h) * mantissa_reciprocal(d, md1);
   const double mh = negate(h);
 #pragma unroll 2
   for (int t = sub; t < L; t += kTP) {
