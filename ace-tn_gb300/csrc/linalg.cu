@@ -601,10 +601,13 @@ __global__ void __launch_bounds__(kCh > 0 ? 128 * kCh : 1024) jacobi_onesided_f3
 // pairs in the same rounds with the same arithmetic (bit for bit), but row r lives
 // in the shared memory of CTA r mod P of a cluster instead of global memory, and
 // pair k of a round is rotated by CTA k mod P through distributed shared memory.
-// kCh > 0: ld = 32 kCh, the two data rows held in registers; 0: any ld.
+// kCh > 0: ld = 32 kCh, the two data rows and their rotations held in registers, which
+// they fill at kCh = 12 (240 of 255); 0: any ld, both data rows read a second time.
+// svd_f32 at q = 289, 300, 340, 384 with rows in registers 22, 23, 31, 41 ms, as any ld
+// 37, 39, 49, 61 ms; at q = 400 any ld 73 ms.
 // (q = 272: 27 ms on one CTA from L2, about 12 us for each of 271 rounds a sweep.)
 template <int kCh>
-__global__ void __launch_bounds__(kCh > 0 ? 160 : 512)
+__global__ void __launch_bounds__(kCh > 0 ? 192 : 512)
     jacobi_spread_f32_kernel(const float* Mc_g, int q, int pp, float* Jc_g, float* norms,
                              int max_sweeps, float tol, int* flags) {
   namespace cg = cooperative_groups;
@@ -1745,8 +1748,13 @@ void jacobi_rotations_impl(Ctx& c, const float* Mc, int64_t q, float* Jc, float*
       CTM_CUDA(cudaLaunchKernelEx(&cfg, kern, Mc, int(q), int(pp), Jc, norms, max_sweeps, 4e-6f,
                                   flags));
     };
-    if (jacobi_ld(int(q)) / 32 == 9) launch(jacobi_spread_f32_kernel<9>);
-    else launch(jacobi_spread_f32_kernel<0>);
+    switch (jacobi_ld(int(q)) / 32) {
+      case 9: launch(jacobi_spread_f32_kernel<9>); break;
+      case 10: launch(jacobi_spread_f32_kernel<10>); break;
+      case 11: launch(jacobi_spread_f32_kernel<11>); break;
+      case 12: launch(jacobi_spread_f32_kernel<12>); break;
+      default: launch(jacobi_spread_f32_kernel<0>); break;
+    }
   } else {
     KernelTimer kt(c.stream, "jacobi_onesided_f32_kernel", kUnitFlop, 0.0);
     jacobi_onesided_f32_kernel<false, 0><<<1, jthreads, 0, c.stream>>>(
