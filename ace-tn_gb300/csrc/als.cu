@@ -5,11 +5,12 @@
 // cuTENSOR plans and cuSOLVER potrf/potrs in its optional extension).  Here
 // the contractions go through the strided GETT engine and each least-squares
 // step is one kernel: the symmetrised, shifted system is factorised in one
-// CTA with the matrix in shared memory (Cholesky, then the triangular solves with
+// CTA with the matrix in shared memory (L D L^T, then the back substitution with
 // one warp per right-hand side; Gaussian elimination with partial pivoting when a
-// pivot is not positive, the reference's torch.linalg.solve fallback).  The pseudo-inverse method runs the FP64
-// one-sided Jacobi SVD of the symmetrised system.  The host loop reads the
-// cost once per iteration for the reference's convergence test.
+// pivot is not positive, the reference's torch.linalg.solve fallback).  The
+// pseudo-inverse method runs the FP64 one-sided Jacobi SVD of the symmetrised
+// system.  The host loop reads the cost once per iteration for the reference's
+// convergence test.
 #include <cmath>
 
 #include "engine.cuh"

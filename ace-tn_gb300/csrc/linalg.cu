@@ -1422,7 +1422,8 @@ void orthonormalize_impl(Ctx& c, T* Y, int64_t n, int64_t q, T* R, int stages,
   CTM_REQUIRE(n >= q && q >= 1, CTM_ERR_INVALID, "orthonormalize: needs n >= q >= 1");
   CTM_REQUIRE(stages == 2 || stages == 3, CTM_ERR_INVALID, "orthonormalize: 2 or 3 stages");
   Scope scope(c);
-  T* V = c.alloc<T>(size_t(n) * q);
+  // the input for the Householder fallback
+  T* V = failed == nullptr ? c.alloc<T>(size_t(n) * q) : nullptr;
   T* beta = c.alloc<T>(q);
   // Householder QR for small problems: FP64 in a cluster's shared memory where
   // it fits, else on one CTA (its cost grows as q^2 barriers; the FP32 slab
@@ -1543,7 +1544,7 @@ void orthonormalize_impl(Ctx& c, T* Y, int64_t n, int64_t q, T* R, int stages,
   }
   // cur holds Q after the stages and G its Gram matrix; check it and fall
   // back when needed
-  T* hv = c.alloc<T>(size_t(n) * q);
+  T* hv = failed == nullptr ? c.alloc<T>(size_t(n) * q) : nullptr;
   if (c.sizing()) return;
   if (!fast_f32) {  // (the FP32 slab path checked G in its last reduction)
     KernelTimer kt(c.stream, "orthogonality_check_kernel", kUnitByte, double(sizeof(T)) * q * q);
