@@ -98,7 +98,8 @@ struct ClusterJacobi {
   int max_sweeps;
   float tol2;       // squared convergence tolerance
   int* flags;       // status word
-  const int* skip;  // nothing to do when (*skip & 1)
+  const int* skip;  // nothing to do when (*skip & 1) is not run_if
+  int run_if;
 };
 
 // Doubles per row in shared memory: the row, its rotations, its squared norm and the first
@@ -192,7 +193,7 @@ template <int kTP>
 __global__ void __launch_bounds__(512) jacobi_cluster_f64_kernel(const ClusterJacobi a) {
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
-  if (a.skip != nullptr && (*a.skip & 1) != 0) return;  // the whole cluster alike
+  if (a.skip != nullptr && (*a.skip & 1) != a.run_if) return;  // the whole cluster alike
   const int P = int(cluster.num_blocks()), k = int(cluster.block_rank());
   const int m = a.m, L = a.L, p = a.p;
   const int RS = jacobi_row(p, L);
@@ -345,7 +346,8 @@ JacobiShape jacobi_shape(int64_t p, int64_t L) {
 }
 
 void jacobi_cluster(Ctx& c, const JacobiShape& sh, double* W, double* J, const double* J0,
-                    double* norm2, int64_t p, int64_t L, double tol, const int* skip) {
+                    double* norm2, int64_t p, int64_t L, double tol, const int* skip,
+                    int run_if = 0) {
   ClusterJacobi a{};
   a.W = W;
   a.J = J;
@@ -358,6 +360,7 @@ void jacobi_cluster(Ctx& c, const JacobiShape& sh, double* W, double* J, const d
   a.tol2 = float(tol * tol);
   a.flags = status_flags(c);
   a.skip = skip;
+  a.run_if = run_if;
   const size_t smem = jacobi_smem(sh.m, p, L);
   auto launch = [&](auto kern) {
     CTM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
@@ -389,7 +392,6 @@ struct JacobiArgs {
   int64_t p, L;
   int64_t pp;     // p rounded up to even
   double tol;
-  const double* first;  // p: squared norms before the sweeps (kCollapsed)
   int max_sweeps;
   unsigned* bar;  // [0] arrival count, [1] generation, [2] abort, [3..4] sweep flags
   int* flags;
@@ -462,9 +464,7 @@ __global__ void __launch_bounds__(64) jacobi_sweeps_kernel(const JacobiArgs a) {
         al = warp_sum(al);
         be = warp_sum(be);
         ga = warp_sum(ga);
-        if (al <= kCollapsed * a.first[i] || be <= kCollapsed * a.first[j] ||
-            !(fabs(ga) > a.tol * sqrt(al) * sqrt(be)))
-          continue;
+        if (al == 0.0 || be == 0.0 || !(fabs(ga) > a.tol * sqrt(al) * sqrt(be))) continue;
         const double zeta = (be - al) / (2.0 * ga);
         const double t = copysign(1.0, zeta) / (fabs(zeta) + sqrt(fma(zeta, zeta, 1.0)));
         const double cs = 1.0 / sqrt(fma(t, t, 1.0));
@@ -492,26 +492,23 @@ __global__ void __launch_bounds__(64) jacobi_sweeps_kernel(const JacobiArgs a) {
   if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(a.flags, 2);
 }
 
-// Squared norms of the rows of W (p x L), one CTA per row; with those before the sweeps,
-// collapsed rows become zero.
-__global__ void __launch_bounds__(LT) row_norms_kernel(double* W, int64_t L, double* norm2,
-                                                       const double* first, const int* only_if) {
+// Squared norms of the rows of W (p x L), one CTA per row.
+__global__ void __launch_bounds__(LT) row_norms_kernel(const double* W, int64_t L, double* norm2,
+                                                       const int* only_if) {
   if (only_if != nullptr && (*only_if & 1) == 0) return;
   __shared__ double sh[LT / 32];
-  double* w = W + int64_t(blockIdx.x) * L;
+  const double* w = W + int64_t(blockIdx.x) * L;
   double part = 0.0;
   for (int64_t t = threadIdx.x; t < L; t += blockDim.x) part = fma(w[t], w[t], part);
   part = block_sum(part, sh);
-  if (first != nullptr && part < kCollapsed * first[blockIdx.x]) {
-    for (int64_t t = threadIdx.x; t < L; t += blockDim.x) w[t] = 0.0;
-    part = 0.0;
-  }
   if (threadIdx.x == 0) norm2[blockIdx.x] = part;
 }
 
-// The input is scaled by a power of two that puts its largest entry's exponent at kTop:
-// squared norms stay below 2^1023 and the dot products of rows 2^-900 as long are still
-// normal numbers.  (Exact, so the result has the same bits wherever none underflowed.)
+// The input is scaled by a power of two that puts its largest entry's exponent at kTop for
+// the cluster form: squared norms stay below 2^1023 and the dot products of rows 2^-900 as
+// long are still normal numbers.  The form in global memory compares subnormal ones too, and
+// rows that collapse have to underflow there: 0.  (Exact, so the result has the same bits
+// wherever none underflowed.)
 constexpr int kTop = 440;
 
 // Largest exponent field of the finite entries; *top zeroed where the grid has several CTAs.
@@ -543,15 +540,15 @@ __device__ __forceinline__ double scaled(double x, int e) {
 }
 
 // Exponent of the scaling (even: the halves of the exponents that a square root sees stay).
-__device__ __forceinline__ int scale_exponent(int top) {
-  return (kTop + 1023 - max(top, 1)) & ~1;
+__device__ __forceinline__ int scale_exponent(int top, int target) {
+  return (target + 1023 - max(top, 1)) & ~1;
 }
 
 // dst[r][c] = X[r s0 + c s1] 2^e, rows x cols.
 __global__ void __launch_bounds__(256) scaled_copy_kernel(const double* X, int64_t rows,
                                                           int64_t cols, int64_t s0, int64_t s1,
-                                                          const int* top, double* dst) {
-  const int e = scale_exponent(*top);
+                                                          const int* top, int target, double* dst) {
+  const int e = scale_exponent(*top, target);
   for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < rows * cols;
        i += int64_t(gridDim.x) * blockDim.x) {
     const int64_t r = i / cols, q = i - r * cols;
@@ -567,7 +564,7 @@ __global__ void __launch_bounds__(256) scaled_copy_kernel(const double* X, int64
 __global__ void __launch_bounds__(LT) jacobi_finish_kernel(const double* W, const double* J,
                                                            const double* norm2, int64_t p,
                                                            int64_t L, double* Vs, double* S,
-                                                           double* Vl, const int* top,
+                                                           double* Vl, const int* top, int target,
                                                            const int* only_if) {
   if (only_if != nullptr && (*only_if & 1) == 0) return;
   const int64_t j = blockIdx.x;
@@ -587,7 +584,7 @@ __global__ void __launch_bounds__(LT) jacobi_finish_kernel(const double* W, cons
   const int64_t rk = s_rank;
   const double sj = sqrt(nj2);
   const double inv = sj > 0.0 ? 1.0 / sj : 0.0;
-  if (threadIdx.x == 0) S[rk] = scaled(sj, -scale_exponent(*top));
+  if (threadIdx.x == 0) S[rk] = scaled(sj, -scale_exponent(*top, target));
   for (int64_t t = threadIdx.x; t < p; t += blockDim.x) Vs[t * p + rk] = J[j * p + t];
   for (int64_t t = threadIdx.x; t < L; t += blockDim.x) Vl[t * p + rk] = W[j * L + t] * inv;
 }
@@ -600,9 +597,9 @@ __global__ void __launch_bounds__(LT) jacobi_finish_kernel(const double* W, cons
 // loose[r]: whether column r, of a value below 1e-8 of the largest, is not orthonormal to the
 // others.  One CTA per column (2 us without small values).
 __global__ void __launch_bounds__(LT) loose_columns_kernel(const double* V, const double* S, int p,
-                                                           int* loose) {
+                                                           int* loose, const int* skip) {
   const int r = blockIdx.x, tid = threadIdx.x;
-  if (!(S[r] < 1e-8 * S[0] || S[r] == 0.0)) {
+  if ((skip != nullptr && (*skip & 1) != 0) || !(S[r] < 1e-8 * S[0] || S[r] == 0.0)) {
     if (tid == 0) loose[r] = 0;
     return;
   }
@@ -693,9 +690,9 @@ __global__ void identity_kernel(double* X, int64_t p, const int* only_if) {
 }
 
 void finish(Ctx& c, const double* W, const double* J, const double* norm2, int64_t p, int64_t L,
-            double* Vs, double* S, double* Vl, const int* top, const int* only_if) {
+            double* Vs, double* S, double* Vl, const int* top, int target, const int* only_if) {
   KernelTimer kt(c.stream, "jacobi_finish_kernel", kUnitByte, 16.0 * double(p) * (p + L));
-  jacobi_finish_kernel<<<unsigned(p), LT, 0, c.stream>>>(W, J, norm2, p, L, Vs, S, Vl, top, only_if);
+  jacobi_finish_kernel<<<unsigned(p), LT, 0, c.stream>>>(W, J, norm2, p, L, Vs, S, Vl, top, target, only_if);
   CTM_LAUNCH_CHECK();
 }
 
@@ -704,10 +701,7 @@ void jacobi_grid(Ctx& c, double* W, double* J, double* norm2, int64_t p, int64_t
                  const int* only_if) {
   Scope scope(c);
   unsigned* bar = c.alloc<unsigned>(8);
-  double* first = c.alloc<double>(size_t(p));
   if (c.sizing()) return;
-  row_norms_kernel<<<unsigned(p), LT, 0, c.stream>>>(W, L, first, nullptr, only_if);
-  CTM_LAUNCH_CHECK();
   identity_kernel<<<grid_for(p * p, 256), 256, 0, c.stream>>>(J, p, only_if);
   CTM_LAUNCH_CHECK();
   CTM_CUDA(cudaMemsetAsync(bar, 0, 8 * sizeof(unsigned), c.stream));
@@ -718,7 +712,6 @@ void jacobi_grid(Ctx& c, double* W, double* J, double* norm2, int64_t p, int64_t
   a.L = L;
   a.pp = p + (p & 1);
   a.tol = 2.220446049250313e-16 * std::sqrt(double(L));
-  a.first = first;
   a.max_sweeps = 60;
   a.bar = bar;
   a.flags = status_flags(c);
@@ -741,13 +734,19 @@ void jacobi_grid(Ctx& c, double* W, double* J, double* norm2, int64_t p, int64_t
                                          dim3(unsigned(blocks)), dim3(threads), args, 0, c.stream));
     CTM_LAUNCH_CHECK();
   }
-  row_norms_kernel<<<unsigned(p), LT, 0, c.stream>>>(W, L, norm2, first, only_if);
+  row_norms_kernel<<<unsigned(p), LT, 0, c.stream>>>(W, L, norm2, only_if);
   CTM_LAUNCH_CHECK();
 }
 
 // FP32 copy of X (n entries) scaled by a power of two so that its largest entry
-// is below 2 (one CTA; entries below the FP32 range become zeros).
-__global__ void __launch_bounds__(1024) scaled_f32_kernel(const double* X, int n, float* Y) {
+// is below 2 (one CTA; entries below the FP32 range become zeros; all of them when
+// (*skip & 1): what follows then has nothing to do).
+__global__ void __launch_bounds__(1024) scaled_f32_kernel(const double* X, int n, float* Y,
+                                                          const int* skip) {
+  if (skip != nullptr && (*skip & 1) != 0) {
+    for (int i = threadIdx.x; i < n; i += blockDim.x) Y[i] = 0.f;
+    return;
+  }
   __shared__ int s_top;
   if (threadIdx.x == 0) s_top = 0;
   __syncthreads();
@@ -797,7 +796,7 @@ void jacobi_square(Ctx& c, double* W, double* J, double* norm2, int64_t p, const
   double* G = c.alloc<double>(pp);
   int* unused = c.alloc<int>(1);  // an unfinished FP32 stage is not a failure
   if (!c.sizing()) {
-    scaled_f32_kernel<<<1, 1024, 0, c.stream>>>(W, int(pp), Wf);
+    scaled_f32_kernel<<<1, 1024, 0, c.stream>>>(W, int(pp), Wf, skip);
     CTM_LAUNCH_CHECK();
   }
   // what is left after ten sweeps lies at the FP32 rounding level
@@ -865,21 +864,23 @@ void svd_thin(Ctx& c, const double* X, int64_t m, int64_t n, double* U, double* 
   double* norm2 = c.alloc<double>(p);
   int* top = c.alloc<int>(1);
   // dst = X (rows first) or X^T, scaled
-  auto load = [&](double* dst, bool transposed) {
+  auto load = [&](double* dst, bool transposed, int target) {
     if (c.sizing()) return;
     KernelTimer kt(c.stream, "scaled_copy_kernel", kUnitByte, 16.0 * double(m) * n);
     scaled_copy_kernel<<<grid_for(m * n, 256), 256, 0, c.stream>>>(
-        X, transposed ? n : m, transposed ? m : n, transposed ? 1 : n, transposed ? n : 1, top, dst);
+        X, transposed ? n : m, transposed ? m : n, transposed ? 1 : n, transposed ? n : 1, top, target,
+        dst);
     CTM_LAUNCH_CHECK();
   };
-  auto load_w = [&] { load(W, tall); };  // W rows = columns of X (tall) or rows of X
+  const JacobiShape direct = jacobi_shape(p, L), square = jacobi_shape(p, p);
+  const int target = direct.ctas > 0 ? kTop : 0;  // of W, which is rotated as it is
+  auto load_w = [&] { load(W, tall, target); };   // W rows = columns of X (tall) or rows of X
   if (!c.sizing()) {
     const int ctas = int(std::min<int64_t>(sm_count_linalg(), (m * n + 32767) / 32768));
     if (ctas > 1) CTM_CUDA(cudaMemsetAsync(top, 0, sizeof(int), c.stream));
     top_field_kernel<<<ctas, 1024, 0, c.stream>>>(X, m * n, top);
     CTM_LAUNCH_CHECK();
   }
-  const JacobiShape direct = jacobi_shape(p, L), square = jacobi_shape(p, p);
   // The one-cluster Householder QR up to the size where the Cholesky-QR (about
   // 20 launches and three one-SM factorisations) is faster; the latter only
   // where it saves long rows, as it takes well-conditioned input.  No QR for
@@ -898,7 +899,7 @@ void svd_thin(Ctx& c, const double* X, int64_t m, int64_t n, double* U, double* 
     } else {
       jacobi_grid(c, W, J, norm2, p, L, nullptr);
     }
-    if (!c.sizing()) finish(c, W, J, norm2, p, L, Vs, S, Vl, top, nullptr);
+    if (!c.sizing()) finish(c, W, J, norm2, p, L, Vs, S, Vl, top, target, nullptr);
     return;
   }
   // long side = Y R.  The rows of R are rotated, R = J^T W: the short side's
@@ -911,7 +912,7 @@ void svd_thin(Ctx& c, const double* X, int64_t m, int64_t n, double* U, double* 
   double* Xs = c.alloc<double>(size_t(p) * p);
   int* failed = c.alloc<int>(1);
   int* loose = c.alloc<int>(p);
-  load(Y, !tall);
+  load(Y, !tall, kTop);
   if (!house) orthonormalize_try(c, Y, L, p, R, failed);
   else if (!c.sizing()) householder_cluster(c, Y, L, p, R);
   const int* const flag = house ? nullptr : failed;
@@ -919,10 +920,10 @@ void svd_thin(Ctx& c, const double* X, int64_t m, int64_t n, double* U, double* 
     CTM_CUDA(cudaMemcpyAsync(W2, R, sizeof(double) * p * p, cudaMemcpyDeviceToDevice, c.stream));
   jacobi_square(c, W2, J, norm2, p, flag);
   if (!c.sizing()) {
-    finish(c, W2, J, norm2, p, p, Xs, S, Vs, top, nullptr);
+    finish(c, W2, J, norm2, p, p, Xs, S, Vs, top, kTop, nullptr);
     KernelTimer kt(c.stream, "loose_columns_kernel", kUnitByte, 8.0 * double(p) * p);
-    loose_columns_kernel<<<unsigned(p), LT, size_t(p) * sizeof(double), c.stream>>>(Vs, S, int(p),
-                                                                                   loose);
+    loose_columns_kernel<<<unsigned(p), LT, size_t(p) * sizeof(double), c.stream>>>(
+        Vs, S, int(p), loose, flag);
     CTM_LAUNCH_CHECK();
     tighten_columns_kernel<<<1, LT, size_t(p) * (sizeof(double) + sizeof(int)), c.stream>>>(
         Vs, int(p), loose);
@@ -930,10 +931,13 @@ void svd_thin(Ctx& c, const double* X, int64_t m, int64_t n, double* U, double* 
   }
   einsum(c, "ik,kj->ij", View(Y, {L, p}), View(Xs, {p, p}), View(Vl, {L, p}));
   if (house) return;
-  // when the Cholesky-QR has failed: the whole matrix again, in global memory
+  // when the Cholesky-QR has failed: the whole matrix again, in a cluster where it fits (100
+  // x 601 with values from 1 to 1e-15: 42 ms in global memory), else in global memory
   load_w();
-  jacobi_grid(c, W, J, norm2, p, L, failed);
-  if (!c.sizing()) finish(c, W, J, norm2, p, L, Vs, S, Vl, top, failed);
+  if (direct.ctas == 0) jacobi_grid(c, W, J, norm2, p, L, failed);
+  else if (!c.sizing())
+    jacobi_cluster(c, direct, W, J, nullptr, norm2, p, L, eps * std::sqrt(double(L)), failed, 1);
+  if (!c.sizing()) finish(c, W, J, norm2, p, L, Vs, S, Vl, top, target, failed);
 }
 
 }  // namespace ctm
