@@ -879,9 +879,9 @@ bool unit_stride(const Group& g, bool second) {
 
 }  // namespace
 
-// From about 2e7 multiply-adds on the digit form is the faster one: 256^3 takes
-// 40 us in the FP64 GETT, 400^3 (6.4e7) 70 us in digits and about 150 in the
-// GETT; 5184 x 5184 x 144 takes 0.33 ms against 11 ms.
+// From about 2e7 multiply-adds on the digit form is the faster one, whole calls: 256^3
+// takes 49 us in the FP64 GETT, 272^3 72 us in digits and 68 to 80 in the GETT, 400^3
+// (6.4e7) 78 against 200; 5184 x 5184 x 144 takes 0.33 ms against 11 ms.
 bool digits_pay(int64_t rows, int64_t columns, int64_t K) {
   return double(rows) * double(columns) * double(K) >= 2.0e7 && K >= 16 &&
          std::min(rows, columns) >= 16;

@@ -25,8 +25,9 @@ constexpr int BK = 16, NT = 256;
 // (its global loads are in flight while the current step computes).  Each tile
 // loader walks whichever of its two index groups has unit stride, so warps
 // read contiguous memory for either operand orientation.
-template <class T, int kT>
-__global__ void __launch_bounds__(NT) gett_kernel(const GettArgs<T> p) {
+template <int kT>
+__global__ void __launch_bounds__(NT) gett_kernel(const GettArgs<double> p) {
+  using T = double;
   constexpr int BM = 16 * kT, BN = 16 * kT;
   __shared__ int64_t sAm[BM], sCm[BM], sBn[BN], sCn[BN];
   __shared__ int64_t sAk[2][BK], sBk[2][BK];
@@ -525,9 +526,9 @@ void einsum_impl(Ctx& c, const char* spec, const ViewT<T>& A, const ViewT<T>& B,
     if constexpr (sizeof(T) == 4) {
       gett_f32(c, p);
     } else {
-      if (tile == 4) gett_kernel<T, 4><<<grid, NT, 0, c.stream>>>(p);
-      else if (tile == 2) gett_kernel<T, 2><<<grid, NT, 0, c.stream>>>(p);
-      else gett_kernel<T, 1><<<grid, NT, 0, c.stream>>>(p);
+      if (tile == 4) gett_kernel<4><<<grid, NT, 0, c.stream>>>(p);
+      else if (tile == 2) gett_kernel<2><<<grid, NT, 0, c.stream>>>(p);
+      else gett_kernel<1><<<grid, NT, 0, c.stream>>>(p);
     }
     CTM_LAUNCH_CHECK();
   }

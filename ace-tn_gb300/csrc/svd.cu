@@ -4,7 +4,8 @@
 //    of up to 16 CTAs (up to about 320 x 320), from the rotations of an FP32
 //    Jacobi when the matrix is square (144 x 144: 2.6 to 4.3 ms, 27 ms as
 //    jacobi_sweeps_kernel; 80 x 80: 1.2 to 2.0 ms against 11 ms).
-//  * From 32 to 160 columns, and for long matrices, a QR factorisation first: the
+//  * From 32 columns to what the Householder cluster holds (149 square, L p^2 <= 4e6),
+//    and for matrices more than six times as long as wide, a QR factorisation first: the
 //    rows of the p x p factor R are rotated and the long singular vectors are
 //    one product with Q.  R is graded even when the matrix is not, which is
 //    what one-sided Jacobi needs: a 144 x 144 product of four enlarged corners
@@ -13,9 +14,10 @@
 //    rank), else a shifted Cholesky-QR3.
 //  * jacobi_sweeps_kernel: rows in global memory, a cooperative grid with a
 //    bounded grid barrier (Demmel & Veselic, SIAM J. Matrix Anal. Appl. 13
-//    (1992) 1204): matrices beyond the cluster's shared memory, and inputs on
-//    which the Cholesky-QR fails its orthogonality check (numerically
-//    rank-deficient ones; decided on the device, no synchronisation).
+//    (1992) 1204): matrices beyond the cluster's shared memory, those on which
+//    the Cholesky-QR fails its orthogonality check among them (numerically
+//    rank-deficient ones; decided on the device, no synchronisation; in the
+//    cluster form where they fit).
 #include <cooperative_groups.h>
 
 #include <algorithm>

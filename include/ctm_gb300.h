@@ -10,7 +10,10 @@
  * Workspace protocol: call with ws == NULL and *ws_bytes ignored; the entry
  * point stores the bytes it needs in *ws_bytes and returns CTM_OK without
  * launching anything.  Call again with a buffer of at least that size
- * (256-byte aligned).
+ * (256-byte aligned).  Sizes depend on the library's version: the FP64 path
+ * keeps operands of large contractions in digits of 16 bytes per entry (up to
+ * 2 GB for a contraction and 4 GB for the factors of a randomized SVD, for
+ * each move or projector pair that a call runs at once).
  *
  * Tensor layouts (reference: acetn/ipeps/site_tensor.py:41-83):
  *   A    (D, D, D, D, d)          legs (left, up, right, down, phys)
