@@ -183,10 +183,13 @@ __device__ __noinline__ void chain_marked(const ChainOutputs& a, int blocks, Whe
       where(b, r, w);
       const int lane = threadIdx.x & 31;
       uint32_t left[kCRows / 32];
+      // (no bits beyond the columns: a product that gave up has not written its words)
+      const uint32_t valid =
+          low_bits(int(min(int64_t(a.marks.per), a.columns - w * a.marks.per)));
 #pragma unroll
       for (int i = 0; i < kCRows / 32; ++i) {
         const int64_t row = r + 32 * i + lane;
-        left[i] = row < a.marks.rows ? a.marks.word[w * a.marks.rows + row] : 0u;
+        left[i] = row < a.marks.rows ? a.marks.word[w * a.marks.rows + row] & valid : 0u;
       }
 #pragma unroll
       for (int i = 0; i < kCRows / 32; ++i) {
