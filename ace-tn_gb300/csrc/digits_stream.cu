@@ -13,7 +13,8 @@
 // kernel, and eight warps read the accumulators of one group of columns while
 // the MMAs of the next run: 0.40 ms in one kernel.  K = 72 with 36 columns (two
 // phases of the contracted index, one accumulator buffer) takes 0.72 ms, 1.16 ms
-// as digit_gemm_kernel.
+// as digit_gemm_kernel.  (Both before the splitting warps noted which entries are
+// large, for the outputs far below their scales: 0.42 ms for the first.)
 #include <algorithm>
 #include <type_traits>
 
