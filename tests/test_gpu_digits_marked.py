@@ -1,7 +1,7 @@
 """Outputs that the FP64 digit products leave to the FMA chain: those on rows and
 columns with an infinity or a NaN, in each form of the products (column tiles, K ranges
 that are summed, the streaming form) and each form of the chain kernel (listed outputs
-of short and long chains, tiles)."""
+of short and long chains, whole blocks)."""
 
 import pytest
 import torch
